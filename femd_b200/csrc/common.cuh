@@ -84,8 +84,6 @@ struct DevBuf {
     ~DevBuf() { release(); }
 };
 
-struct Workspace;
-
 }  // namespace femd
 
 struct femd_ctx_s {
@@ -98,6 +96,11 @@ struct femd_ctx_s {
     // a small device status block: [0] error flags, [1] first bad row, [2..] spare
     int *status_dev = nullptr;
     int *status_host = nullptr;   // pinned
+    // the on-chip solve (resident.cu): device scratch, grown to the largest such system (a few MB at
+    // most), pinned room for its result, and the events that time it
+    femd::DevBuf<double> res_scratch;
+    void *res_host = nullptr;
+    cudaEvent_t res_e0 = nullptr, res_e1 = nullptr;
 };
 
 namespace femd {
@@ -170,6 +173,7 @@ struct femd_matrix_s : femd::HandleBase {
     // every preconditioned solve refuses the matrix instead of reading uninitialised memory
     bool inv_valid = false;
     int spmv_tpr = 0;                    // autotuned threads per row (0: not tuned)
+    bool resident_unfit = false;         // the on-chip solve has found that a block's rows do not fit
     // the solver workspace of this matrix (vectors, pinned state, captured CUDA graphs), kept
     // between solves so that a solve allocates nothing once it has run once
     void *solver_ws = nullptr;

@@ -7,6 +7,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "resident.h"
 
 namespace femd {
 
@@ -228,6 +229,9 @@ void ctx_release(femd_ctx ctx)
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->status_dev);
     cudaFreeHost(ctx->status_host);
+    cudaFreeHost(ctx->res_host);
+    if (ctx->res_e0) cudaEventDestroy(ctx->res_e0);
+    if (ctx->res_e1) cudaEventDestroy(ctx->res_e1);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -262,9 +266,16 @@ int femd_cuda_ctx_create(int device, femd_ctx *out)
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, 4 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, 4 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->res_host, sizeof(femd::ResidentOut));
+    if (e == cudaSuccess) e = cudaEventCreate(&c->res_e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&c->res_e1);
     if (e != cudaSuccess) {
         set_error(std::string("femd_cuda_ctx_create: ") + cudaGetErrorString(e));
         if (c->status_dev) cudaFree(c->status_dev);
+        if (c->status_host) cudaFreeHost(c->status_host);
+        if (c->res_host) cudaFreeHost(c->res_host);
+        if (c->res_e0) cudaEventDestroy(c->res_e0);
+        if (c->res_e1) cudaEventDestroy(c->res_e1);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
         return FEMD_ECUDA;

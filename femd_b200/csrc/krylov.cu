@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "resident.h"
 
 namespace femd {
 
@@ -716,13 +717,80 @@ static int capture_cg64(femd_ctx ctx, femd_matrix K, SolverWS &W, bool jac)
     return FEMD_OK;
 }
 
-// One FP64 CG solve (cg.hpp:296-350) on the matrix's workspace.
+// The result of a solve from its device state: ||b||, ||b - A x||, iterations, breakdown (cg.hpp:222-237, 306).
+static void cg_result(double nb, double res64, int it, int breakdown, int max_iter, double tol, femd_cg_result *res)
+{
+    if (nb == 0.0) {
+        res->converged = 1; res->iterations = 0; res->residual = 0.0; res->breakdown = 0;
+        return;
+    }
+    res->iterations = it;
+    res->breakdown = breakdown;
+    res->residual = res64 / nb;
+    int conv = !breakdown && res->residual <= tol * (1.0 + 1e-6) + 1e-15;
+    if (!conv && !breakdown && res->residual <= 10.0 * tol && it < max_iter) conv = 1;
+    res->converged = conv;
+}
+
+// The on-chip solve where the system fits (resident.cu); *ran says whether it did. scratch: n +
+// RES_SLOT_DOUBLES + RES_OUT_DOUBLES doubles; timed: with the context's events.
+static int cg_resident(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double *x, int max_iter, double tol,
+                       const ResidentPlan &plan, double *zx, double *slots, ResidentOut *out, bool timed, bool *ran,
+                       femd_cg_result *res)
+{
+    femd_pattern P = K->pattern;
+    cudaStream_t s = ctx->stream;
+    *ran = false;
+    if (timed) FEMD_TRY_CUDA(cudaEventRecord(ctx->res_e0, s));
+    const cudaError_t e = resident_launch(plan, P->indptr.p, P->indices.p, K->data.p, jac ? K->inv.p : nullptr, b, x, P->nrows,
+                                          max_iter, tol, zx, slots, out, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {
+        cudaGetLastError();                     // part of the device is taken away: the streaming loop needs no co-residency
+        K->resident_unfit = true;
+        return FEMD_OK;
+    }
+    FEMD_TRY_CUDA(e);
+    if (timed) FEMD_TRY_CUDA(cudaEventRecord(ctx->res_e1, s));
+    ResidentOut *S = static_cast<ResidentOut *>(ctx->res_host);
+    FEMD_TRY_CUDA(cudaMemcpyAsync(S, out, sizeof(ResidentOut), cudaMemcpyDeviceToHost, s));
+    FEMD_TRY_CUDA(cudaStreamSynchronize(s));
+    if (S->timeout) {
+        set_error("cg: a block of the solve waited too long for the others");
+        return FEMD_ETIMEOUT;
+    }
+    if (S->unfit) {
+        K->resident_unfit = true;
+        return FEMD_OK;
+    }
+    *ran = true;
+    cg_result(S->nb, S->res64, S->it, S->breakdown, max_iter, tol, res);
+    res->status = FEMD_OK;
+    res->outer = 0;
+    if (timed) {
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->res_e0, ctx->res_e1);
+        res->seconds = ms * 1e-3;
+    }
+    return FEMD_OK;
+}
+
+// One FP64 CG solve (cg.hpp:296-350): on chip where the system fits, else on the matrix's workspace.
 static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double *x, int max_iter, double tol,
                   femd_cg_result *res)
 {
     femd_pattern P = K->pattern;
     const int n = P->nrows;
     cudaStream_t s = ctx->stream;
+    ResidentPlan plan;
+    if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+        const size_t need = (size_t)n + 1 + RES_SLOT_DOUBLES + RES_OUT_DOUBLES;
+        if (ctx->res_scratch.n < need) FEMD_TRY(ctx->res_scratch.alloc(need + need / 4));
+        double *slots = ctx->res_scratch.p, *out = slots + RES_SLOT_DOUBLES;
+        bool ran = false;
+        FEMD_TRY(cg_resident(ctx, K, jac, b, x, max_iter, tol, plan, out + RES_OUT_DOUBLES, slots,
+                             reinterpret_cast<ResidentOut *>(out), true, &ran, res));
+        if (ran) return FEMD_OK;
+    }
     SolverWS *Wp = nullptr;
     FEMD_TRY(get_ws(ctx, K, &Wp));
     SolverWS &W = *Wp;
@@ -782,15 +850,8 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
         if (S.nb == 0.0) {
             cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), s);
             cudaStreamSynchronize(s);
-            res->converged = 1; res->iterations = 0; res->residual = 0.0; res->breakdown = 0;
-        } else {
-            res->iterations = S.it;
-            res->breakdown = S.breakdown;
-            res->residual = S.res64 / S.nb;
-            int conv = !S.breakdown && res->residual <= tol * (1.0 + 1e-6) + 1e-15;
-            if (!conv && !S.breakdown && res->residual <= 10.0 * tol && S.it < max_iter) conv = 1;
-            res->converged = conv;
         }
+        cg_result(S.nb, S.res64, S.it, S.breakdown, max_iter, tol, res);
         res->status = FEMD_OK;
         res->outer = 0;
         float ms = 0.f;
@@ -1621,6 +1682,15 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     double *part = base + 3 * (size_t)NOALLOC_MAX_ROWS;
     CGState<double> *st = reinterpret_cast<CGState<double> *>(part + NOALLOC_PART);
     cudaStream_t s = ctx->stream;
+    static_assert(sizeof(ResidentOut) <= sizeof(CGState<double>) && RES_SLOT_DOUBLES <= (size_t)NOALLOC_PART,
+                  "the on-chip solve's scratch fits the fixed array");
+    ResidentPlan plan;
+    if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+        bool ran = false;
+        FEMD_TRY(cg_resident(ctx, K, jac, b_dev, x_dev, max_iter, tol, plan, r, part, reinterpret_cast<ResidentOut *>(st),
+                             false, &ran, res));
+        if (ran) return FEMD_OK;
+    }
     // the array keeps the previous call's contents: the state (with its reduction ticket) must
     // start at zero; r, p, Ap and the partials are written before they are read
     FEMD_TRY_CUDA(cudaMemsetAsync(st, 0, sizeof(CGState<double>), s));
@@ -1657,14 +1727,8 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     if (S.nb == 0.0) {
         FEMD_TRY_CUDA(cudaMemsetAsync(x_dev, 0, (size_t)n * sizeof(double), s));
         FEMD_TRY_CUDA(cudaStreamSynchronize(s));
-        return FEMD_OK;
     }
-    res->iterations = S.it;
-    res->breakdown = S.breakdown;
-    res->residual = S.res64 / S.nb;
-    int conv = !S.breakdown && res->residual <= tol * (1.0 + 1e-6) + 1e-15;
-    if (!conv && !S.breakdown && res->residual <= 10.0 * tol && S.it < max_iter) conv = 1;
-    res->converged = conv;
+    cg_result(S.nb, S.res64, S.it, S.breakdown, max_iter, tol, res);
     return FEMD_OK;
 }
 
