@@ -5,22 +5,24 @@
 // the finished rows k < i of its lower part) and the triangular solves of every application.  Row
 // i depends only on the rows its lower (forward) or upper (backward) part names, so the rows fall
 // into levels -- level(i) = 1 + the largest level among them -- and the rows of one level are
-// independent.  The level schedules are built once per pattern on the host.  Each sweep then runs
-// as ONE thread block that walks the levels in order with a block barrier between them: a thread
-// takes a row and does that row's arithmetic exactly as the reference writes it (the same
-// operations in the same order, no contraction), so the factors and every application are
-// bit-identical to the reference's; only the order in which independent rows are done differs.
-// No block waits on another, so nothing can hang.
+// independent.  The level schedules are built once per pattern on the host.  The factorization and
+// each application then run as ONE thread block that walks the levels in order with a block barrier
+// between them: a thread takes a row and does that row's arithmetic exactly as the reference
+// writes it (the same operations in the same order, no contraction), so the factors and every
+// application are bit-identical to the reference's; only the order in which independent rows are
+// done differs.  No block waits on another, so nothing can hang.
 //
-// The price is parallelism: one SM per sweep, latency-bound by the number of levels (about 4 N
-// for P2 on an N x N rectangle).  The reference's natural-order ILU(0) has no more parallelism to
-// give; a faster preconditioner would be a different one (another ordering), with other iterates.
+// The price is parallelism: one SM per application, latency-bound by the number of levels (about
+// 4 N for P2 on an N x N rectangle, each way).  The reference's natural-order ILU(0) has no more
+// parallelism to give; a faster preconditioner would be a different one (another ordering), with
+// other iterates.
 #include <algorithm>
 #include <climits>
 #include <cmath>
 #include <limits>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -31,9 +33,12 @@ struct femd_precond_s : femd::HandleBase {
     int pc_kind = 0;                     // FEMD_PC_ILU0 / FEMD_PC_SSOR
     double omega = 1.0, min_pivot = 0.0;
     int n = 0, nlf = 0, nlb = 0;
-    femd::DevBuf<double> v;              // ILU(0): the factors L (unit, strict lower) and U; SSOR: the values
-    femd::DevBuf<int> diag;              // position of (i, i)
-    femd::DevBuf<int> frows, fptr, brows, bptr;   // rows by forward / backward level
+    // the sweeps' chunks, one per forward and backward level in order (k_pc_apply), their places and
+    // sizes, and the launch
+    femd::DevBuf<uint4> chunks;
+    femd::DevBuf<int2> places;
+    int threads = 0, slot = 0, zs = 0, ring = 0;
+    size_t smem = 0;
     femd_precond_s() : HandleBase(femd::KIND_PRECOND) {}
     ~femd_precond_s() override { femd::ctx_release(ctx); }
 };
@@ -71,57 +76,299 @@ __global__ void __launch_bounds__(PC_BLOCK) k_ilu0_factor(const int *__restrict_
     }
 }
 
-// forward sweep: ILU(0) z_i = r_i - sum_{p < d_i} v_p z_col (precond.hpp:193-198); SSOR
-// z_i = (r_i - sum ...) w / v_ii (:127-132)
-template <bool SSOR>
-__global__ void __launch_bounds__(PC_BLOCK) k_pc_forward(const int *__restrict__ ip, const int *__restrict__ ix,
-                                                        const int *__restrict__ diag, const double *__restrict__ v, int nl,
-                                                        const int *__restrict__ lptr, const int *__restrict__ rows,
-                                                        double w, const double *__restrict__ r, double *__restrict__ z,
-                                                        const int *__restrict__ skip)
+// ---- an application: the forward and the backward sweep, level by level ------------------------
+// What bounds it is the chain of one level, most of all the instructions one warp issues in it: the
+// barrier, the gathers of z, the row's subtractions in order (and in the backward sweep a
+// division), the store of z.  So everything that does not depend on z is brought near beforehand:
+// the levels' rows are packed into chunks in the order of the sweeps, a warp of its own has
+// them copied into a ring of shared memory 8 or 4 levels ahead (bulk copies; the block's barrier of a
+// level also hands them over), a row's first entries are in registers before the barrier that
+// frees it, and z itself lies in shared memory (ZS) while it fits; all of it at 32-bit places in
+// shared memory with constant strides.  One application at P2 64 x 64 (16,129 rows, 254 + 254
+// levels): 935 us with rows read from CSR through the level lists by two launches, 272 here; of
+// that the division takes 6 %, the subtractions 20 %, loading the next level's rows 24 %.
+//
+// A chunk that no slot holds (the inner nodes of all cells at P3 are one level) is read where it lies.
+//
+// Chunk: int4 {its rows, the next chunk's rows, the next chunk's place (in 16 B) where it is read
+// there or -1, 0};
+// a PcRow per row; values double x E; columns int x E.  A chunk's rows are sorted by length and lie
+// in slices of PC_SLICE rows, two values or four columns of a row side by side (16-byte loads, a
+// slice's 128 B together).  The 32 rows of a warp are filled up to the same number of entries, a
+// multiple of 4, with the value +0 on column n, whose z is +0: s - (+0 * +0) is s, bit for bit, so
+// no lane needs a test in the chain.  With z in shared memory a column is its place there in bytes.
+static constexpr int PC_AHEAD = 8, PC_SLICE = 8;
+static constexpr int PC_ROWS = 256, PC_COPY = 32;    // threads that take rows (at most), and that copy
+static constexpr size_t PC_SMEM = 220 * 1024;
+
+struct __align__(16) PcRow {
+    int row, len, val, col;              // len: filled up; bytes from the chunk's start to the first value and column
+    double diag, pad;
+};
+
+__host__ __device__ inline size_t pc_chunk_bytes(int m, int E)
 {
-    if (skip && *skip) return;
-    for (int L = 0; L < nl; ++L) {
-        for (int t = lptr[L] + (int)threadIdx.x; t < lptr[L + 1]; t += PC_BLOCK) {
-            const int i = rows[t];
-            double s = r[i];
-            const int di = diag[i];
-            for (int p = ip[i]; p < di; ++p) s = __dsub_rn(s, __dmul_rn(v[p], z[ix[p]]));
-            z[i] = SSOR ? __ddiv_rn(__dmul_rn(s, w), v[di]) : s;
+    return 16 + sizeof(PcRow) * (size_t)m + 12 * (size_t)E;   // E: a multiple of 4 PC_SLICE
+}
+
+// Fill the chunks: one thread per row in level order (rows; lptr: the levels' first).
+__global__ void k_pc_pack(const int *__restrict__ ip, const int *__restrict__ ix, const int *__restrict__ diag,
+                          const double *__restrict__ v, const int *__restrict__ rows, const int *__restrict__ lptr, int nl,
+                          const int *__restrict__ eoff, const int *__restrict__ etot, const int *__restrict__ place,
+                          const int *__restrict__ next_m, int l0, int nchunk, int slot, int n, bool forward, bool zs, char *__restrict__ chunks)
+{
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        int lo = 0, hi = nl - 1;                             // the level of t
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (lptr[mid] <= t) lo = mid; else hi = mid - 1;
         }
-        __syncthreads();
+        const int first = lptr[lo], m = lptr[lo + 1] - first, u = t - first, c = l0 + lo, E = etot[c];
+        char *base = chunks + 16 * (size_t)place[c];
+        if (u == 0)
+            *reinterpret_cast<int4 *>(base) =
+                make_int4(m, next_m[c], c + 1 < nchunk && 16ll * (place[c + 2] - place[c + 1]) > slot ? place[c + 1] : -1, 0);
+        const int i = rows[t], d = diag[i];
+        const int q0 = forward ? ip[i] : d + 1, len = forward ? d - q0 : ip[i + 1] - q0;
+        PcRow rec;
+        int most = 0;                                        // of the warp's rows
+        for (int x = u & ~31; x < min(m, (u & ~31) + 32); ++x) {
+            const int k = rows[first + x];
+            most = max(most, forward ? diag[k] - ip[k] : ip[k + 1] - diag[k] - 1);
+        }
+        rec.row = i;
+        rec.len = (most + 3) & ~3;
+        rec.val = 16 + (int)sizeof(PcRow) * m + 8 * eoff[t] + 16 * (u % PC_SLICE);
+        rec.col = 16 + (int)sizeof(PcRow) * m + 8 * E + 4 * eoff[t] + 16 * (u % PC_SLICE);
+        rec.diag = v[d];
+        rec.pad = 0.0;
+        reinterpret_cast<PcRow *>(base + 16)[u] = rec;
+        for (int j = 0; j < rec.len; ++j) {
+            const int k = j < len ? ix[q0 + j] : n;
+            *reinterpret_cast<double *>(base + rec.val + 16 * PC_SLICE * (j / 2) + 8 * (j % 2)) = j < len ? v[q0 + j] : 0.0;
+            *reinterpret_cast<int *>(base + rec.col + 16 * PC_SLICE * (j / 4) + 4 * (j % 4)) = zs ? 8 * k : k;
+        }
     }
 }
 
-// SSOR's middle step, z_i *= c v_ii / w with c = (2 - w) / w (precond.hpp:134-135)
-__global__ void k_ssor_scale(int n, const int *__restrict__ diag, const double *__restrict__ v, double w,
-                             double *__restrict__ z, const int *__restrict__ skip)
+// The ring's copies: one mbarrier a slot, waited on by the copying warp alone.  A wait is bounded.
+static constexpr int PC_SPINS = 1 << 22;
+
+__device__ __forceinline__ void pc_copy(char *dst, const uint4 *src, int n16, uint64_t *bar)
 {
-    if (skip && *skip) return;
-    const double c = __ddiv_rn(__dsub_rn(2.0, w), w);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        z[i] = __dmul_rn(z[i], __ddiv_rn(__dmul_rn(c, v[diag[i]]), w));
+    const unsigned b = (unsigned)__cvta_generic_to_shared(bar), d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(16u * n16) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(d), "l"(src), "r"(16u * n16), "r"(b) : "memory");
 }
 
-// backward sweep: z_i = (z_i - sum_{p > d_i} v_p z_col) / v_ii (ILU(0), :199-204) or * w / v_ii
-// (SSOR, :137-142)
-template <bool SSOR>
-__global__ void __launch_bounds__(PC_BLOCK) k_pc_backward(const int *__restrict__ ip, const int *__restrict__ ix,
-                                                         const int *__restrict__ diag, const double *__restrict__ v, int nl,
-                                                         const int *__restrict__ lptr, const int *__restrict__ rows,
-                                                         double w, double *__restrict__ z, const int *__restrict__ skip)
+__device__ __forceinline__ bool pc_wait(uint64_t *bar, unsigned parity)
 {
-    if (skip && *skip) return;
-    for (int L = 0; L < nl; ++L) {
-        for (int t = lptr[L] + (int)threadIdx.x; t < lptr[L + 1]; t += PC_BLOCK) {
-            const int i = rows[t];
-            const int di = diag[i];
-            double s = z[i];
-            for (int p = di + 1; p < ip[i + 1]; ++p) s = __dsub_rn(s, __dmul_rn(v[p], z[ix[p]]));
-            z[i] = SSOR ? __ddiv_rn(__dmul_rn(s, w), v[di]) : __ddiv_rn(s, v[di]);
-        }
-        __syncthreads();
+    for (int spin = 0; spin < PC_SPINS; ++spin) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+        if (ok) return true;
     }
+    return false;
+}
+
+// z = M^{-1} r.  ILU(0): z_i = r_i - sum_{p < d_i} v_p z_col, then z_i = (z_i - sum_{p > d_i} v_p
+// z_col) / v_ii (precond.hpp:193-204).  SSOR: (r_i - sum) w / v_ii; z_i c v_ii / w with c = (2 -
+// w) / w; (z_i - sum) w / v_ii (:127-142).  ZS: z in shared memory; RING: the ring's slots; places: the
+// chunks' places and sizes in 16 B (size 0: read where it lies).
+template <bool SSOR, bool ZS, int RING>
+__global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__restrict__ chunks, const int2 *__restrict__ places, int nlf,
+                                                      int nl, int slot, int n, double w, const double *__restrict__ r,
+                                                      double *z, const int *__restrict__ skip)
+{
+    extern __shared__ __align__(16) char dyn[];
+    if (skip && *skip) return;
+    // shared memory: z (ZS), then the ring; places are 32-bit
+    const unsigned ring0 = ZS ? ((unsigned)n * 8u + 23u) / 16u * 16u : 0u;   // z and its +0
+    const unsigned dyn0 = (unsigned)__cvta_generic_to_shared(dyn);
+    auto z_at = [&](int i) -> double & { return ZS ? reinterpret_cast<double *>(dyn)[i] : z[i]; };
+    const int tid = threadIdx.x, T = blockDim.x - PC_COPY;   // threads that take rows
+    const double c = SSOR ? __ddiv_rn(__dsub_rn(2.0, w), w) : 0.0;
+    if (ZS) {
+        constexpr int U = 8;                                 // loads in flight
+        for (int i0 = tid; i0 < n; i0 += U * blockDim.x) {
+            double t[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) t[u] = i0 + u * blockDim.x < n ? r[i0 + u * blockDim.x] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * blockDim.x < n) z_at(i0 + u * blockDim.x) = t[u];
+        }
+        if (tid == 0) z_at(n) = 0.0;
+    }
+    __shared__ uint64_t bar[RING];
+    __shared__ int s_late;                                   // a copy did not arrive: z is given back as NaN
+    if (tid >= T) {
+        // the copying warp: chunk L + 2 is in when level L ends (its threads then load from it)
+        const bool lead = tid == T;
+        int issued = 0, arrived = 0;
+        bool late = false;
+        // chunk k into its slot; one that no slot holds only counts as arrived
+        auto issue = [&](int2 c) {
+            if (c.y) pc_copy(dyn + ring0 + issued % RING * slot, chunks + c.x, c.y, &bar[issued % RING]);
+            else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"((unsigned)__cvta_generic_to_shared(&bar[issued % RING])) : "memory");
+            ++issued;
+        };
+        int2 next = make_int2(0, 0);                         // the chunk issued after the next barrier
+        if (lead) {
+            s_late = 0;
+            for (int k = 0; k < RING; ++k)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((unsigned)__cvta_generic_to_shared(&bar[k])) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            while (issued < RING && issued < nl) issue(places[issued]);
+            if (issued < nl) next = places[issued];
+        }
+        for (int L = -1; L < nl; ++L) {
+            if (lead) {
+                for (; arrived < min(L + 3, issued) && !late; ++arrived)
+                    late = !pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u);
+                if (late) s_late = 1;
+            }
+            __syncwarp();
+            __syncthreads();                                 // the level's rows are final, its slot is free
+            if (lead && L >= 0 && issued < nl && !late) {
+                issue(next);
+                if (issued < nl) next = places[issued];
+            }
+        }
+        if (lead && late)                                    // leave no copy in flight
+            for (; arrived < issued; ++arrived) pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u);
+        __syncwarp();
+    } else {
+        __syncthreads();
+        unsigned place = dyn0 + ring0;                       // of the level's chunk in the ring
+        const char *chunk = nullptr;                         // or where it lies (AT)
+        auto get4 = [&](auto AT, int o) {
+            int4 t;
+            if (AT) t = *reinterpret_cast<const int4 *>(chunk + o);
+            else asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w) : "r"(place + o));
+            return t;
+        };
+        auto get2 = [&](auto AT, int o) {
+            double2 t;
+            if (AT) t = *reinterpret_cast<const double2 *>(chunk + o);
+            else asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(place + o));
+            return t;
+        };
+        auto z_get = [&](int col) {                          // col as the chunk has it
+            double t;
+            if (ZS) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(t) : "r"(dyn0 + col));
+            else t = col < n ? z[col] : 0.0;
+            return t;
+        };
+        // a row's record and first entries
+        int4 me = make_int4(0, 0, 0, 0), col[PC_AHEAD / 4];
+        double2 v[PC_AHEAD / 2];
+        double dg = 1.0;
+        bool have = false;
+        auto load = [&](auto AT, int u, int m) {
+            have = u < m;
+            if (!have) return;
+            me = get4(AT, 16 + 32 * u);
+            dg = get2(AT, 32 + 32 * u).x;
+#pragma unroll
+            for (int h = 0; h < PC_AHEAD / 4; ++h)
+                if (4 * h < me.y) {
+                    col[h] = get4(AT, me.w + 16 * PC_SLICE * h);
+                    v[2 * h] = get2(AT, me.z + 32 * PC_SLICE * h);
+                    v[2 * h + 1] = get2(AT, me.z + 32 * PC_SLICE * h + 16 * PC_SLICE);
+                }
+        };
+        auto subtract4 = [&](double s, const int4 &k, const double2 &a, const double2 &b) {
+            const double g0 = z_get(k.x), g1 = z_get(k.y), g2 = z_get(k.z), g3 = z_get(k.w);
+            s = __dsub_rn(s, __dmul_rn(a.x, g0));
+            s = __dsub_rn(s, __dmul_rn(a.y, g1));
+            s = __dsub_rn(s, __dmul_rn(b.x, g2));
+            return __dsub_rn(s, __dmul_rn(b.y, g3));
+        };
+        auto row = [&](auto AT, auto forward) {
+            if (!have) return;
+            constexpr bool FWD = decltype(forward)::value;
+            double s = !ZS && FWD ? r[me.x] : z_get(ZS ? 8 * me.x : me.x);
+            if (SSOR && !FWD) s = __dmul_rn(s, __ddiv_rn(__dmul_rn(c, dg), w));
+#pragma unroll
+            for (int h = 0; h < PC_AHEAD / 4; ++h)
+                if (4 * h < me.y) s = subtract4(s, col[h], v[2 * h], v[2 * h + 1]);
+            if (PC_AHEAD < me.y) {
+                // the rest: the next four are loaded while these are subtracted
+                int ov = me.z + 8 * PC_SLICE * PC_AHEAD, oc = me.w + 4 * PC_SLICE * PC_AHEAD;
+                int4 k = get4(AT, oc);
+                double2 a = get2(AT, ov), b = get2(AT, ov + 16 * PC_SLICE);
+                for (int left = me.y - PC_AHEAD - 4; left >= 0; left -= 4) {
+                    const int4 kk = k;
+                    const double2 aa = a, bb = b;
+                    if (left > 0) {
+                        oc += 16 * PC_SLICE;
+                        ov += 32 * PC_SLICE;
+                        k = get4(AT, oc);
+                        a = get2(AT, ov);
+                        b = get2(AT, ov + 16 * PC_SLICE);
+                    }
+                    s = subtract4(s, kk, aa, bb);
+                }
+            }
+            if (SSOR) s = __ddiv_rn(__dmul_rn(s, w), dg);
+            else if (!FWD) s = __ddiv_rn(s, dg);
+            if (ZS) asm volatile("st.shared.f64 [%0], %1;" :: "r"(dyn0 + 8 * me.x), "d"(s) : "memory");
+            else z[me.x] = s;
+        };
+        const std::true_type lies{};
+        const std::false_type ringed{};
+        // rows of this level and the next, and whether this level is read where it lies
+        int4 head = make_int4(0, 0, -1, 0);
+        bool at = places[0].y == 0;
+        if (at) chunk = reinterpret_cast<const char *>(chunks + places[0].x);
+        else {
+            head = get4(ringed, 0);
+            load(ringed, tid, head.x);
+        }
+        auto levels = [&](auto forward, int L0, int L1) {
+            for (int L = L0; L < L1; ++L) {
+                if (at) {
+                    head = get4(lies, 0);
+                    for (int u = tid; u < head.x; u += T) {
+                        load(lies, u, head.x);
+                        row(lies, forward);
+                    }
+                } else {
+                    row(ringed, forward);
+                    for (int u = tid + T; u < head.x; u += T) {
+                        load(ringed, u, head.x);
+                        row(ringed, forward);
+                    }
+                }
+                // the next level's rows: its chunk was handed over by the last barrier
+                place = (L + 1) % RING ? place + slot : dyn0 + ring0;
+                at = head.z >= 0;
+                if (at) chunk = reinterpret_cast<const char *>(chunks + head.z);
+                else if (L + 1 < nl) {
+                    load(ringed, tid, head.y);
+                    head = get4(ringed, 0);
+                }
+                __syncthreads();                             // the level's rows are final
+            }
+        };
+        levels(std::true_type(), 0, nlf);
+        levels(std::false_type(), nlf, nl);
+    }
+    const bool late = s_late;
+    if (ZS || late)
+        for (int i = tid; i < n; i += blockDim.x) z[i] = late ? __longlong_as_double(0x7ff8000000000000ll) : z_at(i);
+}
+
+using PcKernel = void (*)(const uint4 *, const int2 *, int, int, int, int, double, const double *, double *, const int *);
+
+template <bool SSOR>
+static PcKernel pc_kernel(bool zs, int ring)
+{
+    if (zs) return ring == 8 ? k_pc_apply<SSOR, true, 8> : k_pc_apply<SSOR, true, 4>;
+    return ring == 8 ? k_pc_apply<SSOR, false, 8> : k_pc_apply<SSOR, false, 4>;
 }
 
 __global__ void k_pc_min_diag(int n, const int *__restrict__ diag, const double *__restrict__ v, double *out)
@@ -164,6 +411,30 @@ static void level_schedule(int n, const std::vector<int> &ip, const std::vector<
     for (int i = 0; i < n; ++i) rows[fill[lev[i]]++] = i;
 }
 
+// The chunks of one sweep's levels: per row (in level order) its first entry, per level its entries;
+// the chunks' sizes are appended to place (in 16 B, running).
+static void chunk_layout(const std::vector<int> &ip, const std::vector<int> &dg, bool forward, std::vector<int> &rows,
+                         const std::vector<int> &ptr, std::vector<int> &eoff, std::vector<int> &etot, std::vector<int> &rtot,
+                         std::vector<long long> &place)
+{
+    const int nl = (int)ptr.size() - 1;
+    auto length = [&](int i) { return forward ? dg[i] - ip[i] : ip[i + 1] - dg[i] - 1; };
+    eoff.assign(rows.size(), 0);
+    for (int l = 0; l < nl; ++l) {
+        std::stable_sort(rows.begin() + ptr[l], rows.begin() + ptr[l + 1], [&](int a, int b) { return length(a) > length(b); });
+        const int m = ptr[l + 1] - ptr[l];
+        int E = 0;
+        for (int u = 0; u < m; u += PC_SLICE) {
+            for (int j = 0; j < std::min(PC_SLICE, m - u); ++j) eoff[ptr[l] + u + j] = E;
+            E += PC_SLICE * ((length(rows[ptr[l] + (u & ~31)]) + 3) & ~3);
+        }
+        etot.push_back(E);
+        rtot.push_back(m);
+        const size_t bytes = pc_chunk_bytes(m, E);
+        place.push_back(place.back() + (long long)(bytes / 16));
+    }
+}
+
 static femd_precond_s *as_precond(void *h)
 {
     femd_precond_s *p = static_cast<femd_precond_s *>(h);
@@ -173,21 +444,10 @@ static femd_precond_s *as_precond(void *h)
 // z = M^{-1} r on the stream, every kernel skipped when *skip is set (a finished CG loop)
 int precond_enqueue(femd_precond P, const double *r, double *z, const int *skip, cudaStream_t s)
 {
-    femd_pattern Q = P->pattern;
-    const int *ip = Q->indptr.p, *ix = Q->indices.p;
     if (P->n == 0) return FEMD_OK;
-    if (P->pc_kind == FEMD_PC_ILU0) {
-        k_pc_forward<false><<<1, PC_BLOCK, 0, counted(s)>>>(ip, ix, P->diag.p, P->v.p, P->nlf, P->fptr.p, P->frows.p, 1.0, r, z,
-                                                           skip);
-        k_pc_backward<false><<<1, PC_BLOCK, 0, counted(s)>>>(ip, ix, P->diag.p, P->v.p, P->nlb, P->bptr.p, P->brows.p, 1.0, z,
-                                                            skip);
-    } else {
-        k_pc_forward<true><<<1, PC_BLOCK, 0, counted(s)>>>(ip, ix, P->diag.p, P->v.p, P->nlf, P->fptr.p, P->frows.p, P->omega,
-                                                          r, z, skip);
-        k_ssor_scale<<<grid_for((size_t)P->n, 256, 1u << 16), 256, 0, counted(s)>>>(P->n, P->diag.p, P->v.p, P->omega, z, skip);
-        k_pc_backward<true><<<1, PC_BLOCK, 0, counted(s)>>>(ip, ix, P->diag.p, P->v.p, P->nlb, P->bptr.p, P->brows.p,
-                                                           P->omega, z, skip);
-    }
+    PcKernel k = P->pc_kind == FEMD_PC_ILU0 ? pc_kernel<false>(P->zs, P->ring) : pc_kernel<true>(P->zs, P->ring);
+    FEMD_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC_SMEM));
+    k<<<1, P->threads, P->smem, counted(s)>>>(P->chunks.p, P->places.p, P->nlf, P->nlf + P->nlb, P->slot, P->n, P->omega, r, z, skip);
     FEMD_TRY_CUDA(cudaGetLastError());
     return FEMD_OK;
 }
@@ -245,23 +505,61 @@ int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, double omega
     level_schedule(n, ip, ix, dg, false, br, bp);
     P->nlf = (int)fp.size() - 1;
     P->nlb = (int)bp.size() - 1;
-    int st;
-    if ((st = P->v.alloc((size_t)std::max<long long>(nnz, 1))) || (st = P->diag.alloc((size_t)std::max(n, 1))) ||
-        (st = P->frows.alloc((size_t)std::max(n, 1))) || (st = P->fptr.alloc(fp.size())) ||
-        (st = P->brows.alloc((size_t)std::max(n, 1))) || (st = P->bptr.alloc(bp.size())))
-        return st;
-    if (nnz) FEMD_TRY_CUDA(cudaMemcpyAsync(P->v.p, K->data.p, (size_t)nnz * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (n) {
-        FEMD_TRY_CUDA(cudaMemcpyAsync(P->diag.p, dg.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, s));
-        FEMD_TRY_CUDA(cudaMemcpyAsync(P->frows.p, fr.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, s));
-        FEMD_TRY_CUDA(cudaMemcpyAsync(P->brows.p, br.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, s));
+    std::vector<int> feoff, beoff, etot, rtot;
+    std::vector<long long> pl(1, 0);
+    chunk_layout(ip, dg, true, fr, fp, feoff, etot, rtot, pl);
+    chunk_layout(ip, dg, false, br, bp, beoff, etot, rtot, pl);
+    FEMD_CHECK_ARG(pl.back() < INT_MAX, std::string(what) + ": the matrix is too large");
+    std::vector<int> place(pl.begin(), pl.end());
+    const int nch = P->nlf + P->nlb;
+    rtot.push_back(0);                   // the chunk after the last
+    // A thread per row of most levels, in whole warps, at most PC_ROWS.  z in shared memory where it
+    // fits beside four slots for nearly all chunks (P2: up to about 20,000 rows), else slots alone.
+    std::vector<int> sizes((size_t)nch), widths(rtot.begin(), rtot.end() - 1);
+    for (int k = 0; k < nch; ++k) sizes[k] = 16 * (place[k + 1] - place[k]);
+    std::sort(sizes.begin(), sizes.end());
+    std::sort(widths.begin(), widths.end());
+    const int usual = nch ? sizes[(size_t)(nch - 1) * 49 / 50] : 16, width = nch ? widths[(size_t)(nch - 1) * 49 / 50] : 1;
+    P->threads = std::min(PC_ROWS, std::max(64, (width + 31) / 32 * 32)) + PC_COPY;
+    const size_t zbytes = ((size_t)n * sizeof(double) + 23) / 16 * 16;
+    P->zs = zbytes + 4 * (size_t)usual <= PC_SMEM;
+    const size_t room = PC_SMEM - (P->zs ? zbytes : 0);
+    P->ring = 8 * (size_t)usual <= room ? 8 : 4;
+    P->slot = 16;
+    for (int b : sizes)
+        if ((size_t)b * P->ring <= room) P->slot = std::max(P->slot, b);
+    P->smem = (size_t)P->ring * P->slot + (P->zs ? zbytes : 0);
+    std::vector<int2> first((size_t)std::max(nch, 1));
+    for (int k = 0; k < nch; ++k) {
+        const int size = place[k + 1] - place[k];
+        first[k] = make_int2(place[k], 16ll * size <= P->slot ? size : 0);
     }
-    FEMD_TRY_CUDA(cudaMemcpyAsync(P->fptr.p, fp.data(), fp.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    FEMD_TRY_CUDA(cudaMemcpyAsync(P->bptr.p, bp.data(), bp.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    DevBuf<double> v;                    // ILU(0): the factors L (unit, strict lower) and U; SSOR: the values
+    DevBuf<int> diag, frows, fptr, brows, bptr, fe, be, et, rt, plc;
+    int st;
+    if ((st = v.alloc((size_t)std::max<long long>(nnz, 1))) || (st = diag.alloc((size_t)std::max(n, 1))) ||
+        (st = frows.alloc((size_t)std::max(n, 1))) || (st = fptr.alloc(fp.size())) ||
+        (st = brows.alloc((size_t)std::max(n, 1))) || (st = bptr.alloc(bp.size())) || (st = fe.alloc(feoff.size() + 1)) ||
+        (st = be.alloc(beoff.size() + 1)) || (st = et.alloc(etot.size() + 1)) || (st = rt.alloc(rtot.size())) ||
+        (st = plc.alloc(place.size())) || (st = P->chunks.alloc((size_t)pl.back() + 1)) || (st = P->places.alloc(first.size())))
+        return st;
+    auto up = [&](void *d, const void *h, size_t bytes) { return bytes ? cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess; };
+    if (nnz) FEMD_TRY_CUDA(cudaMemcpyAsync(v.p, K->data.p, (size_t)nnz * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    FEMD_TRY_CUDA(up(diag.p, dg.data(), (size_t)n * sizeof(int)));
+    FEMD_TRY_CUDA(up(frows.p, fr.data(), (size_t)n * sizeof(int)));
+    FEMD_TRY_CUDA(up(brows.p, br.data(), (size_t)n * sizeof(int)));
+    FEMD_TRY_CUDA(up(fptr.p, fp.data(), fp.size() * sizeof(int)));
+    FEMD_TRY_CUDA(up(bptr.p, bp.data(), bp.size() * sizeof(int)));
+    FEMD_TRY_CUDA(up(fe.p, feoff.data(), (size_t)n * sizeof(int)));
+    FEMD_TRY_CUDA(up(be.p, beoff.data(), (size_t)n * sizeof(int)));
+    FEMD_TRY_CUDA(up(et.p, etot.data(), etot.size() * sizeof(int)));
+    FEMD_TRY_CUDA(up(rt.p, rtot.data(), rtot.size() * sizeof(int)));
+    FEMD_TRY_CUDA(up(plc.p, place.data(), place.size() * sizeof(int)));
+    FEMD_TRY_CUDA(up(P->places.p, first.data(), first.size() * sizeof(int2)));
     if (kind == FEMD_PC_ILU0 && n) {
         FEMD_TRY(reset_status(ctx));
         // status [1] holds the first row with a zero pivot (INT_MAX: none)
-        k_ilu0_factor<<<1, PC_BLOCK, 0, counted(s)>>>(Q->indptr.p, Q->indices.p, P->diag.p, P->v.p, P->nlf, P->fptr.p, P->frows.p,
+        k_ilu0_factor<<<1, PC_BLOCK, 0, counted(s)>>>(Q->indptr.p, Q->indices.p, diag.p, v.p, P->nlf, fptr.p, frows.p,
                                                        ctx->status_dev + 1);
         FEMD_TRY_CUDA(cudaGetLastError());
         int flags = 0, bad = 0;
@@ -272,9 +570,19 @@ int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, double omega
         }
         DevBuf<double> mp;
         FEMD_TRY(mp.alloc(1));
-        k_pc_min_diag<<<1, 1024, 0, counted(s)>>>(n, P->diag.p, P->v.p, mp.p);
+        k_pc_min_diag<<<1, 1024, 0, counted(s)>>>(n, diag.p, v.p, mp.p);
         FEMD_TRY_CUDA(cudaGetLastError());
         FEMD_TRY_CUDA(cudaMemcpyAsync(&P->min_pivot, mp.p, sizeof(double), cudaMemcpyDeviceToHost, s));
+        FEMD_TRY_CUDA(cudaStreamSynchronize(s));   // mp is released here
+    }
+    if (n) {
+        const unsigned grid = grid_for((size_t)n, 128, 1u << 16);
+        char *dst = reinterpret_cast<char *>(P->chunks.p);
+        k_pc_pack<<<grid, 128, 0, counted(s)>>>(Q->indptr.p, Q->indices.p, diag.p, v.p, frows.p, fptr.p, P->nlf, fe.p, et.p, plc.p,
+                                                rt.p + 1, 0, nch, P->slot, n, true, P->zs, dst);
+        k_pc_pack<<<grid, 128, 0, counted(s)>>>(Q->indptr.p, Q->indices.p, diag.p, v.p, brows.p, bptr.p, P->nlb, be.p, et.p, plc.p,
+                                                rt.p + 1, P->nlf, nch, P->slot, n, false, P->zs, dst);
+        FEMD_TRY_CUDA(cudaGetLastError());
     }
     FEMD_TRY_CUDA(cudaStreamSynchronize(s));   // the host vectors are released on return
     *out = reinterpret_cast<femd_precond>(guard.release());
