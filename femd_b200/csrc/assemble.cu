@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(256) k_assemble_vector(
 //   H_{q,rs} = rw_q |det J| sum_{t varying} c_t(q) A[a_t][r] A[b_t][s]   (coefficients at points)
 // and the reference tensors S^{rs}(l, j) = sum_q rw_q R_r(q,l) R_s(q,j) computed on the host.
 // K3a forms F and H once per cell (evaluating closed-form and field coefficients there), K3b
-// walks each row's cells in increasing order and adds the entries in shared memory.
+// walks each row's cells in increasing order and adds the entries in shared memory.  H is for P4 and
+// higher; up to P3 a form with varying coefficients takes element matrices (below).
 static constexpr int MAX_PAIRS = 9;
 static constexpr int FAST_BLOCK = 128;
 
@@ -306,6 +307,8 @@ struct FastSpec {
     int psym[MAX_PAIRS];                      // pair k stands for (r, s) and (s, r) of a symmetric form
     int has_const, has_var, nf;               // factors per cell: npair (const) + nq npair (varying)
     int vector;
+    int ncof, cof[MAX_TERMS], cof_term[MAX_TERMS];   // distinct coefficients, each term's, a term of each
+    int rows, cols;                           // bits r (s): a term takes reference row r of the test (s of the trial) side
     // the constant terms folded per pair onto the 15 monomials of degree <= 2 in J^-1 (1, Ji0..3,
     // Ji_a Ji_b with a <= b): F_k = |det J| sum_m cm[k][m] mono_m (filled by fast_spec)
     double cm[MAX_PAIRS][15];
@@ -340,6 +343,233 @@ __device__ __forceinline__ double coef_at(const FastSpec &fs, int t, int e, int 
         return s;
     }
     default: return fs.cval[t];
+    }
+}
+
+// ---- forms with coefficients at the points, and every linear form: element tensors -------------
+// One thread per cell evaluates every distinct coefficient once at each point and contracts it
+// with the tabulation into the element vector (k_elem_vector) or matrix (k_elem_matrix), which the
+// rows' owners then only gather and add in increasing cell order.  Before, a cell's factors at all
+// points went to HBM and every row of the cell read and contracted them again: 1024^2 P2 load of a
+// closed form 142 + 186 us, 512^2 P2 matrix of one 153 + 321 us (P3, 300^2: 261 + 641); now 121 + 55
+// us and 104 + 100 us (235 + 95).
+//
+// What bounds the element kernels is the instructions of two double-precision sines a point (load:
+// 29 M sines, 61 % of the issue slots) and, for a matrix, NLOC (2 NLOC + 4) multiply-adds a point
+// at the occupancy their accumulators leave: 3 rows of a P2 matrix at a time 104 us, 2 rows 111, 6
+// rows 110; P3 5 rows 329, 2 rows 235.  The gathers move 8 nloc (8 nloc^2) bytes a cell twice.
+//
+// g[k] = sum over the coefficient's terms of A[a][r_k] (B[b][s_k]): the terms' derivatives in
+// reference directions, once per cell.
+struct CellGeo {
+    double x0, y0, J0, J1, J2, J3, ad, Ji0, Ji1, Ji2, Ji3;
+};
+
+__device__ __forceinline__ CellGeo cell_geo(const double *__restrict__ pts, const int *__restrict__ tris, int e)
+{
+    const int v0 = tris[3 * e], v1 = tris[3 * e + 1], v2 = tris[3 * e + 2];
+    const double2 p0 = make_double2(pts[2 * v0], pts[2 * v0 + 1]), p1 = make_double2(pts[2 * v1], pts[2 * v1 + 1]),
+                  p2 = make_double2(pts[2 * v2], pts[2 * v2 + 1]);
+    CellGeo g;
+    g.x0 = p0.x;
+    g.y0 = p0.y;
+    g.J0 = p1.x - p0.x;
+    g.J1 = p2.x - p0.x;
+    g.J2 = p1.y - p0.y;
+    g.J3 = p2.y - p0.y;
+    const double d = g.J0 * g.J3 - g.J1 * g.J2, rd = 1.0 / d;
+    g.ad = fabs(d);
+    g.Ji0 = g.J3 * rd;
+    g.Ji1 = -g.J1 * rd;
+    g.Ji2 = -g.J2 * rd;
+    g.Ji3 = g.J0 * rd;
+    return g;
+}
+
+// sum over the terms t with coefficient u of A[a_t][r] (and B[b_t][s])
+__device__ __forceinline__ double fold_terms(const FastSpec &fs, int u, int r, int s, const CellGeo &g)
+{
+    double v = 0.0;
+    for (int t = 0; t < fs.nterms; ++t)
+        if (fs.cof[t] == u)
+            v += amat(fs.a[t], r, g.Ji0, g.Ji1, g.Ji2, g.Ji3) * (fs.vector ? 1.0 : amat(fs.b[t], s, g.Ji0, g.Ji1, g.Ji2, g.Ji3));
+    return v;
+}
+
+// body(q, value of term t's coefficient at point q of cell e): the kind is told once, not per point
+template <class Body>
+__device__ __forceinline__ void each_point(const FastSpec &fs, int t, int e, int nq, const CellGeo &g, const double *qxi,
+                                           const double *qeta, const int *__restrict__ dofs, int nloc, const double *ref,
+                                           Body body)
+{
+    const int kind = fs.kind[t];
+    if (kind == FEMD_COEF_SINSIN || kind == FEMD_COEF_SINSIN_HELM) {
+        const bool helm = kind == FEMD_COEF_SINSIN_HELM;
+        const double p0 = fs.p[t][0], p1 = fs.p[t][1], p2 = fs.p[t][2], p3 = fs.p[t][3];
+        for (int q = 0; q < nq; ++q) {
+            const double x = g.x0 + g.J0 * qxi[q] + g.J1 * qeta[q], y = g.y0 + g.J2 * qxi[q] + g.J3 * qeta[q];
+            const double s = sin(p2 * x) * sin(p3 * y);
+            body(q, helm ? p1 * s + s : p0 + p1 * s);
+        }
+    } else if (kind == FEMD_COEF_POINTS) {
+        const double *c = fs.pts[t] + (size_t)e * nq;
+        for (int q = 0; q < nq; ++q) body(q, c[q]);
+    } else if (kind == FEMD_COEF_FIELD) {
+        const double *f = fs.field[t];
+        const int *d = dofs + (size_t)e * nloc;
+        for (int q = 0; q < nq; ++q) {
+            double c = 0.0;
+            for (int l = 0; l < nloc; ++l) c += ref[q * 3 * nloc + l] * (d[l] >= 0 ? f[d[l]] : 0.0);
+            body(q, c);
+        }
+    } else {
+        const double c = fs.cval[t];
+        for (int q = 0; q < nq; ++q) body(q, c);
+    }
+}
+
+static constexpr int ELEM_BLOCK = 128;
+
+// tables: rw[nq], xi[nq], eta[nq], ref[nq][3][nloc].  NL >= nloc: the registers' room.
+template <int NL>
+__global__ void __launch_bounds__(ELEM_BLOCK) k_elem_vector(const double *__restrict__ pts, const int *__restrict__ tris, int ne,
+                                                            int nq, int nloc, const int *__restrict__ dofs,
+                                                            const double *__restrict__ tables, FastSpec fs,
+                                                            double *__restrict__ fe)
+{
+    extern __shared__ double smem[];
+    const double *rw = smem, *qxi = smem + nq, *qeta = smem + 2 * nq, *ref = smem + 3 * nq;
+    double *stage = smem + 3 * nq + nq * 3 * nloc;           // the block's element vectors, nloc | 1 apart
+    for (int t = threadIdx.x; t < 3 * nq + nq * 3 * nloc; t += ELEM_BLOCK) smem[t] = tables[t];
+    __syncthreads();
+    for (int e0 = blockIdx.x * ELEM_BLOCK; e0 < ne; e0 += gridDim.x * ELEM_BLOCK) {
+        const int e = min(e0 + (int)threadIdx.x, ne - 1);    // past the last cell: that cell again, not written
+        const CellGeo g = cell_geo(pts, tris, e);
+        double acc[NL];
+#pragma unroll
+        for (int l = 0; l < NL; ++l) acc[l] = 0.0;
+        for (int u = 0; u < fs.ncof; ++u) {
+            const int t = fs.cof_term[u];
+            double gk[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) gk[r] = fold_terms(fs, u, r, 0, g);
+            each_point(fs, t, e, nq, g, qxi, qeta, dofs, nloc, ref, [&](int q, double c) {
+                const double h = rw[q] * g.ad * c;
+                const double *R = ref + q * 3 * nloc;
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    if (fs.rows & (1 << r)) {
+                        const double hr = h * gk[r];
+#pragma unroll
+                        for (int l = 0; l < NL; ++l)
+                            if (l < nloc) acc[l] += hr * R[r * nloc + l];
+                    }
+            });
+        }
+#pragma unroll
+        for (int l = 0; l < NL; ++l)
+            if (l < nloc) stage[threadIdx.x * (nloc | 1) + l] = acc[l];
+        __syncthreads();
+        const int m = min(ELEM_BLOCK, ne - e0) * nloc;
+        for (int i = threadIdx.x; i < m; i += ELEM_BLOCK) fe[(size_t)e0 * nloc + i] = stage[i / nloc * (nloc | 1) + i % nloc];
+        __syncthreads();
+    }
+}
+
+// f_i = the row's element entries, in increasing cell order
+__global__ void __launch_bounds__(256) k_gather_vector(const int *__restrict__ rc_ptr, const int *__restrict__ rc_code, int nrows,
+                                                       const double *__restrict__ fe, double *__restrict__ f)
+{
+    constexpr int U = 4;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += gridDim.x * blockDim.x) {
+        const int c1 = rc_ptr[i + 1];
+        double s = 0.0;
+        for (int c = rc_ptr[i]; c < c1; c += U) {
+            int code[U];
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) code[u] = c + u < c1 ? __ldcs(&rc_code[c + u]) : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = c + u < c1 ? fe[code[u]] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c + u < c1) s += v[u];
+        }
+        f[i] = s;
+    }
+}
+
+// Element matrices, Ke[e][l][j].  A coefficient times w |det J| at the points waits in shared memory
+// (one column per thread); LR rows of Ke at a time in registers, so a tabulated value is read once
+// per point for all of them; they go out through shared memory, since a thread's own rows are 8-byte
+// stores into 32 lines at once (512^2 P2: 158 us that way).
+template <int NLOC, int LR>
+__global__ void __launch_bounds__(ELEM_BLOCK) k_elem_matrix(const double *__restrict__ pts, const int *__restrict__ tris, int ne,
+                                                            int nq, const int *__restrict__ dofs,
+                                                            const double *__restrict__ tables, FastSpec fs,
+                                                            double *__restrict__ Ke)
+{
+    static_assert(NLOC % LR == 0, "whole rows");
+    extern __shared__ double smem[];
+    const int ntab = 3 * nq + nq * 3 * NLOC;
+    const double *rw = smem, *qxi = smem + nq, *qeta = smem + 2 * nq, *ref = smem + 3 * nq;
+    constexpr int C = LR * NLOC, CS = C | 1;
+    double *sh = smem + ntab + threadIdx.x;                  // point q at stride ELEM_BLOCK
+    double *stage = smem + ntab + nq * ELEM_BLOCK;           // LR rows of the block's matrices, CS apart
+    for (int t = threadIdx.x; t < ntab; t += ELEM_BLOCK) smem[t] = tables[t];
+    __syncthreads();
+    const int rows = fs.rows, cols = fs.cols;
+    for (int e0 = blockIdx.x * ELEM_BLOCK; e0 < ne; e0 += gridDim.x * ELEM_BLOCK) {
+        const int e = min(e0 + (int)threadIdx.x, ne - 1), m = min(ELEM_BLOCK, ne - e0) * C;
+        const CellGeo g = cell_geo(pts, tris, e);
+        double *out = Ke + (size_t)e * NLOC * NLOC;
+        for (int u = 0; u < fs.ncof; ++u) {
+            each_point(fs, fs.cof_term[u], e, nq, g, qxi, qeta, dofs, NLOC, ref,
+                       [&](int q, double c) { sh[q * ELEM_BLOCK] = rw[q] * g.ad * c; });
+            double gk[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) gk[k] = (rows & (1 << (k / 3))) && (cols & (1 << (k % 3))) ? fold_terms(fs, u, k / 3, k % 3, g) : 0.0;
+            for (int l0 = 0; l0 < NLOC; l0 += LR) {
+                double acc[LR][NLOC];
+#pragma unroll
+                for (int l = 0; l < LR; ++l)
+#pragma unroll
+                    for (int j = 0; j < NLOC; ++j) acc[l][j] = u ? out[(l0 + l) * NLOC + j] : 0.0;
+                for (int q = 0; q < nq; ++q) {
+                    const double h = sh[q * ELEM_BLOCK];
+                    const double *R = ref + q * 3 * NLOC;
+#pragma unroll
+                    for (int s = 0; s < 3; ++s)
+                        if (cols & (1 << s)) {
+                            double t[LR];
+#pragma unroll
+                            for (int l = 0; l < LR; ++l) t[l] = 0.0;
+#pragma unroll
+                            for (int r = 0; r < 3; ++r)
+                                if (rows & (1 << r)) {
+                                    const double hg = h * gk[3 * r + s];
+#pragma unroll
+                                    for (int l = 0; l < LR; ++l) t[l] += hg * R[r * NLOC + l0 + l];
+                                }
+#pragma unroll
+                            for (int j = 0; j < NLOC; ++j) {
+                                const double rj = R[s * NLOC + j];
+#pragma unroll
+                                for (int l = 0; l < LR; ++l) acc[l][j] += t[l] * rj;
+                            }
+                        }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int l = 0; l < LR; ++l)
+#pragma unroll
+                    for (int j = 0; j < NLOC; ++j) stage[threadIdx.x * CS + l * NLOC + j] = acc[l][j];
+                __syncthreads();
+                for (int i = threadIdx.x; i < m; i += ELEM_BLOCK)
+                    Ke[(size_t)(e0 + i / C) * (NLOC * NLOC) + l0 * NLOC + i % C] = stage[i / C * CS + i % C];
+            }
+            __syncthreads();                                 // a further coefficient adds to what was written
+        }
     }
 }
 
@@ -476,31 +706,53 @@ __global__ void __launch_bounds__(FAST_BLOCK) k_assemble_rows(
 
 // ---- K3d: one thread per row over the pair offsets ----------------------------------------------
 // As K3b, with the scatter map replaced by the row-local byte offsets (a quarter of the bytes),
-// the next pair's code, offsets and factors loaded while the current pair's entries are formed,
-// and the row written back from the shared-memory accumulator. P1 / P2 with up to 4 pair
+// the next pair's code, offsets and factors (NPAIR = 0: its row of the element matrix, factors =
+// Ke) loaded while the current pair's entries are formed, and the row written back from the
+// shared-memory accumulator. P1 / P2 with up to 4 pair
 // factors are held to 64 registers, 8 blocks per SM (no spills; 5 % faster at 1024^2 P2 than 7
 // blocks at 72 registers).
 template <int NLOC, int NPAIR>
 __global__ void __launch_bounds__(FAST_BLOCK, (NLOC <= 6 && NPAIR <= 4) ? 8 : 1) k_assemble_rows_off(
     const int *__restrict__ indptr, const int *__restrict__ rc_ptr, const int *__restrict__ rc_code,
-    const unsigned char *__restrict__ pair_off, const int *__restrict__ diag_pos, int nrows, int nq,
-    const double *__restrict__ factors, const double *__restrict__ g_S, const double *__restrict__ g_R, FastSpec fs,
-    int maxlen, double *__restrict__ data, double *__restrict__ inv, int *__restrict__ status)
+    const unsigned char *__restrict__ pair_off, const int *__restrict__ diag_pos, int nrows,
+    const double *__restrict__ factors, const double *__restrict__ g_S, int maxlen, double *__restrict__ data, double *__restrict__ inv, int *__restrict__ status)
 {
     extern __shared__ double smem[];
     constexpr int NL2 = NLOC * NLOC;
     constexpr int OFFS = (NLOC + 3) / 4 * 4;
     constexpr int NW = OFFS / 4;                             // 32-bit words of offsets per pair
+    constexpr int NV = NPAIR ? NPAIR : NLOC;                 // doubles loaded per pair
     double *sS = smem;
-    double *sR = sS + (fs.has_const ? NPAIR * NL2 : 0);
-    double *acc = sR + (fs.has_var ? nq * 3 * NLOC : 0);
-    if (fs.has_const)
-        for (int t = threadIdx.x; t < NPAIR * NL2; t += blockDim.x) sS[t] = g_S[t];
-    if (fs.has_var)
-        for (int t = threadIdx.x; t < nq * 3 * NLOC; t += blockDim.x) sR[t] = g_R[t];
+    double *acc = sS + NPAIR * NL2;
+    for (int t = threadIdx.x; t < NPAIR * NL2; t += blockDim.x) sS[t] = g_S[t];
     __syncthreads();
-    const int cst = fs.has_const ? NPAIR : 0;
-    const unsigned *offw = reinterpret_cast<const unsigned *>(pair_off);
+    // what a pair brings: its cell's factors, or its row of the element matrix
+    auto fetch = [&](int code, double (&v)[NV]) {
+        if (NV % 2 == 0) {
+            // 16-byte loads: a lane's doubles start on 16 bytes, and the gather is bound by the lines it touches
+            const double2 *F = reinterpret_cast<const double2 *>(factors + (size_t)(NPAIR ? code / NLOC : code) * NV);
+#pragma unroll
+            for (int k = 0; k < NV / 2; ++k) {
+                const double2 t = __ldg(&F[k]);
+                v[2 * k] = t.x;
+                v[2 * k + 1] = t.y;
+            }
+        } else {
+            const double *F = factors + (size_t)(NPAIR ? code / NLOC : code) * NV;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) v[k] = __ldg(&F[k]);
+        }
+    };
+    auto fetch_off = [&](int c, unsigned (&o)[NW]) {
+        if (NW == 2) {
+            const uint2 t = __ldcs(reinterpret_cast<const uint2 *>(pair_off) + c);
+            o[0] = t.x;
+            o[NW - 1] = t.y;
+        } else {
+#pragma unroll
+            for (int ww = 0; ww < NW; ++ww) o[ww] = __ldcs(reinterpret_cast<const unsigned *>(pair_off) + (size_t)c * NW + ww);
+        }
+    };
     // per warp: the first position of each of its 32 rows (+ the end), and for every position of
     // the warp's range the lane that owns it -- for the coalesced write-out below
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -520,59 +772,49 @@ __global__ void __launch_bounds__(FAST_BLOCK, (NLOC <= 6 && NPAIR <= 4) ? 8 : 1)
         const int c0 = rc_ptr[i], c1 = rc_ptr[i + 1];
         int code = 0;
         unsigned ow[NW];
-        double Fc[NPAIR];
+        double Fc[NV];
         if (c0 < c1) {
             code = __ldcs(&rc_code[c0]);
-#pragma unroll
-            for (int ww = 0; ww < NW; ++ww) ow[ww] = __ldcs(&offw[(size_t)c0 * NW + ww]);
-            const double *F = factors + (size_t)(code / NLOC) * fs.nf;
-#pragma unroll
-            for (int k = 0; k < NPAIR; ++k) Fc[k] = fs.has_const ? __ldg(&F[k]) : 0.0;
+            fetch_off(c0, ow);
+            fetch(code, Fc);
         }
         for (int c = c0; c < c1; ++c) {
             const int cur = code;
             unsigned oq[NW];
-            double Fq[NPAIR];
+            double Fq[NV];
 #pragma unroll
             for (int ww = 0; ww < NW; ++ww) oq[ww] = ow[ww];
 #pragma unroll
-            for (int k = 0; k < NPAIR; ++k) Fq[k] = Fc[k];
+            for (int k = 0; k < NV; ++k) Fq[k] = Fc[k];
             if (c + 1 < c1) {                                 // the next pair's loads
                 code = __ldcs(&rc_code[c + 1]);
-#pragma unroll
-                for (int ww = 0; ww < NW; ++ww) ow[ww] = __ldcs(&offw[(size_t)(c + 1) * NW + ww]);
-                const double *F = factors + (size_t)(code / NLOC) * fs.nf;
-#pragma unroll
-                for (int k = 0; k < NPAIR; ++k) Fc[k] = fs.has_const ? __ldg(&F[k]) : 0.0;
+                fetch_off(c + 1, ow);
+                fetch(code, Fc);
             }
-            const int e = cur / NLOC, l = cur - e * NLOC;
+            const int l = cur % NLOC;
             double v[NLOC];
 #pragma unroll
             for (int j = 0; j < NLOC; ++j) {
-                double s = 0.0;
-                if (fs.has_const) {
+                if (NPAIR == 0) {
+                    v[j] = Fq[j < NV ? j : 0];
+                } else {
+                    double s = 0.0;
 #pragma unroll
                     for (int k = 0; k < NPAIR; ++k) s += Fq[k] * sS[k * NL2 + l * NLOC + j];
+                    v[j] = s;
                 }
-                v[j] = s;
             }
-            if (fs.has_var) {
-                const double *H = factors + (size_t)e * fs.nf + cst;
-                for (int q = 0; q < nq; ++q) {
-                    const double *R = sR + q * 3 * NLOC;
+            // a pair's columns are distinct: every load of the accumulator before the stores
+            double t[NLOC];
 #pragma unroll
-                    for (int k = 0; k < NPAIR; ++k) {
-                        const double h = H[q * NPAIR + k] * R[fs.pr[k] * NLOC + l];
-                        const double *Rs = R + fs.ps[k] * NLOC;
-#pragma unroll
-                        for (int j = 0; j < NLOC; ++j) v[j] += h * Rs[j];
-                    }
-                }
+            for (int j = 0; j < NLOC; ++j) {
+                const unsigned o = (oq[j >> 2] >> (8 * (j & 3))) & 0xffu;
+                t[j] = o != 0xffu ? slot((int)o) : 0.0;
             }
 #pragma unroll
             for (int j = 0; j < NLOC; ++j) {
                 const unsigned o = (oq[j >> 2] >> (8 * (j & 3))) & 0xffu;
-                if (o != 0xffu) slot((int)o) += v[j];
+                if (o != 0xffu) slot((int)o) = t[j] + v[j];
             }
         }
         if (inv) {
@@ -594,9 +836,19 @@ __global__ void __launch_bounds__(FAST_BLOCK, (NLOC <= 6 && NPAIR <= 4) ? 8 : 1)
     const int first = wrlo[0];
     for (int k = 0; k < len; ++k) owner[rlo - first + k] = (unsigned char)lane;
     __syncwarp();
-    for (int p = first + lane; p < wrlo[32]; p += 32) {
-        const int t = owner[p - first], k = p - wrlo[t];
-        data[p] = acc[(size_t)k * FAST_BLOCK + w * 32 + ((t + k) & 31)];
+    constexpr int WU = 4;                                     // positions of a lane in flight
+    for (int p0 = first + lane; p0 < end_all; p0 += 32 * WU) {
+        int t[WU], k[WU];
+        double v[WU];
+#pragma unroll
+        for (int u = 0; u < WU; ++u) t[u] = p0 + 32 * u < end_all ? owner[p0 + 32 * u - first] : 0;
+#pragma unroll
+        for (int u = 0; u < WU; ++u) k[u] = p0 + 32 * u < end_all ? p0 + 32 * u - wrlo[t[u]] : 0;
+#pragma unroll
+        for (int u = 0; u < WU; ++u) v[u] = acc[(size_t)k[u] * FAST_BLOCK + w * 32 + ((t[u] + k[u]) & 31)];
+#pragma unroll
+        for (int u = 0; u < WU; ++u)
+            if (p0 + 32 * u < end_all) data[p0 + 32 * u] = v[u];
     }
     __syncwarp();
     }
@@ -606,17 +858,33 @@ __global__ void __launch_bounds__(FAST_BLOCK, (NLOC <= 6 && NPAIR <= 4) ? 8 : 1)
 // The pair offsets: for rc index c (row i, cell entry code = cell nloc + l), byte j of
 // off[c * OFFS + j] = position of (i, dof(cell, j)) minus indptr[i], 255 where constrained.
 // OFFS = nloc rounded up to a multiple of 4, so a pair's offsets load as whole 32-bit words.
-__global__ void k_pair_offsets(const int *__restrict__ rc_ptr, const int *__restrict__ rc_code,
-                               const int *__restrict__ indptr, const int *__restrict__ map, int nrows, int nloc, int offs,
-                               unsigned char *__restrict__ off)
+// Found by a search of the row, as the scatter map is; the map itself (4 bytes an entry against 1)
+// is not needed where every row kernel goes by these.
+__global__ void __launch_bounds__(128) k_pair_offsets(const int *__restrict__ rc_ptr, const int *__restrict__ rc_code,
+                                                      const int *__restrict__ indptr, const int *__restrict__ indices,
+                                                      const int *__restrict__ dofs, int nrows, int nloc, int offs,
+                                                      unsigned *__restrict__ off, int *__restrict__ status)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += gridDim.x * blockDim.x) {
-        const int rlo = indptr[i];
+        const int rlo = indptr[i], len = indptr[i + 1] - rlo;
+        const int *row = indices + rlo;
         for (int c = rc_ptr[i]; c < rc_ptr[i + 1]; ++c) {
-            const int code = rc_code[c];
-            for (int j = 0; j < offs; ++j) {
-                const int m = j < nloc ? map[(size_t)code * nloc + j] : -1;
-                off[(size_t)c * offs + j] = m < 0 ? (unsigned char)255 : (unsigned char)(m - rlo);
+            const int *d = dofs + (size_t)(rc_code[c] / nloc) * nloc;
+            for (int w = 0; w < offs / 4; ++w) {
+                unsigned word = 0xffffffffu;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int j = 4 * w + k, J = j < nloc ? d[j] : -1;
+                    if (J < 0) continue;
+                    int lo = 0, hi = len;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (row[mid] < J) lo = mid + 1; else hi = mid;
+                    }
+                    if (lo == len || row[lo] != J) atomicOr(status, ST_OUTSIDE);
+                    else word = (word & ~(0xffu << (8 * k))) | (unsigned)lo << (8 * k);
+                }
+                off[(size_t)c * (offs / 4) + w] = word;
             }
         }
     }
@@ -628,44 +896,20 @@ static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
     const int offs = (p->nloc + 3) / 4 * 4;
     const size_t npairs = (size_t)p->ncells * p->nloc;
     FEMD_TRY(p->pair_off.alloc(npairs * offs + 4));
+    FEMD_TRY(reset_status(ctx));
     if (p->nrows)
-        k_pair_offsets<<<grid_for((size_t)p->nrows, 256, 1u << 20), 256, 0, counted(ctx->stream)>>>(
-            p->rc_ptr.p, p->rc_code.p, p->indptr.p, p->map.p, p->nrows, p->nloc, offs, p->pair_off.p);
+        k_pair_offsets<<<grid_for((size_t)p->nrows, 128, 1u << 20), 128, 0, counted(ctx->stream)>>>(
+            p->rc_ptr.p, p->rc_code.p, p->indptr.p, p->indices.p, p->cell_dofs.p, p->nrows, p->nloc, offs,
+            reinterpret_cast<unsigned *>(p->pair_off.p), ctx->status_dev);
     FEMD_TRY_CUDA(cudaGetLastError());
-    return FEMD_OK;
-}
-
-// K4 FAST: one thread per row, f_i = sum over the row's cells (increasing order) of
-// sum_k F_k R_{r_k}(l) (constant) + sum_q sum_k H_{q,k} R_{r_k}(q, l) (varying), where the
-// constant part uses the tabulation integrated against the weights (Sv^{r}(l) = sum_q rw_q R_r(q,l)).
-__global__ void __launch_bounds__(256) k_assemble_vector_fast(const int *__restrict__ rc_ptr, const int *__restrict__ rc_code,
-                                                              int nrows, int nloc, int nq, const double *__restrict__ factors,
-                                                              const double *__restrict__ g_Sv, const double *__restrict__ g_R,
-                                                              FastSpec fs, double *__restrict__ f)
-{
-    extern __shared__ double smem[];
-    double *sSv = smem;                        // 3 * nloc
-    double *sR = sSv + 3 * nloc;               // nq * 3 * nloc
-    for (int t = threadIdx.x; t < 3 * nloc; t += blockDim.x) sSv[t] = g_Sv[t];
-    for (int t = threadIdx.x; t < nq * 3 * nloc; t += blockDim.x) sR[t] = g_R[t];
-    __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += gridDim.x * blockDim.x) {
-        double fi = 0.0;
-        for (int c = rc_ptr[i]; c < rc_ptr[i + 1]; ++c) {
-            const int code = rc_code[c];
-            const int e = code / nloc, l = code - e * nloc;
-            const double *F = factors + (size_t)e * fs.nf;
-            double v = 0.0;
-            int o = 0;
-            if (fs.has_const)
-                for (int k = 0; k < fs.npair; ++k) v += F[o++] * sSv[fs.pr[k] * nloc + l];
-            if (fs.has_var)
-                for (int q = 0; q < nq; ++q)
-                    for (int k = 0; k < fs.npair; ++k) v += F[o++] * sR[(q * 3 + fs.pr[k]) * nloc + l];
-            fi += v;
-        }
-        f[i] = fi;
+    int flags = 0;
+    FEMD_TRY(read_status(ctx, &flags, nullptr));
+    if (flags & ST_OUTSIDE) {
+        p->pair_off.release();
+        set_error("assemble_matrix_2d: entry outside the pattern");
+        return FEMD_EOUTSIDE;
     }
+    return FEMD_OK;
 }
 
 // ---- host side -----------------------------------------------------------------------------
@@ -695,6 +939,26 @@ static void fast_spec(int nterms, const int *a, const int *b, const femd_coef *c
                 const bool sb = vector ? s == 0 : (b[t] == 0 ? s == 0 : s != 0);
                 if (ra && sb) act[r][s] = true;
             }
+    }
+    for (int t = 0; t < nterms; ++t) {
+        const femd_coef &c = coef[t];
+        fs.cof[t] = -1;
+        for (int u = 0; u < t && fs.cof[t] < 0; ++u) {
+            const femd_coef &d = coef[u];
+            bool same = c.kind == d.kind;
+            if (c.kind == FEMD_COEF_CONST) same = same && c.value == d.value;
+            else if (c.kind == FEMD_COEF_POINTS) same = same && c.points_dev == d.points_dev;
+            else if (c.kind == FEMD_COEF_FIELD) same = same && c.field_dev == d.field_dev;
+            else
+                for (int i = 0; i < 4; ++i) same = same && c.p[i] == d.p[i];
+            if (same) fs.cof[t] = fs.cof[u];
+        }
+        if (fs.cof[t] < 0) {
+            fs.cof[t] = fs.ncof;
+            fs.cof_term[fs.ncof++] = t;
+        }
+        fs.rows |= a[t] == 0 ? 1 : 6;
+        fs.cols |= vector ? 1 : b[t] == 0 ? 1 : 6;
     }
     // a symmetric form with constant coefficients (every term (a, b) has its mirror (b, a) with
     // the same coefficient) has F_rs = F_sr on every cell: (r, s) and (s, r) share one factor
@@ -839,6 +1103,7 @@ static int prepare_terms(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     return FEMD_OK;
 }
 
+static constexpr size_t ASM_SHARED = 32u << 20;   // doubles (256 MB) of the context's workspace
 static constexpr int FAST_MAX_ROW = 96;   // longest row the shared-memory accumulator holds
 
 // FAST assembly of a matrix (K non-null) or a vector (f non-null).  Tables and factors live in
@@ -851,21 +1116,19 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     const int nq = rule->nq, nl = rule->nloc, nl2 = nl * nl, n = p->nrows, ne = p->ncells;
     FastSpec fs;
     fast_spec(nterms, a, b, coef, nq, vector, fs);
-    // host tables: [rw | xi | eta | ref (nq 3 nl) | S (npair nl^2) or Sv (3 nl)]
+    // host tables: [rw | xi | eta | ref (nq 3 nl) | S (npair nl^2)]
     const size_t nref = (size_t)nq * 3 * nl;
-    const size_t nS = vector ? (size_t)3 * nl : (size_t)fs.npair * nl2;
+    // element matrices where a coefficient varies, and for constant forms whose factors the row
+    // kernel below has no instance for; factors per cell else (P2: 24-32 B a cell against 288)
+    const bool listed = fs.npair == 1 || fs.npair == 3 || fs.npair == 4 || fs.npair == 5;
+    const bool element = !vector && (nl == 3 || nl == 6 || nl == 10) && (fs.has_var || !listed);
+    const bool tensors = !vector && !element;
+    const size_t nS = tensors ? (size_t)fs.npair * nl2 : 0;
     std::vector<double> tab(3 * (size_t)nq + nref + nS, 0.0);
     for (int q = 0; q < nq; ++q) { tab[q] = rule->w_host[q]; tab[nq + q] = rule->xi_host[q]; tab[2 * nq + q] = rule->eta_host[q]; }
     std::copy(rule->ref_host, rule->ref_host + nref, tab.begin() + 3 * nq);
     double *S = tab.data() + 3 * nq + nref;
-    if (vector) {
-        for (int r = 0; r < 3; ++r)
-            for (int l = 0; l < nl; ++l) {
-                double acc = 0.0;
-                for (int q = 0; q < nq; ++q) acc += rule->w_host[q] * rule->ref_host[((size_t)q * 3 + r) * nl + l];
-                S[r * nl + l] = acc;
-            }
-    } else {
+    if (tensors) {
         for (int k = 0; k < fs.npair; ++k)
             for (int l = 0; l < nl; ++l)
                 for (int j = 0; j < nl; ++j) {
@@ -878,7 +1141,12 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
                     S[(size_t)k * nl2 + l * nl + j] = acc;
                 }
     }
-    if (p->ws_factors.n < (size_t)ne * fs.nf + 1) FEMD_TRY(p->ws_factors.alloc((size_t)ne * fs.nf + 1));
+    const size_t per_cell = vector ? (size_t)nl : element ? (size_t)nl2 : (size_t)fs.nf;
+    // the cells' factors, vectors or matrices: in the context's workspace up to its bound (the
+    // context's stream orders the assemblies that share it), else in the pattern's own
+    const size_t cells = (size_t)ne * per_cell + 1;
+    DevBuf<double> &W = cells <= ASM_SHARED ? ctx->asm_scratch : p->ws_factors;
+    if (W.n < cells) FEMD_TRY(W.alloc(std::min(cells + cells / 4, std::max(cells, ASM_SHARED))));
     // the slot holding these tables, else the least recently used one, refilled (stream-ordered,
     // so kernels still reading the slot's old tables finish first)
     femd_pattern_s::TableSlot *slot = nullptr;
@@ -896,20 +1164,47 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     slot->used = ++p->table_clock;
     const double *d_tab = slot->dev.p;
     const double *d_ref = d_tab + 3 * nq, *d_S = d_ref + nref;
-    if (ne)
-        k_elem_factors<<<grid_for((size_t)ne, 256, 1u << 22), 256, 0, counted(s)>>>(
-            mesh->points_dev, mesh->tris_dev, ne, nq, nl, p->cell_dofs.p, d_tab, fs, p->ws_factors.p);
-    FEMD_TRY_CUDA(cudaGetLastError());
+    const size_t tshm = (3 * (size_t)nq + nref) * sizeof(double);
+    const unsigned egrid = grid_for((size_t)ne, ELEM_BLOCK, 1u << 22);
     if (vector) {
-        const size_t shm = (3 * (size_t)nl + nref) * sizeof(double);
-        if (n) {
-            cudaFuncSetAttribute(k_assemble_vector_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-            k_assemble_vector_fast<<<grid_for((size_t)n, 256, 1u << 22), 256, shm, counted(s)>>>(
-                p->rc_ptr.p, p->rc_code.p, n, nl, nq, p->ws_factors.p, d_S, d_ref, fs, f);
+        double *fe = W.p;
+        if (ne) {
+            const size_t vshm = tshm + (size_t)(nl | 1) * ELEM_BLOCK * sizeof(double);
+#define FEMD_ELEM_VECTOR(NL)                                                                                           \
+    cudaFuncSetAttribute(k_elem_vector<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vshm),                   \
+    k_elem_vector<NL><<<egrid, ELEM_BLOCK, vshm, counted(s)>>>(mesh->points_dev, mesh->tris_dev, ne, nq, nl, p->cell_dofs.p, \
+                                                               d_tab, fs, fe)
+            if (nl <= 3) FEMD_ELEM_VECTOR(3);
+            else if (nl <= 6) FEMD_ELEM_VECTOR(6);
+            else if (nl <= 10) FEMD_ELEM_VECTOR(10);
+            else if (nl <= 15) FEMD_ELEM_VECTOR(15);
+            else FEMD_ELEM_VECTOR(MAX_NLOC);
+#undef FEMD_ELEM_VECTOR
         }
+        FEMD_TRY_CUDA(cudaGetLastError());
+        if (n) k_gather_vector<<<grid_for((size_t)n, 256, 1u << 22), 256, 0, counted(s)>>>(p->rc_ptr.p, p->rc_code.p, n, fe, f);
         FEMD_TRY_CUDA(cudaGetLastError());
         return FEMD_OK;
     }
+    if (ne && element) {
+        const size_t eshm = tshm + (size_t)(nq + (nl == 10 ? 21 : nl == 6 ? 19 : 9)) * ELEM_BLOCK * sizeof(double);
+#define FEMD_ELEM_MATRIX(NL, LR)                                                                                         \
+    do {                                                                                                               \
+        FEMD_TRY_CUDA(cudaFuncSetAttribute((k_elem_matrix<NL, LR>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eshm)); \
+        k_elem_matrix<NL, LR><<<egrid, ELEM_BLOCK, eshm, counted(s)>>>(mesh->points_dev, mesh->tris_dev, ne, nq, p->cell_dofs.p, \
+                                                                   d_tab, fs, W.p);                        \
+    } while (0)
+        if (nl == 3) FEMD_ELEM_MATRIX(3, 3);
+        else if (nl == 6) FEMD_ELEM_MATRIX(6, 3);
+        else FEMD_ELEM_MATRIX(10, 2);
+#undef FEMD_ELEM_MATRIX
+    } else if (ne) {
+        k_elem_factors<<<grid_for((size_t)ne, 256, 1u << 22), 256, 0, counted(s)>>>(
+            mesh->points_dev, mesh->tris_dev, ne, nq, nl, p->cell_dofs.p, d_tab, fs, W.p);
+    }
+    FEMD_TRY_CUDA(cudaGetLastError());
+    const bool by_pairs = (nl == 3 || nl == 6 || nl == 10) && (element || listed);
+    FEMD_TRY(by_pairs ? build_pair_offsets(ctx, p) : build_scatter_map(ctx, p));
     FEMD_TRY(reset_status(ctx));
     double *inv = nullptr;
     if (want_inv) {
@@ -921,27 +1216,24 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
                            sizeof(double) + (FAST_BLOCK / 32) * 33 * sizeof(int);
     if (n) {
         const unsigned grid = grid_for((size_t)n, FAST_BLOCK, 1u << 22);
-        bool done = false;
-        const size_t sho = ((fs.has_const ? (size_t)fs.npair * nl2 : 0) + (fs.has_var ? nref : 0) +
-                            (size_t)maxlen * FAST_BLOCK) * sizeof(double) +
+        const int np = element ? 0 : fs.npair;
+        const size_t sho = ((size_t)np * nl2 + (size_t)maxlen * FAST_BLOCK) * sizeof(double) +
                            (FAST_BLOCK / 32) * 33 * sizeof(int) + (size_t)FAST_BLOCK * maxlen;
 #define FEMD_ROWS_OFF(NL, NP)                                                                                          \
-        if (!done && nl == NL && fs.npair == NP && maxlen < 255) {                                                     \
-            FEMD_TRY(build_pair_offsets(ctx, p));                                                                      \
+        if (nl == NL && np == NP) {                                                                                    \
             cudaFuncSetAttribute(k_assemble_rows_off<NL, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sho); \
             k_assemble_rows_off<NL, NP><<<grid, FAST_BLOCK, sho, counted(s)>>>(                                        \
-                p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->pair_off.p, p->diag_pos.p, n, nq, p->ws_factors.p, d_S,     \
-                d_ref, fs, maxlen, K->data.p, inv, ctx->status_dev);                                                   \
-            done = true;                                                                                               \
+                p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->pair_off.p, p->diag_pos.p, n, W.p, d_S, maxlen, \
+                K->data.p, inv, ctx->status_dev);                                                                      \
         }
-        FEMD_ROWS_OFF(3, 1) FEMD_ROWS_OFF(3, 3) FEMD_ROWS_OFF(3, 4) FEMD_ROWS_OFF(3, 5)
-        FEMD_ROWS_OFF(6, 1) FEMD_ROWS_OFF(6, 3) FEMD_ROWS_OFF(6, 4) FEMD_ROWS_OFF(6, 5)
-        FEMD_ROWS_OFF(10, 1) FEMD_ROWS_OFF(10, 3) FEMD_ROWS_OFF(10, 4) FEMD_ROWS_OFF(10, 5)
+        FEMD_ROWS_OFF(3, 0) FEMD_ROWS_OFF(3, 1) FEMD_ROWS_OFF(3, 3) FEMD_ROWS_OFF(3, 4) FEMD_ROWS_OFF(3, 5)
+        FEMD_ROWS_OFF(6, 0) FEMD_ROWS_OFF(6, 1) FEMD_ROWS_OFF(6, 3) FEMD_ROWS_OFF(6, 4) FEMD_ROWS_OFF(6, 5)
+        FEMD_ROWS_OFF(10, 0) FEMD_ROWS_OFF(10, 1) FEMD_ROWS_OFF(10, 3) FEMD_ROWS_OFF(10, 4) FEMD_ROWS_OFF(10, 5)
 #undef FEMD_ROWS_OFF
-        if (!done) {
+        if (!by_pairs) {
             cudaFuncSetAttribute(k_assemble_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
             k_assemble_rows<<<grid, FAST_BLOCK, shm, counted(s)>>>(p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->map.p,
-                                                                   p->diag_pos.p, n, nl, nq, p->ws_factors.p, d_S, d_ref,
+                                                                   p->diag_pos.p, n, nl, nq, W.p, d_S, d_ref,
                                                                    fs, maxlen, K->data.p, inv, ctx->status_dev);
         }
     }
@@ -974,9 +1266,9 @@ int femd_cuda_assemble_matrix(femd_ctx ctx, const femd_mesh2d *mesh, const femd_
     FEMD_CHECK_ARG(K && K->kind == KIND_MATRIX && K->pattern == p, "assemble_matrix_2d: K is not a matrix on this pattern");
     FEMD_TRY_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    FEMD_TRY(build_scatter_map(ctx, p));
     if (mode == FEMD_ASM_FAST && p->max_row_len <= FAST_MAX_ROW)
         return fast_assemble(ctx, mesh, rule, p, nterms, a, b, coef, K, want_inv, nullptr);
+    FEMD_TRY(build_scatter_map(ctx, p));
     RuleDev R;
     FEMD_TRY(upload_rule(rule, mode == FEMD_ASM_FAST, R, s));
     DevBuf<double> scratch;

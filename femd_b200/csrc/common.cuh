@@ -100,6 +100,8 @@ struct femd_ctx_s {
     // most), pinned room for its result, and the events that time it
     femd::DevBuf<double> res_scratch;
     void *res_host = nullptr;
+    // the cells' factors, vectors or matrices of an assembly, up to 256 MB; a larger one's belong to its pattern
+    femd::DevBuf<double> asm_scratch;
     cudaEvent_t res_e0 = nullptr, res_e1 = nullptr;
 };
 
@@ -128,8 +130,7 @@ struct femd_pattern_s : femd::HandleBase {
     femd::DevBuf<int> diag_pos;        // position of (i, i), -1 when absent
     bool all_diag = false;             // every row i holds the position (i, i)
     int max_row_cells = 0, max_row_len = 0;
-    // assembly workspace, grown on demand and reused across calls (no allocation per call
-    // once it has its size): per-element factors, the rule's tables
+    // assembly workspace past the context's shared one, grown on demand and reused across calls
     femd::DevBuf<double> ws_factors;
     // the rule's tables (weights, points, reference values, the pair tensors) of the last few
     // forms, each with the host copy it was uploaded from: a repeated assembly of the same form
@@ -144,7 +145,7 @@ struct femd_pattern_s : femd::HandleBase {
     unsigned long long table_clock = 0;
     // for every (row, cell) pair of the rc lists, the offsets within the row of the cell's nloc
     // columns (uint8, 255 = constrained): the scatter map in the rows' own order, a quarter of
-    // its size (built on the first FAST assembly when every row is shorter than 255)
+    // its size (built on the first FAST assembly of P1 to P3)
     femd::DevBuf<unsigned char> pair_off;
     // the batched engine's compact layout of the pattern, built on first use: a reverse
     // Cuthill-McKee order with the rows of every 256 sorted by length (iperm: original row ->
