@@ -159,6 +159,13 @@ struct femd_pattern_s : femd::HandleBase {
     femd::DevBuf<int> cl_iperm, cl_indptr, cl_dst;
     femd::DevBuf<short> cl_off;
     std::vector<int> cl_tile_lo, cl_tile_hi;
+    // the single solve's layout (krylov.cu): slices of 32 consecutive rows, entry j of every row side by
+    // side, filled up to the slice's longest row (column -1).  sl_state: 0 not looked at, 1 suitable, -1
+    // too much filling; sl_slots entries in all; the slices' first entries (in 32) and the columns, built
+    // at the first solve that uses them
+    int sl_state = 0;
+    long long sl_slots = 0;
+    femd::DevBuf<int> sl_ptr, sl_col;
     femd_pattern_s() : HandleBase(femd::KIND_PATTERN) {}
     ~femd_pattern_s() override { femd::ctx_release(ctx); }
 };
@@ -169,6 +176,7 @@ struct femd_matrix_s : femd::HandleBase {
     femd::DevBuf<double> data, inv;
     femd::DevBuf<float> data32, inv32;   // FP32 copies (mixed precision), built on demand
     bool f32_valid = false;
+    bool f32_slices = false;             // data32 is in the pattern's slices
     // the inverse diagonal has been written (assembly with want_inv, femd_cuda_matrix_jacobi,
     // femd_cuda_matrix_set_inv_diag, or the host upload of femd_cuda_cg_solve_host); until then
     // every preconditioned solve refuses the matrix instead of reading uninitialised memory

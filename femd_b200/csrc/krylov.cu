@@ -5,15 +5,18 @@
 // Reference: krylov::cg_jacobi (include/femd/krylov/cg.hpp:296-350), cg_update_chunk_jacobi
 // (:99-171), detail_cg::finish (:222-237), CSRMatrix::apply (include/femd/sparse/csr.hpp:203-215).
 //
-// Reductions.  Every kernel that produces a dot product writes one partial per block; the
-// last block to finish (an atomic ticket, no waiting) adds the partials in block order and
-// updates the scalar state (alpha, beta, the stopping test).  The grid of each kernel depends
+// Reductions.  Every kernel that produces a dot product writes one partial per block; every block
+// of the next kernel adds them all in one fixed tree and so knows alpha, or beta and the stopping
+// test, without a word from the others (its first block writes the state down).  A last block that
+// adds the partials at the end of a kernel (an atomic ticket; the start and finish kernels, which
+// run once, do that) put 3 to 6 us behind every SpMV and update.  The grid of each kernel depends
 // only on n, so the sums -- and the iterates -- have the same bits on every run.  Kernels of an
 // iteration that starts after the stopping test has fired return at once, so whole chunks of
 // iterations are queued (captured in a CUDA graph) and the host only polls between chunks.
 //
 // HBM bytes per FP64 iteration (n rows, nnz entries): SpMV 12 nnz + 4 (n+1) + 8 n (p) + 8 n (Ap);
 // update 40 n read + 16 n written; direction 24 n read + 8 n written.
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 #include <cmath>
@@ -31,11 +34,13 @@ static constexpr int RED_BLOCK = 256;
 
 template <class T>
 struct CGState {
-    double rz, pAp, alpha, beta, rr;       // scalars and dot products in FP64 for both precisions
+    // scalars and dot products in FP64 for both precisions.  r.z and the iterations done have two
+    // places: the kernels of iteration k read place k % 2 while the last of them writes the other
+    double rz[2], beta, rr;
     double nb, tol_nb, rn, res64;          // FP64 scalars (norms of b and of the true residual)
     double maxr;                           // mixed precision: largest ||r|| since the last reliable update
     double rz_prev;                        // mixed precision: r.z before the last recurrence step
-    int it, done, breakdown, max_iter;
+    int it, done, breakdown, max_iter, itn[2];
     int want_ru, ru_count;
     // mixed precision: the true residual of the last reliable update, the updates in a row that
     // reduced it by less than 2x, and the switch to FP64 after two of them (or a non-finite one)
@@ -94,6 +99,35 @@ __device__ __forceinline__ void reduce_partials(const T *part, int np, int ld, T
     for (int k = 0; k < NV; ++k) out[k] = v[k];
 }
 
+// the block's share of p.Ap
+__device__ __forceinline__ void write_partial(double dot, double *part, double *sh)
+{
+    double v[1] = {dot};
+    block_reduce<double, 1>(v, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+
+// The sums of NV partial arrays (np long, stride ld) in every thread, by a fixed tree; sh: 33 NV.
+template <int NV>
+__device__ __forceinline__ void all_partials(const double *part, int np, int ld, double (&out)[NV], double *sh)
+{
+    double v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < np; b += RED_BLOCK)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] += __ldcg(part + k * ld + b);
+    block_reduce<double, NV>(v, sh);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) sh[32 * NV + k] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = sh[32 * NV + k];
+    __syncthreads();
+}
+
 // ---- SpMV: y = A x, TPR lanes per row; DOT adds x_i y_i into the block partial ------------
 // Each lane takes the entries lo + lane, lo + lane + TPR, ... of its row, U at a time: the U
 // index and value loads are issued together, then the U gathers of x, then the U products
@@ -150,83 +184,260 @@ __global__ void __launch_bounds__(RED_BLOCK) k_spmv(const int *__restrict__ indp
             if (DOT) dot += (double)x[i] * (double)s;
         }
     }
-    if (!DOT) return;
-    double v[1] = {dot};
-    block_reduce<double, 1>(v, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
-    if (!last_block(&st->ticket)) return;
-    double tot[1];
-    reduce_partials<double, 1>(part, gridDim.x, 0, tot, sh);
-    if (threadIdx.x == 0) {
-        st->ticket = 0;
-        const double pAp = tot[0];
-        st->pAp = pAp;
-        if (!(pAp > 0.0)) { st->breakdown = 1; st->done = 1; }
-        else st->alpha = st->rz / pAp;
-    }
+    if (DOT) write_partial(dot, part, sh);
 }
 
-// ---- fused update: x += a p; r -= a Ap; rr = r.r; rz = r.(inv r) ------------------------------
-// JAC: with the Jacobi inverse diagonal; otherwise rz = rr (cg.hpp:330-331).
+// ---- SpMV of a solve: one lane a row, the rows in slices of 32 ---------------------------------
+// An iterating solve streams its matrix hundreds of times, so it keeps the entries in slices: entry
+// j of 32 consecutive rows side by side, a warp to a slice.  Every load of the stream is then 128
+// or 256 contiguous bytes, the gathers of x run along neighbouring columns, and there is no tree
+// of shuffles; U entries of every lane are in flight.  It is bound by HBM (or L2): 57.2 us at P2
+// 768^2 (27.1 M entries; the bytes take 56.9 us at the measured copy rate) against 82.1 us with lane
+// groups over CSR rows; P3 216^2 18.5 against 34.8 us, P1 1000^2 18.5 against 26.7.  U = 5 at 5
+// blocks an SM: 10 entries at 3 blocks 61.3 us, 8 at 4 blocks 58.1, 4 at 6 blocks 59.5.  Two waves of
+// blocks: one leaves the last slices uneven (P3 216^2 22.6 us), of four every block of the update
+// adds up twice the partials (mixed P2 512^2: 37.3 us an iteration against 35.0).
+// A lane sums its row in entry order, as the CSR form below does, so both give the same bits.
+// FP32 values: row-sum form, as k_spmv.
+static constexpr int SL_U64 = 5, SL_U32 = 8, SL_BLOCKS = 5;
+
+template <class V, class T, bool DOT>
+__global__ void __launch_bounds__(RED_BLOCK, SL_BLOCKS) k_spmv_slices(const int *__restrict__ sptr, const int *__restrict__ cols,
+                                                                      const V *__restrict__ vals, const T *__restrict__ x,
+                                                                      T *__restrict__ y, int n, double *__restrict__ part,
+                                                                      CGState<T> *__restrict__ st)
+{
+    __shared__ double sh[32];
+    constexpr bool ROWSUM = std::is_same<V, float>::value;
+    constexpr int U = ROWSUM ? SL_U32 : SL_U64;
+    if (DOT && (st->done || st->want_ru)) return;
+    const int lane = threadIdx.x & 31, nsl = (n + 31) >> 5;
+    const int gwarp = (blockIdx.x * RED_BLOCK + threadIdx.x) >> 5, nwarp = (gridDim.x * RED_BLOCK) >> 5;
+    double dot = 0.0;
+    for (int sl = gwarp; sl < nsl; sl += nwarp) {
+        const int b = sptr[sl], width = sptr[sl + 1] - b, i = 32 * sl + lane;
+        const int *cp = cols + (size_t)32 * b + lane;
+        const V *vp = vals + (size_t)32 * b + lane;
+        const T xi = (ROWSUM || DOT) && i < n ? __ldg(&x[i]) : T(0);
+        T acc = T(0);
+        for (int j0 = 0; j0 < width; j0 += U) {
+            int c[U];
+            V v[U];
+            T xv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = j0 + u < width;
+                c[u] = in ? __ldcs(cp + 32 * (j0 + u)) : -1;
+                v[u] = in ? __ldcs(vp + 32 * (j0 + u)) : V(0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) xv[u] = c[u] >= 0 ? __ldg(&x[c[u]]) : T(0);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c[u] >= 0) acc = fma((T)v[u], ROWSUM && c[u] != i ? xv[u] - xi : xv[u], acc);
+        }
+        if (i < n) {
+            y[i] = acc;
+            if (DOT) dot += (double)xi * (double)acc;
+        }
+    }
+    if (DOT) write_partial(dot, part, sh);
+}
+
+// The same sums from CSR, for the solve that keeps nothing (its own slices among it): a warp takes its
+// 32 rows' entries through shared memory, SL_CAP at a time (one entry in 16 left out of the banks'
+// order, or rows of 16 entries would put all lanes on one bank).  42.3 us at P2 512^2, lane groups 43.2.
+static constexpr int SL_CAP = 320;
+
+template <bool DOT>
+__global__ void __launch_bounds__(RED_BLOCK, 6) k_spmv_csr_slices(const int *__restrict__ indptr, const int *__restrict__ indices,
+                                                                  const double *__restrict__ vals, const double *__restrict__ x,
+                                                                  double *__restrict__ y, int n, double *__restrict__ part,
+                                                                  CGState<double> *__restrict__ st)
+{
+    __shared__ double sh[32];
+    __shared__ double sv[RED_BLOCK / 32][SL_CAP + SL_CAP / 16];
+    __shared__ int sc[RED_BLOCK / 32][SL_CAP + SL_CAP / 32];
+    if (DOT && (st->done || st->want_ru)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nsl = (n + 31) >> 5;
+    const int gwarp = (blockIdx.x * RED_BLOCK + threadIdx.x) >> 5, nwarp = (gridDim.x * RED_BLOCK) >> 5;
+    double dot = 0.0;
+    for (int sl = gwarp; sl < nsl; sl += nwarp) {
+        const int i = 32 * sl + lane, lo = indptr[min(i, n)], hi = indptr[min(i + 1, n)];
+        const int q0 = __shfl_sync(0xffffffffu, lo, 0), q1 = __shfl_sync(0xffffffffu, hi, 31);
+        double acc = 0.0;
+        for (int c0 = q0; c0 < q1; c0 += SL_CAP) {
+            const int m = min(SL_CAP, q1 - c0);
+#pragma unroll 5
+            for (int t = lane; t < m; t += 32) {
+                sv[w][t + (t >> 4)] = __ldcs(&vals[c0 + t]);
+                sc[w][t + (t >> 5)] = __ldcs(&indices[c0 + t]);
+            }
+            __syncwarp();
+            const int a = max(lo, c0) - c0, e = min(hi, c0 + m) - c0;
+#pragma unroll 8
+            for (int t = a; t < e; ++t) acc = fma(sv[w][t + (t >> 4)], __ldg(&x[sc[w][t + (t >> 5)]]), acc);
+            __syncwarp();
+        }
+        if (i < n) {
+            y[i] = acc;
+            if (DOT) dot += x[i] * acc;
+        }
+    }
+    if (DOT) write_partial(dot, part, sh);
+}
+
+// The widths of the slices: their sum (into *sum), or one each.
+__global__ void k_slice_widths(const int *__restrict__ indptr, int n, int nsl, int *__restrict__ sum, int *__restrict__ width)
+{
+    const int sl = blockIdx.x * (RED_BLOCK / 32) + (threadIdx.x >> 5), i = 32 * sl + (threadIdx.x & 31);
+    if (sl >= nsl) return;
+    const int len = __reduce_max_sync(0xffffffffu, i < n ? indptr[i + 1] - indptr[i] : 0);
+    if ((threadIdx.x & 31) != 0) return;
+    if (sum) atomicAdd(sum, len);
+    if (width) width[sl] = len;
+}
+
+// The slices' columns (cols), FP64 values (v64) and FP32 values in row-sum form (v32), each where given.
+__global__ void __launch_bounds__(RED_BLOCK) k_slice_fill(const int *__restrict__ indptr, const int *__restrict__ indices,
+                                                          const double *__restrict__ data, const int *__restrict__ diag_pos,
+                                                          const int *__restrict__ sptr, int n, int nsl, int *__restrict__ cols,
+                                                          double *__restrict__ v64, float *__restrict__ v32)
+{
+    const int sl = blockIdx.x * (RED_BLOCK / 32) + (threadIdx.x >> 5), i = 32 * sl + (threadIdx.x & 31);
+    if (sl >= nsl) return;
+    const int lo = i < n ? indptr[i] : 0, len = i < n ? indptr[i + 1] - lo : 0, width = sptr[sl + 1] - sptr[sl];
+    const size_t base = (size_t)32 * sptr[sl] + (threadIdx.x & 31);
+    double sum = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < width; ++j) {
+        const bool in = j < len;
+        if (cols) cols[base + 32 * (size_t)j] = in ? indices[lo + j] : -1;
+        if (data) {
+            const double v = in ? data[lo + j] : 0.0;
+            if (v64) v64[base + 32 * (size_t)j] = v;
+            if (v32) {
+                v32[base + 32 * (size_t)j] = (float)v;
+                sum += v;
+            }
+        }
+    }
+    if (v32 && i < n) v32[base + 32 * (size_t)(diag_pos[i] - lo)] = (float)sum;
+}
+
+// ---- fused update: alpha = r.z / p.Ap; x += a p; r -= a Ap; rr = r.r; rz = r.(inv r) ------------
+// pap: the SpMV's npap partials.  JAC: with the Jacobi inverse diagonal; otherwise rz = rr
+// (cg.hpp:330-331).  place: the iteration's parity.
+static constexpr int VEC_U = 4;               // rows of a thread in flight
+
 template <class T, bool JAC>
 __global__ void __launch_bounds__(RED_BLOCK) k_cg_update(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p,
                                                          const T *__restrict__ Ap, const T *__restrict__ inv, int n,
-                                                         double *__restrict__ part, CGState<T> *__restrict__ st,
-                                                         int mixed)
+                                                         const double *__restrict__ pap, int npap, double *__restrict__ part,
+                                                         CGState<T> *__restrict__ st, int place)
 {
-    __shared__ double sh[64];
+    __shared__ double sh[66];
     if (st->done || st->want_ru) return;                  // want_ru: paused for a reliable update (mixed)
-    const T a = (T)st->alpha;
+    const double rz0 = st->rz[place];
+    double tot[1];
+    all_partials<1>(pap, npap, 0, tot, sh);
+    if (!(tot[0] > 0.0)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) { st->breakdown = 1; st->done = 1; }
+        return;
+    }
+    const T a = (T)(rz0 / tot[0]);
     double rr = 0.0, rz = 0.0;                            // FP64 accumulation (FP32 vectors too)
-    for (int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < n; i += gridDim.x * RED_BLOCK) {
-        const T ri = r[i] - a * Ap[i];
-        r[i] = ri;
-        x[i] = x[i] + a * p[i];
-        const double t = (double)ri * (double)ri;
-        rr += t;
-        if (JAC) rz += t * (double)inv[i];
+    const int step = gridDim.x * RED_BLOCK;
+    for (int i0 = blockIdx.x * RED_BLOCK + threadIdx.x; i0 < n; i0 += VEC_U * step) {
+        T rv[VEC_U], av[VEC_U], xv[VEC_U], pv[VEC_U], iv[VEC_U];
+#pragma unroll
+        for (int u = 0; u < VEC_U; ++u) {
+            const int i = i0 + u * step;
+            const bool in = i < n;
+            rv[u] = in ? r[i] : T(0);
+            av[u] = in ? Ap[i] : T(0);
+            xv[u] = in ? x[i] : T(0);
+            pv[u] = in ? p[i] : T(0);
+            iv[u] = JAC && in ? inv[i] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < VEC_U; ++u) {
+            const int i = i0 + u * step;
+            if (i < n) {
+                const T ri = rv[u] - a * av[u];
+                r[i] = ri;
+                x[i] = xv[u] + a * pv[u];
+                const double t = (double)ri * (double)ri;
+                rr += t;
+                if (JAC) rz += t * (double)iv[u];
+            }
+        }
     }
     double v[2] = {rr, rz};
     block_reduce<double, 2>(v, sh);
     if (threadIdx.x == 0) { part[blockIdx.x] = v[0]; part[gridDim.x + blockIdx.x] = v[1]; }
-    if (!last_block(&st->ticket)) return;
-    double tot[2];
-    reduce_partials<double, 2>(part, gridDim.x, gridDim.x, tot, sh);
-    if (threadIdx.x == 0) {
-        st->ticket = 0;
-        const double rrn = tot[0], rzn = JAC ? tot[1] : tot[0];
-        st->rr = rrn;
-        st->it += 1;
-        const double rn = sqrt((double)rrn);
-        st->rn = rn;
-        if (!mixed) {
-            if (rn <= st->tol_nb) { st->done = 1; return; }            // cg.hpp:334
-            if (st->it >= st->max_iter) { st->done = 1; return; }      // loop condition
-            st->beta = rzn / st->rz;                                   // cg.hpp:335-336
-            st->rz = rzn;
-            if (!(rzn > 0.0)) { st->breakdown = 1; st->done = 1; }     // cg.hpp:324 at the next loop top
-        } else {
-            // mixed precision: ask for a reliable update when the recurrence residual has
-            // dropped by a decade since the last one, or looks converged
-            if (rn <= 0.1 * st->maxr || rn <= st->tol_nb || st->it >= st->max_iter) st->want_ru = 1;
-            st->rz_prev = st->rz;
-            st->beta = rzn / st->rz;
-            st->rz = rzn;
-            if (!(rzn > 0.0)) st->want_ru = 1;
-        }
-    }
 }
 
-// ---- direction: p = inv r + beta p (or r + beta p) ------------------------------------------
-template <class T, bool JAC>
+// ---- direction: the stopping test, beta, p = inv r + beta p (or r + beta p) -------------------
+// GIVEN: beta is the state's (after a reliable update), no test.  part: the update's np partials.
+template <class T, bool JAC, bool MIXED, bool GIVEN>
 __global__ void __launch_bounds__(RED_BLOCK) k_cg_direction(T *__restrict__ p, const T *__restrict__ r,
                                                             const T *__restrict__ inv, int n,
-                                                            const CGState<T> *__restrict__ st)
+                                                            const double *__restrict__ part, int np,
+                                                            CGState<T> *__restrict__ st, int place)
 {
+    __shared__ double sh[66];
     if (st->done || st->want_ru) return;
-    const T b = (T)st->beta;
-    for (int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < n; i += gridDim.x * RED_BLOCK)
-        p[i] = (JAC ? inv[i] * r[i] : r[i]) + b * p[i];
+    double beta;
+    if (GIVEN) {
+        beta = st->beta;
+    } else {
+        const double rz0 = st->rz[place], tol_nb = st->tol_nb, maxr = MIXED ? st->maxr : 0.0;
+        const int it = st->itn[place] + 1, max_iter = st->max_iter;
+        double tot[2];
+        all_partials<2>(part, np, np, tot, sh);
+        const double rn = sqrt(tot[0]), rzn = JAC ? tot[1] : tot[0];
+        beta = rzn / rz0;                                              // cg.hpp:335-336
+        // the residual small enough (cg.hpp:334), the loop condition, the test at the next loop top (:324)
+        const bool stop = rn <= tol_nb || it >= max_iter, bad = !(rzn > 0.0);
+        // mixed precision: ask for a reliable update when the recurrence residual has dropped by a
+        // decade since the last one, or looks converged
+        const bool pause = MIXED && (rn <= 0.1 * maxr || stop || bad);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->rr = tot[0];
+            st->it = it;
+            st->itn[place ^ 1] = it;
+            st->rn = rn;
+            if (MIXED) {
+                st->rz_prev = rz0;
+                if (pause) st->want_ru = 1;
+            } else if (stop || bad) {
+                if (!stop) st->breakdown = 1;
+                st->done = 1;
+            }
+            st->beta = beta;
+            st->rz[place ^ 1] = rzn;
+        }
+        if (MIXED ? pause : stop || bad) return;
+    }
+    const T b = (T)beta;
+    const int step = gridDim.x * RED_BLOCK;
+    for (int i0 = blockIdx.x * RED_BLOCK + threadIdx.x; i0 < n; i0 += VEC_U * step) {
+        T rv[VEC_U], pv[VEC_U], iv[VEC_U];
+#pragma unroll
+        for (int u = 0; u < VEC_U; ++u) {
+            const int i = i0 + u * step;
+            const bool in = i < n;
+            rv[u] = in ? r[i] : T(0);
+            pv[u] = in ? p[i] : T(0);
+            iv[u] = JAC && in ? inv[i] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < VEC_U; ++u) {
+            const int i = i0 + u * step;
+            if (i < n) p[i] = (JAC ? iv[u] * rv[u] : rv[u]) + b * pv[u];
+        }
+    }
 }
 
 // ---- start: r = b - Ax; p = inv r; nb, ||r||, rz ------------------------------------------
@@ -264,9 +475,9 @@ __global__ void __launch_bounds__(RED_BLOCK) k_cg_start(const double *__restrict
         st->tol_nb = tol * nb;
         st->rn = rn;
         st->maxr = rn;
-        st->rz = tot[2];
+        st->rz[0] = st->rz[1] = tot[2];
         st->rr = tot[1];
-        st->it = 0;
+        st->it = st->itn[0] = st->itn[1] = 0;
         st->breakdown = 0;
         st->done = 0;
         if (nb == 0.0) { st->done = 1; return; }                        // cg.hpp:306
@@ -354,8 +565,8 @@ __global__ void __launch_bounds__(RED_BLOCK) k_pc_rz(const double *__restrict__ 
     if (threadIdx.x == 0) {
         st->ticket = 0;
         const double rzn = tot[0];
-        if (!FIRST) st->beta = rzn / st->rz;
-        st->rz = rzn;
+        if (!FIRST) st->beta = rzn / st->rz[0];
+        st->rz[0] = rzn;
         if (!(rzn > 0.0)) { st->breakdown = 1; st->done = 1; }
     }
 }
@@ -363,11 +574,18 @@ __global__ void __launch_bounds__(RED_BLOCK) k_pc_rz(const double *__restrict__ 
 // x += a p; r -= a Ap; ||r||; the stopping test (cg.hpp:278-281)
 __global__ void __launch_bounds__(RED_BLOCK) k_pc_update(double *__restrict__ x, double *__restrict__ r,
                                                          const double *__restrict__ p, const double *__restrict__ Ap, int n,
-                                                         double *__restrict__ part, CGState<double> *__restrict__ st)
+                                                         const double *__restrict__ pap, int npap, double *__restrict__ part,
+                                                         CGState<double> *__restrict__ st)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[33];
     if (st->done) return;
-    const double a = st->alpha;
+    double pAp[1];
+    all_partials<1>(pap, npap, 0, pAp, sh);
+    if (!(pAp[0] > 0.0)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) { st->breakdown = 1; st->done = 1; }
+        return;
+    }
+    const double a = st->rz[0] / pAp[0];
     double rr = 0.0;
     for (int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < n; i += gridDim.x * RED_BLOCK) {
         const double ri = r[i] - a * Ap[i];
@@ -482,7 +700,8 @@ __global__ void __launch_bounds__(RED_BLOCK) k_mixed_residual(const double *__re
         const double rzn = t32[0];
         if (!(rzn > 0.0)) { st->breakdown = 1; st->done = 1; return; }
         st->beta = rn > 2.0 * rn_rec ? 0.0 : rzn / st->rz_prev;
-        st->rz = rzn;
+        st->rz[0] = st->rz[1] = rzn;
+        st->itn[0] = st->itn[1] = st->it;
     }
 }
 
@@ -559,7 +778,8 @@ __global__ void k_combine(double alpha, const double *__restrict__ A, double bet
 unsigned red_grid(femd_ctx ctx, int n)
 {
     // a fixed function of n (deterministic reductions): enough blocks to fill the GPU
-    const unsigned cap = (unsigned)ctx->sm_count * 8;
+    // three blocks an SM: each reads every block's partials (8: 100 us an iteration at P2 768^2, 3: 91.5)
+    const unsigned cap = (unsigned)ctx->sm_count * 3;
     return grid_for((size_t)n, RED_BLOCK * 4, cap);
 }
 
@@ -610,6 +830,58 @@ unsigned spmv_grid(femd_ctx ctx, int n, int shape)
     return grid_for((size_t)n, gpb, cap);
 }
 
+static unsigned slices_grid(femd_ctx ctx, int n)
+{
+    return grid_for((size_t)(n + 31) / 32, RED_BLOCK / 32, (unsigned)ctx->sm_count * SL_BLOCKS * 2);
+}
+
+// Whether the solves on this matrix use the slices: not where they would be filled up by over a fifth
+// (very uneven rows), nor where a shape of the lane groups was chosen for the matrix.
+static int use_slices(femd_ctx ctx, femd_matrix K, bool *use)
+{
+    femd_pattern P = K->pattern;
+    const int n = P->nrows, nsl = (n + 31) / 32;
+    *use = false;
+    if (K->spmv_tpr || n == 0) return FEMD_OK;
+    if (P->sl_state == 0) {
+        FEMD_TRY(reset_status(ctx));
+        k_slice_widths<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(P->indptr.p, n, nsl,
+                                                                                                     ctx->status_dev + 2, nullptr);
+        FEMD_TRY_CUDA(cudaGetLastError());
+        FEMD_TRY(read_status(ctx, nullptr, nullptr));
+        P->sl_slots = 32ll * ctx->status_host[2];
+        P->sl_state = P->sl_slots <= P->nnz + P->nnz / 5 + 4096 ? 1 : -1;
+    }
+    *use = P->sl_state == 1;
+    return FEMD_OK;
+}
+
+// The slices' places and columns, once per pattern.
+static int slice_layout(femd_ctx ctx, femd_pattern P)
+{
+    if (P->sl_col.p) return FEMD_OK;
+    const int n = P->nrows, nsl = (n + 31) / 32;
+    cudaStream_t s = ctx->stream;
+    DevBuf<int> width, tmp;
+    FEMD_TRY(width.alloc((size_t)nsl + 1));
+    FEMD_TRY(tmp.alloc(scan_tmp_ints((size_t)nsl + 1)));
+    FEMD_TRY(P->sl_ptr.alloc((size_t)nsl + 1));
+    DevBuf<int> cols;
+    FEMD_TRY(cols.alloc((size_t)P->sl_slots + 1));
+    FEMD_TRY_CUDA(cudaMemsetAsync(width.p + nsl, 0, sizeof(int), s));
+    const unsigned grid = grid_for((size_t)nsl, RED_BLOCK / 32);
+    k_slice_widths<<<grid, RED_BLOCK, 0, counted(s)>>>(P->indptr.p, n, nsl, nullptr, width.p);
+    FEMD_TRY_CUDA(cudaGetLastError());
+    FEMD_TRY(exclusive_scan_int(width.p, P->sl_ptr.p, (size_t)nsl + 1, tmp.p, s));
+    k_slice_fill<<<grid, RED_BLOCK, 0, counted(s)>>>(P->indptr.p, P->indices.p, nullptr, nullptr, P->sl_ptr.p, n, nsl, cols.p,
+                                                    nullptr, nullptr);
+    FEMD_TRY_CUDA(cudaGetLastError());
+    FEMD_TRY_CUDA(cudaStreamSynchronize(s));   // width and tmp are released here
+    std::swap(P->sl_col.p, cols.p);
+    std::swap(P->sl_col.n, cols.n);
+    return FEMD_OK;
+}
+
 // The solver workspace of a matrix: vectors, reduction partials, device and pinned host state,
 // events, and the CUDA graphs of a chunk of iterations.  The graphs run on the workspace's own
 // solution and right-hand-side vectors (wx, wb), so their pointers never change and a graph is
@@ -617,8 +889,12 @@ unsigned spmv_grid(femd_ctx ctx, int n, int shape)
 // matrix, a solve makes no allocation, capture or instantiation.
 struct SolverWS {
     int n = 0, shape = 0;
-    unsigned gs = 0, gr = 0;
+    unsigned gs = 0, gr = 0, gl = 0;             // grids of the lane-group SpMV, the reductions, the sliced SpMV
+    bool slices = false;
+    unsigned npap() const { return slices ? gl : gs; }       // partials of p.Ap, at the front of part
+    unsigned upd() const { return std::max(gs, gl); }        // where the update's begin
     // FP64
+    DevBuf<double> sv;                           // the matrix's values in slices, taken at the start of a solve
     DevBuf<double> r, p, Ap, part, wx, wb;
     DevBuf<CGState<double>> st;
     CGState<double> *st_host = nullptr;
@@ -661,8 +937,10 @@ static void solver_ws_free(void *w) { delete static_cast<SolverWS *>(w); }
 static int get_ws(femd_ctx ctx, femd_matrix K, SolverWS **out)
 {
     const int n = K->pattern->nrows, shape = pick_tpr(K);
+    bool slices = false;
+    FEMD_TRY(use_slices(ctx, K, &slices));
     SolverWS *W = static_cast<SolverWS *>(K->solver_ws);
-    if (W && W->n == n && W->shape == shape) { *out = W; return FEMD_OK; }
+    if (W && W->n == n && W->shape == shape && W->slices == slices) { *out = W; return FEMD_OK; }
     if (W) { solver_ws_free(W); K->solver_ws = nullptr; K->solver_ws_free = nullptr; }
     W = new SolverWS();
     std::unique_ptr<SolverWS> guard(W);
@@ -670,8 +948,10 @@ static int get_ws(femd_ctx ctx, femd_matrix K, SolverWS **out)
     W->shape = shape;
     W->gs = spmv_grid(ctx, n, shape);
     W->gr = red_grid(ctx, n);
+    W->gl = slices_grid(ctx, n);
+    W->slices = slices;
     for (DevBuf<double> *b : {&W->r, &W->p, &W->Ap, &W->wx, &W->wb}) FEMD_TRY(b->alloc((size_t)n + 1));
-    FEMD_TRY(W->part.alloc(3 * (size_t)std::max(W->gs, W->gr) + 3));
+    FEMD_TRY(W->part.alloc(3 * (size_t)std::max({W->gs, W->gr, W->gl}) + 3));
     FEMD_TRY(W->st.alloc(1));
     FEMD_TRY_CUDA(cudaMallocHost(&W->st_host, sizeof(CGState<double>)));
     FEMD_TRY_CUDA(cudaMallocHost(&W->maxit_host, sizeof(int)));
@@ -686,6 +966,46 @@ static int get_ws(femd_ctx ctx, femd_matrix K, SolverWS **out)
     return FEMD_OK;
 }
 
+// The update and the direction of FP64 iteration k (place = k % 2): the SpMV's npap partials at part,
+// the update's at part + upd.
+static void update_direction(bool jac, double *x, double *r, double *p, const double *Ap, const double *inv, int n, double *part,
+                             unsigned npap, unsigned upd, unsigned gr, CGState<double> *st, int place, cudaStream_t s)
+{
+    if (jac) {
+        k_cg_update<double, true><<<gr, RED_BLOCK, 0, counted(s)>>>(x, r, p, Ap, inv, n, part, npap, part + upd, st, place);
+        k_cg_direction<double, true, false, false><<<gr, RED_BLOCK, 0, counted(s)>>>(p, r, inv, n, part + upd, gr, st, place);
+    } else {
+        k_cg_update<double, false><<<gr, RED_BLOCK, 0, counted(s)>>>(x, r, p, Ap, nullptr, n, part, npap, part + upd, st, place);
+        k_cg_direction<double, false, false, false><<<gr, RED_BLOCK, 0, counted(s)>>>(p, r, nullptr, n, part + upd, gr, st, place);
+    }
+}
+
+// The FP64 SpMV of a solve on its workspace (y = A x; DOT: with x.y and alpha)
+template <bool DOT>
+static void solve_spmv(femd_matrix K, SolverWS &W, const double *x, double *y, cudaStream_t s)
+{
+    femd_pattern P = K->pattern;
+    if (W.slices)
+        k_spmv_slices<double, double, DOT><<<W.gl, RED_BLOCK, 0, counted(s)>>>(P->sl_ptr.p, P->sl_col.p, W.sv.p, x, y, W.n, W.part.p,
+                                                                              W.st.p);
+    else
+        launch_spmv<double, double, DOT>(W.shape, W.gs, s, P->indptr.p, P->indices.p, K->data.p, x, y, W.n, W.part.p, W.st.p);
+}
+
+// The values in slices, at the start of every solve (they may have changed since the last)
+static int take_values(femd_ctx ctx, femd_matrix K, SolverWS &W)
+{
+    if (!W.slices) return FEMD_OK;
+    femd_pattern P = K->pattern;
+    FEMD_TRY(slice_layout(ctx, P));
+    if (!W.sv.p) FEMD_TRY(W.sv.alloc((size_t)P->sl_slots + 1));
+    const int nsl = (W.n + 31) / 32;
+    k_slice_fill<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(
+        P->indptr.p, P->indices.p, K->data.p, nullptr, P->sl_ptr.p, W.n, nsl, nullptr, W.sv.p, nullptr);
+    FEMD_TRY_CUDA(cudaGetLastError());
+    return FEMD_OK;
+}
+
 // Capture CH iterations of the FP64 loop on the workspace vectors (once per matrix and variant).
 static int capture_cg64(femd_ctx ctx, femd_matrix K, SolverWS &W, bool jac)
 {
@@ -696,17 +1016,8 @@ static int capture_cg64(femd_ctx ctx, femd_matrix K, SolverWS &W, bool jac)
     cudaGraph_t graph = nullptr;
     FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < W.ch64; ++k) {
-        launch_spmv<double, double, true>(W.shape, W.gs, s, P->indptr.p, P->indices.p, K->data.p, W.p.p, W.Ap.p, n, W.part.p,
-                                          W.st.p);
-        if (jac) {
-            k_cg_update<double, true><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, K->inv.p, n, W.part.p,
-                                                                          W.st.p, 0);
-            k_cg_direction<double, true><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.r.p, K->inv.p, n, W.st.p);
-        } else {
-            k_cg_update<double, false><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, nullptr, n, W.part.p,
-                                                                           W.st.p, 0);
-            k_cg_direction<double, false><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.r.p, nullptr, n, W.st.p);
-        }
+        solve_spmv<true>(K, W, W.p.p, W.Ap.p, s);
+        update_direction(jac, W.wx.p, W.r.p, W.p.p, W.Ap.p, K->inv.p, n, W.part.p, W.npap(), W.upd(), W.gr, W.st.p, k & 1, s);
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
     if (ce != cudaSuccess) { set_error(std::string("cg: graph capture: ") + cudaGetErrorString(ce)); return FEMD_ECUDA; }
@@ -794,16 +1105,17 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     SolverWS *Wp = nullptr;
     FEMD_TRY(get_ws(ctx, K, &Wp));
     SolverWS &W = *Wp;
+    FEMD_TRY_CUDA(cudaEventRecord(W.e0, s));
+    FEMD_TRY(take_values(ctx, K, W));
     FEMD_TRY(capture_cg64(ctx, K, W, jac));
-    const unsigned gs = W.gs, gr = W.gr;
+    const unsigned gr = W.gr;
     const int CH = W.ch64;
     *W.maxit_host = max_iter;
-    FEMD_TRY_CUDA(cudaEventRecord(W.e0, s));
     FEMD_TRY_CUDA(cudaMemcpyAsync(W.wb.p, b, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     FEMD_TRY_CUDA(cudaMemcpyAsync(W.wx.p, x, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     FEMD_TRY_CUDA(cudaMemsetAsync(W.st.p, 0, sizeof(CGState<double>), s));
     // start (cg.hpp:305-320)
-    launch_spmv<double, double, false>(W.shape, gs, s, P->indptr.p, P->indices.p, K->data.p, W.wx.p, W.Ap.p, n, nullptr, nullptr);
+    solve_spmv<false>(K, W, W.wx.p, W.Ap.p, s);
     if (jac) k_cg_start<true><<<gr, RED_BLOCK, 0, counted(s)>>>(W.wb.p, W.Ap.p, W.r.p, W.p.p, K->inv.p, n, W.part.p, W.st.p, tol);
     else k_cg_start<false><<<gr, RED_BLOCK, 0, counted(s)>>>(W.wb.p, W.Ap.p, W.r.p, W.p.p, nullptr, n, W.part.p, W.st.p, tol);
     FEMD_TRY_CUDA(cudaGetLastError());
@@ -836,8 +1148,7 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     if (ce != cudaSuccess) { set_error(std::string("cg: ") + cudaGetErrorString(ce)); status = FEMD_ECUDA; }
     // finish (cg.hpp:222-237)
     if (status == FEMD_OK) {
-        launch_spmv<double, double, false>(W.shape, gs, s, P->indptr.p, P->indices.p, K->data.p, W.wx.p, W.Ap.p, n, nullptr,
-                                           nullptr);
+        solve_spmv<false>(K, W, W.wx.p, W.Ap.p, s);
         k_cg_finish<<<gr, RED_BLOCK, 0, counted(s)>>>(W.wb.p, W.Ap.p, W.r.p, n, W.part.p, W.st.p);
         ce = cudaMemcpyAsync(W.st_host, W.st.p, sizeof(CGState<double>), cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(x, W.wx.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s);
@@ -890,17 +1201,29 @@ int f32_rowsum_copy(femd_pattern P, const double *a, const int *dst, float *a32,
     return FEMD_OK;
 }
 
-static int ensure_f32(femd_ctx ctx, femd_matrix K)
+// The matrix's FP32 copies, in slices or as the CSR has the entries
+static int ensure_f32(femd_ctx ctx, femd_matrix K, bool slices)
 {
-    if (K->f32_valid) return FEMD_OK;
-    const long long nnz = K->pattern->nnz;
-    const int n = K->pattern->nrows;
-    if (!K->data32.p) FEMD_TRY(K->data32.alloc((size_t)nnz + 1));
+    if (K->f32_valid && K->f32_slices == slices) return FEMD_OK;
+    femd_pattern P = K->pattern;
+    const int n = P->nrows;
+    const size_t room = (size_t)(slices ? P->sl_slots : P->nnz) + 1;
+    if (K->data32.n < room) FEMD_TRY(K->data32.alloc(room));
     if (!K->inv32.p) FEMD_TRY(K->inv32.alloc((size_t)n + 1));
-    FEMD_TRY(f32_rowsum_copy(K->pattern, K->data.p, nullptr, K->data32.p, ctx->stream));
+    if (slices) {
+        if (!P->all_diag) return f32_rowsum_copy(P, K->data.p, nullptr, nullptr, ctx->stream);   // its error
+        FEMD_TRY(slice_layout(ctx, P));
+        const int nsl = (n + 31) / 32;
+        k_slice_fill<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(
+            P->indptr.p, P->indices.p, K->data.p, P->diag_pos.p, P->sl_ptr.p, n, nsl, nullptr, nullptr, K->data32.p);
+        FEMD_TRY_CUDA(cudaGetLastError());
+    } else {
+        FEMD_TRY(f32_rowsum_copy(P, K->data.p, nullptr, K->data32.p, ctx->stream));
+    }
     if (n) k_to_f32<<<grid_for((size_t)n, 256, 1u << 20), 256, 0, counted(ctx->stream)>>>(K->inv.p, K->inv32.p, n);
     FEMD_TRY_CUDA(cudaGetLastError());
     K->f32_valid = true;
+    K->f32_slices = slices;
     return FEMD_OK;
 }
 
@@ -911,7 +1234,7 @@ static int prepare_mixed(femd_ctx ctx, femd_matrix K, SolverWS &W)
     femd_pattern P = K->pattern;
     cudaStream_t s = ctx->stream;
     const int n = W.n;
-    const size_t npart = 3 * (size_t)std::max(W.gs, W.gr) + 3;
+    const size_t npart = 3 * (size_t)std::max({W.gs, W.gr, W.gl}) + 3;
     for (DevBuf<double> *b : {&W.Ax64, &W.r64}) FEMD_TRY(b->alloc((size_t)n + 1));
     for (DevBuf<float> *b : {&W.r32, &W.p32, &W.Ap32, &W.d32}) FEMD_TRY(b->alloc((size_t)n + 1));
     FEMD_TRY(W.part64.alloc(npart));
@@ -926,11 +1249,16 @@ static int prepare_mixed(femd_ctx ctx, femd_matrix K, SolverWS &W)
     cudaGraph_t graph = nullptr;
     FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < W.chm; ++k) {
-        launch_spmv<float, float, true>(W.shape, gs, s, P->indptr.p, P->indices.p, K->data32.p, W.p32.p, W.Ap32.p, n,
-                                        W.part32.p, W.st32.p);
+        if (W.slices)
+            k_spmv_slices<float, float, true><<<W.gl, RED_BLOCK, 0, counted(s)>>>(P->sl_ptr.p, P->sl_col.p, K->data32.p, W.p32.p,
+                                                                                 W.Ap32.p, n, W.part32.p, W.st32.p);
+        else
+            launch_spmv<float, float, true>(W.shape, gs, s, P->indptr.p, P->indices.p, K->data32.p, W.p32.p, W.Ap32.p, n,
+                                            W.part32.p, W.st32.p);
         k_cg_update<float, true><<<gr, RED_BLOCK, 0, counted(s)>>>(W.d32.p, W.r32.p, W.p32.p, W.Ap32.p, K->inv32.p, n, W.part32.p,
-                                                                   W.st32.p, 1);
-        k_cg_direction<float, true><<<gr, RED_BLOCK, 0, counted(s)>>>(W.p32.p, W.r32.p, K->inv32.p, n, W.st32.p);
+                                                                   W.npap(), W.part32.p + W.upd(), W.st32.p, k & 1);
+        k_cg_direction<float, true, true, false><<<gr, RED_BLOCK, 0, counted(s)>>>(W.p32.p, W.r32.p, K->inv32.p, n,
+                                                                                  W.part32.p + W.upd(), gr, W.st32.p, k & 1);
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
     if (ce != cudaSuccess) { set_error(std::string("pcg_mixed: graph capture: ") + cudaGetErrorString(ce)); return FEMD_ECUDA; }
@@ -962,7 +1290,7 @@ static void mixed_ru(femd_ctx ctx, femd_matrix K, SolverWS &W)
     default: k_mixed_spmv64<32><<<gs, RED_BLOCK, 0, counted(s)>>>(P->indptr.p, P->indices.p, K->data.p, x, W.Ax64.p, n, W.st32.p); break;
     }
     k_mixed_residual<<<gr, RED_BLOCK, 0, counted(s)>>>(b, W.Ax64.p, W.r32.p, K->inv32.p, n, W.part64.p, W.part32.p, W.st32.p);
-    k_cg_direction<float, true><<<gr, RED_BLOCK, 0, counted(s)>>>(W.p32.p, W.r32.p, K->inv32.p, n, W.st32.p);
+    k_cg_direction<float, true, true, true><<<gr, RED_BLOCK, 0, counted(s)>>>(W.p32.p, W.r32.p, K->inv32.p, n, nullptr, 0, W.st32.p, 0);
 }
 
 // Mixed precision solve: inner FP32 Jacobi-PCG with reliable FP64 updates, on the workspace.
@@ -972,10 +1300,10 @@ static int mixed_run(femd_ctx ctx, femd_matrix K, const double *b_in, double *x_
     femd_pattern P = K->pattern;
     const int n = P->nrows;
     cudaStream_t s = ctx->stream;
-    FEMD_TRY(ensure_f32(ctx, K));
     SolverWS *Wp = nullptr;
     FEMD_TRY(get_ws(ctx, K, &Wp));
     SolverWS &W = *Wp;
+    FEMD_TRY(ensure_f32(ctx, K, W.slices));
     FEMD_TRY(prepare_mixed(ctx, K, W));
     const unsigned gs = W.gs, gr = W.gr;
     double *x = W.wx.p;
@@ -1007,7 +1335,7 @@ static int mixed_run(femd_ctx ctx, femd_matrix K, const double *b_in, double *x_
     // FP32 state seeded from the FP64 start
     CGState<float> &s32 = *W.st32_host;
     s32 = CGState<float>{};
-    s32.rz = s64.rz;
+    s32.rz[0] = s32.rz[1] = s64.rz[0];
     s32.nb = s64.nb;
     s32.tol_nb = s64.tol_nb;
     s32.rn = s64.rn;
@@ -1098,7 +1426,7 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
         for (int k = 0; k < W.chpc && st == FEMD_OK; ++k) {
             launch_spmv<double, double, true>(W.shape, gs, s, Q->indptr.p, Q->indices.p, K->data.p, W.p.p, W.Ap.p, n, W.part.p,
                                               W.st.p);
-            k_pc_update<<<gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, n, W.part.p, W.st.p);
+            k_pc_update<<<gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, n, W.part.p, gs, W.part.p + W.upd(), W.st.p);
             st = precond_enqueue(P, W.r.p, W.z.p, done, s);
             k_pc_rz<false><<<gr, RED_BLOCK, 0, counted(s)>>>(W.r.p, W.z.p, nullptr, n, W.part.p, W.st.p);
             k_pc_direction<<<gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.z.p, n, W.st.p);
@@ -1463,27 +1791,29 @@ int femd_cuda_kernel_time(femd_ctx ctx, femd_matrix K, int kernel, int reps, dou
     FEMD_TRY(get_ws(ctx, K, &Wp));
     SolverWS &W = *Wp;
     cudaStream_t s = ctx->stream;
-    femd_pattern P = K->pattern;
+    FEMD_TRY(take_values(ctx, K, W));
     // a state that never stops the loop: max_iter huge, r = p = D^-1 (so ||r||, r.z and p.Ap stay
-    // positive for an SPD matrix), alpha and beta 0 (every launch streams the same bytes and leaves
-    // the vectors as they are)
+    // positive for an SPD matrix), the partials of the other kernels' sums huge: alpha is 0, and the
+    // test does not fire (every launch streams the same bytes)
     CGState<double> S{};
-    S.rz = 1.0;
+    S.rz[0] = S.rz[1] = 1.0;
     S.max_iter = INT_MAX;
     *W.st_host = S;
     const unsigned gn = grid_for((size_t)n, 256, 1u << 20);
     k_combine<<<gn, 256, 0, counted(s)>>>(1.0, K->inv.p, 0.0, K->inv.p, W.r.p, n);
     k_combine<<<gn, 256, 0, counted(s)>>>(1.0, K->inv.p, 0.0, K->inv.p, W.p.p, n);
     FEMD_TRY_CUDA(cudaMemsetAsync(W.wx.p, 0, (size_t)n * sizeof(double), s));
+    FEMD_TRY_CUDA(cudaMemsetAsync(W.Ap.p, 0, (size_t)n * sizeof(double), s));
+    FEMD_TRY_CUDA(cudaMemsetAsync(W.part.p, 0x7f, W.part.n * sizeof(double), s));
     auto one = [&]() {
         if (kernel == 0)
-            launch_spmv<double, double, true>(W.shape, W.gs, s, P->indptr.p, P->indices.p, K->data.p, W.p.p, W.Ap.p, n, W.part.p,
-                                              W.st.p);
+            solve_spmv<true>(K, W, W.p.p, W.Ap.p, s);
         else if (kernel == 1)
-            k_cg_update<double, true><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, K->inv.p, n, W.part.p,
-                                                                          W.st.p, 0);
+            k_cg_update<double, true><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, K->inv.p, n, W.part.p, W.npap(),
+                                                                          W.part.p + W.upd(), W.st.p, 0);
         else
-            k_cg_direction<double, true><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.r.p, K->inv.p, n, W.st.p);
+            k_cg_direction<double, true, false, false><<<W.gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.r.p, K->inv.p, n,
+                                                                                          W.part.p + W.upd(), W.gr, W.st.p, 0);
     };
     for (int w = 0; w < 3; ++w) {
         FEMD_TRY_CUDA(cudaMemcpyAsync(W.st.p, W.st_host, sizeof(CGState<double>), cudaMemcpyHostToDevice, s));
@@ -1571,7 +1901,8 @@ int femd_cuda_cg_solve_host(femd_ctx ctx, int n, const int *indptr_host, const i
 // and the device synchronization it may bring are not allowed.  The three work vectors, the
 // reduction partials and the scalar state of the solve live in one fixed static device array,
 // g_cg_scratch, sized for NOALLOC_MAX_ROWS rows; larger systems are rejected.  The kernels and
-// launch shapes are those of femd_cuda_cg_jacobi, so the iterates are the same.
+// launch shapes are those of femd_cuda_cg_jacobi, so the iterates are the same (the sliced
+// SpMV's sums are formed from the CSR: the slices would be an allocation).
 // ==============================================================================================
 namespace femd {
 
@@ -1675,7 +2006,9 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     const femd_pattern P = K->pattern;
     const bool jac = use_jacobi != 0;
     const int tpr = pick_tpr(K);
-    const unsigned gs = spmv_grid(ctx, n, tpr), gr = red_grid(ctx, n);
+    bool slices = false;
+    FEMD_TRY(use_slices(ctx, K, &slices));
+    const unsigned gs = slices ? slices_grid(ctx, n) : spmv_grid(ctx, n, tpr), gr = red_grid(ctx, n);
     FEMD_CHECK_ARG(3 * (size_t)std::max(gs, gr) + 3 <= (size_t)NOALLOC_PART,
                    "cg_jacobi_noalloc: the device has more blocks than the fixed reduction scratch holds");
     double *r = base, *p = base + NOALLOC_MAX_ROWS, *Ap = base + 2 * (size_t)NOALLOC_MAX_ROWS;
@@ -1694,7 +2027,14 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     // the array keeps the previous call's contents: the state (with its reduction ticket) must
     // start at zero; r, p, Ap and the partials are written before they are read
     FEMD_TRY_CUDA(cudaMemsetAsync(st, 0, sizeof(CGState<double>), s));
-    launch_spmv<double, double, false>(tpr, gs, s, P->indptr.p, P->indices.p, K->data.p, x_dev, Ap, n, nullptr, nullptr);
+    auto spmv = [&](auto dot, const double *v) {
+        constexpr bool DOT = decltype(dot)::value;
+        if (slices)
+            k_spmv_csr_slices<DOT><<<gs, RED_BLOCK, 0, counted(s)>>>(P->indptr.p, P->indices.p, K->data.p, v, Ap, n, part, st);
+        else
+            launch_spmv<double, double, DOT>(tpr, gs, s, P->indptr.p, P->indices.p, K->data.p, v, Ap, n, part, st);
+    };
+    spmv(std::false_type(), x_dev);
     if (jac) k_cg_start<true><<<gr, RED_BLOCK, 0, counted(s)>>>(b_dev, Ap, r, p, K->inv.p, n, part, st, tol);
     else k_cg_start<false><<<gr, RED_BLOCK, 0, counted(s)>>>(b_dev, Ap, r, p, nullptr, n, part, st, tol);
     FEMD_TRY_CUDA(cudaGetLastError());
@@ -1704,14 +2044,8 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     const long long max_chunks = (long long)max_iter / CH + 2;
     for (long long c = 0; c < max_chunks; ++c) {
         for (int k = 0; k < CH; ++k) {
-            launch_spmv<double, double, true>(tpr, gs, s, P->indptr.p, P->indices.p, K->data.p, p, Ap, n, part, st);
-            if (jac) {
-                k_cg_update<double, true><<<gr, RED_BLOCK, 0, counted(s)>>>(x_dev, r, p, Ap, K->inv.p, n, part, st, 0);
-                k_cg_direction<double, true><<<gr, RED_BLOCK, 0, counted(s)>>>(p, r, K->inv.p, n, st);
-            } else {
-                k_cg_update<double, false><<<gr, RED_BLOCK, 0, counted(s)>>>(x_dev, r, p, Ap, nullptr, n, part, st, 0);
-                k_cg_direction<double, false><<<gr, RED_BLOCK, 0, counted(s)>>>(p, r, nullptr, n, st);
-            }
+            spmv(std::true_type(), p);
+            update_direction(jac, x_dev, r, p, Ap, K->inv.p, n, part, gs, gs, gr, st, k & 1, s);
         }
         FEMD_TRY_CUDA(cudaGetLastError());
         FEMD_TRY_CUDA(cudaMemcpyAsync(&S, st, sizeof(S), cudaMemcpyDeviceToHost, s));
@@ -1719,7 +2053,7 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
         if (S.done) break;
     }
     // final true residual (cg.hpp:222-237)
-    launch_spmv<double, double, false>(tpr, gs, s, P->indptr.p, P->indices.p, K->data.p, x_dev, Ap, n, nullptr, nullptr);
+    spmv(std::false_type(), x_dev);
     k_cg_finish<<<gr, RED_BLOCK, 0, counted(s)>>>(b_dev, Ap, r, n, part, st);
     FEMD_TRY_CUDA(cudaGetLastError());
     FEMD_TRY_CUDA(cudaMemcpyAsync(&S, st, sizeof(S), cudaMemcpyDeviceToHost, s));
