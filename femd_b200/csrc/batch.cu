@@ -872,10 +872,9 @@ static BatchKernel batch_kernel(bool mixed, int block, int npt)
 // a member's iterates depend on the member alone, whatever else is in the batch.
 
 struct LState {
-    double rz, alpha, beta, nb, maxr, rz_prev, rn_rec, prt, res;
+    double rz, beta, nb, maxr, rz_prev, rn_rec, prt, res;
     int it, done, want_ru, breakdown, conv, rus, stall, fallback, zero, started;
-    unsigned t1, t2, t3;   // last-block tickets of the SpMV, the update and the residual
-    int pad;
+    unsigned t2, t3;       // last-block tickets of the update and the residual
 };
 
 struct LBlock {
@@ -884,12 +883,16 @@ struct LBlock {
 };
 
 static constexpr int LS_BB = 256;
+// Mixed precision: the reliable updates' kernels follow every LS_RU-th iteration (and a chunk's last).
+// Nearly always they find nothing to do, at 5 us a pair; a member waits for them up to 3 iterations,
+// a dozen times in a solve.
+static constexpr int LS_RU = 4;
 
 // y = A g on rows [r0, r1) with TPR lanes per row; out(row, sum) by the row's first lane
-template <int TPR, class V, class F, class Gather, class Pre, class Out>
+template <int BB, int TPR, class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_rows(const BProb &P, const V *A, int r0, int r1, Gather g, Pre pre, Out out)
 {
-    constexpr int U = 4, GPW = 32 / TPR, STEP = (LS_BB / 32) * GPW;
+    constexpr int U = 4, GPW = 32 / TPR, STEP = (BB / 32) * GPW;
     const int lane = threadIdx.x % TPR;
     const int sub = (int)(threadIdx.x & 31) / TPR;
     int i0 = r0 + (int)(threadIdx.x >> 5) * GPW;
@@ -945,10 +948,11 @@ __device__ __forceinline__ void ls_rows(const BProb &P, const V *A, int r0, int 
 // high part is the row's diagonal entry, its low part comes with the row's table entry and is
 // added last, so the FP32 matrix keeps the FP64 matrix's row sums.
 //
-// The warp is latency-bound (a chain of dependent loads per slice), so: SELL_U entries per round,
+// The warp is latency-bound (a chain of dependent loads per slice), so: SELL_U entries per round (10: the usual rows are 7, 9,
+// 10, 16, 19 and 37 long; 12 and 8 took 2 and 7 % more on a dozen members),
 // the next slice's table entries loaded one slice ahead, and the first slice's table entries and
 // first round loaded by sell_prime before the block's window is staged (they do not need it).
-static constexpr int SELL_U = 12;
+static constexpr int SELL_U = 10;
 struct SellCursor {
     int base, width, base1, end1;   // this slice's first position and width; the next slice's bounds
     float dl, dl1;                  // this lane's row's low diagonal part, this slice's and the next's
@@ -981,21 +985,23 @@ __device__ __forceinline__ void sell_round(const BProb &P, const float *__restri
     }
 }
 
+template <int BB>
 __device__ __forceinline__ void sell_prime(const BProb &P, const float *__restrict__ A, int r0, int r1, SellCursor &c)
 {
     const int s0 = r0 + (int)(threadIdx.x >> 5) * 32;
     int end;
     sell_header(P, s0, r1, c.base, end, c.dl);
     c.width = (end - c.base) >> 5;
-    sell_header(P, s0 + LS_BB, r1, c.base1, c.end1, c.dl1);
+    sell_header(P, s0 + BB, r1, c.base1, c.end1, c.dl1);
     sell_round(P, A, c.base, c.width, 0, c.o, c.v);
 }
 
+template <int BB>
 __device__ __forceinline__ void ls_rows_sell(const BProb &P, const float *__restrict__ A, const float *win, int c0, int r0,
                                              int r1, float *__restrict__ Ap, double &dot, SellCursor &c)
 {
     const int lane = threadIdx.x & 31;
-    for (int s0 = r0 + (int)(threadIdx.x >> 5) * 32; s0 < r1; s0 += LS_BB) {
+    for (int s0 = r0 + (int)(threadIdx.x >> 5) * 32; s0 < r1; s0 += BB) {
         const int i = s0 + lane;
         const bool ok = i < r1;                                  // lanes past the member's last row: padding
         const float *wrow = win + (ok ? i - c0 : 0);
@@ -1016,20 +1022,21 @@ __device__ __forceinline__ void ls_rows_sell(const BProb &P, const float *__rest
         c.base = c.base1;
         c.width = (c.end1 - c.base1) >> 5;
         c.dl = c.dl1;
-        sell_header(P, s0 + 2 * LS_BB, r1, c.base1, c.end1, c.dl1);
-        if (s0 + LS_BB < r1) sell_round(P, A, c.base, c.width, 0, c.o, c.v);
+        sell_header(P, s0 + 2 * BB, r1, c.base1, c.end1, c.dl1);
+        if (s0 + BB < r1) sell_round(P, A, c.base, c.width, 0, c.o, c.v);
     }
 }
 
 // SpMV windows: whole rows with at most LS_W nonzeros each (a window's rows start within LS_W -
 // maxlen nonzeros of each other).  A window's column indices and values are read by coalesced
-// loads, LS_NPT per thread, all issued before the gathers; the products go to shared memory
+// loads, LS_W / BB per thread, all issued before the gathers; the products go to shared memory
 // (two buffers, one barrier per window) and each row is summed in order by one thread.
-static constexpr int LS_NPT = 4, LS_W = LS_BB * LS_NPT;
+static constexpr int LS_W = 1024;
 
-template <class V, class F, class Gather, class Pre, class Out>
+template <int BB, class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, int w1, Gather g, Pre pre, Out out)
 {
+    constexpr int LS_NPT = LS_W / BB;
     __shared__ F prod[2][LS_W];
     const int tid = (int)threadIdx.x;
     for (int w = w0; w < w1; ++w) {
@@ -1040,7 +1047,7 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
         V a[LS_NPT];
 #pragma unroll
         for (int t = 0; t < LS_NPT; ++t) {
-            const int q = qs + t * LS_BB + tid;
+            const int q = qs + t * BB + tid;
             col[t] = q < qe ? __ldcs(&P.indices[q]) : -1;
             a[t] = q < qe ? __ldcs(&A[q]) : V(0);
         }
@@ -1055,9 +1062,9 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
         for (int t = 0; t < LS_NPT; ++t) gv[t] = col[t] >= 0 ? g(col[t]) : F(0);
 #pragma unroll
         for (int t = 0; t < LS_NPT; ++t)
-            if (col[t] >= 0) pb[t * LS_BB + tid] = (F)a[t] * gv[t];
+            if (col[t] >= 0) pb[t * BB + tid] = (F)a[t] * gv[t];
         __syncthreads();
-        for (int row = row0; row < re; row += LS_BB) {
+        for (int row = row0; row < re; row += BB) {
             if (row != row0) {
                 lo = P.indptr[row];
                 hi = P.indptr[row + 1];
@@ -1070,30 +1077,45 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
 }
 
 // y = A g over an entry: by windows when the member has a window table, else by row groups
-template <class V, class F, class Gather, class Pre, class Out>
+template <int BB, class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_spmv_entry(const BProb &P, const V *A, const LBlock &L, Gather g, Pre pre, Out out)
 {
     if (P.wrow) {
-        ls_windows<V, F>(P, A, L.w0, L.w1, g, pre, out);
+        ls_windows<BB, V, F>(P, A, L.w0, L.w1, g, pre, out);
         return;
     }
     switch (P.tpr) {
-    case 2: ls_rows<2, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 4: ls_rows<4, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 8: ls_rows<8, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 16: ls_rows<16, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    default: ls_rows<32, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 2: ls_rows<BB, 2, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 4: ls_rows<BB, 4, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 8: ls_rows<BB, 8, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 16: ls_rows<BB, 16, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    default: ls_rows<BB, 32, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
     }
+}
+
+// the block's sum of v, in every thread
+template <int BB>
+__device__ __forceinline__ double ls_block_sum(double v)
+{
+    __shared__ double sh[BB / 32];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < BB / 32; ++w) t += sh[w];
+    __syncthreads();
+    return t;
 }
 
 // The member's totals of NV sums.  The block's sums go to part[k * NE + e]; in the member's last
 // block the function returns true (in every thread) with tot = the member's entry partials
 // summed in entry order, and resets the ticket.
-template <int NV>
+template <int BB, int NV>
 __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *part, int NE, int e, const LBlock &L,
                                               unsigned *ticket, double (&tot)[NV])
 {
-    __shared__ double sh[NV][LS_BB / 32];
+    __shared__ double sh[NV][BB / 32];
     __shared__ int last;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -1106,7 +1128,7 @@ __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *par
         for (int k = 0; k < NV; ++k) {
             double t = 0.0;
 #pragma unroll
-            for (int w = 0; w < LS_BB / 32; ++w) t += sh[k][w];
+            for (int w = 0; w < BB / 32; ++w) t += sh[k][w];
             part[(size_t)k * NE + e] = t;
         }
         __threadfence();
@@ -1119,14 +1141,14 @@ __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *par
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         double t = 0.0;
-        for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += LS_BB) t += __ldcg(part + (size_t)k * NE + b);
+        for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += BB) t += __ldcg(part + (size_t)k * NE + b);
         t = warp_sum(t);
         __syncthreads();
         if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = t;
         __syncthreads();
         double u = 0.0;
 #pragma unroll
-        for (int w = 0; w < LS_BB / 32; ++w) u += sh[k][w];
+        for (int w = 0; w < BB / 32; ++w) u += sh[k][w];
         tot[k] = u;
     }
     __syncthreads();
@@ -1141,22 +1163,25 @@ __device__ __forceinline__ void ls_finish(LState &S, int *active)
 }
 
 // SpMV with the direction formed on the fly: p = z + beta pold (pold = 0 at the start); p.Ap.
-// Block 0 also empties the reliable-update list of the iteration.  Mixed precision: at most 64
-// registers, 4 blocks per SM. The sliced rows' 12 entries per round need them: at 5 blocks (51
-// registers) the rounds spilled and ran 33 % slower than at 4 (64 config-4 problems x 120
-// iterations). FP64: at most 51 registers, 5 blocks per SM.
+// Block 0 also empties the reliable-update list (clear: the launch after the reliable updates).  A
+// member that waits for its reliable update does nothing.  Mixed precision: at most 64 registers,
+// 32 warps per SM. The sliced rows' 10 entries per round need them: at 51 registers the rounds
+// spilled and ran 33 % slower (64 problems of the mixed-size stream x 120 iterations). FP64: at most
+// 51 registers, 5 blocks per SM.
 template <bool MIXED>
-__global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5) k_ls_spmv(const BProb *__restrict__ probs, const LBlock *__restrict__ blks, int NE,
-                                                   LState *st, double *part, int *active, int *ru_count)
+__global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5)
+    k_ls_spmv(const BProb *__restrict__ probs, const LBlock *__restrict__ blks, int NE, LState *st, double *part, int *active,
+              int *ru_count, int clear)
 {
+    constexpr int BB = LS_BB;
     using F = typename std::conditional<MIXED, float, double>::type;
     extern __shared__ float ls_win[];
-    if (MIXED && blockIdx.x == 0 && threadIdx.x == 0) *ru_count = 0;
+    if (MIXED && clear && blockIdx.x == 0 && threadIdx.x == 0) *ru_count = 0;
     const int e = blockIdx.x;
     const LBlock L = blks[e];
     const BProb P = probs[L.m];
     LState &S = st[L.m];
-    if (S.done) return;
+    if (S.done || (MIXED && S.want_ru)) return;
     const F *z = MIXED ? (const F *)P.z32 : (const F *)P.z64;
     F *pa = MIXED ? (F *)P.pa32 : (F *)P.pa64;
     F *pb = MIXED ? (F *)P.pb32 : (F *)P.pb64;
@@ -1178,18 +1203,18 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5) k_ls_spmv(const BProb *_
         float *pn = (float *)pnew;
         const float bf = (float)beta;
         SellCursor cur;
-        sell_prime(P, (const float *)A, L.r0, L.r1, cur);
-        for (int w0 = c0 + (int)threadIdx.x; w0 < c1; w0 += WU * LS_BB) {
+        sell_prime<BB>(P, (const float *)A, L.r0, L.r1, cur);
+        for (int w0 = c0 + (int)threadIdx.x; w0 < c1; w0 += WU * BB) {
             float zv[WU], pv[WU];
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int w = w0 + u * LS_BB;
+                const int w = w0 + u * BB;
                 zv[u] = w < c1 ? zf[w] : 0.0f;
                 pv[u] = w < c1 ? pf[w] : 0.0f;
             }
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int w = w0 + u * LS_BB;
+                const int w = w0 + u * BB;
                 if (w < c1) {
                     const float pw = __fmaf_rn(bf, pv[u], zv[u]);
                     ls_win[w - c0] = pw;
@@ -1198,9 +1223,9 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5) k_ls_spmv(const BProb *_
             }
         }
         __syncthreads();
-        ls_rows_sell(P, (const float *)A, ls_win, c0, L.r0, L.r1, (float *)Ap, dot, cur);
+        ls_rows_sell<BB>(P, (const float *)A, ls_win, c0, L.r0, L.r1, (float *)Ap, dot, cur);
     } else {
-        ls_spmv_entry<F, F>(
+        ls_spmv_entry<BB, F, F>(
             P, A, L, [&](int j) { return pdir(z, pold, beta, j); }, [&](int i) { return pdir(z, pold, beta, i); },
             [&](int i, F s, F pi) {
                 pnew[i] = pi;
@@ -1208,16 +1233,9 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5) k_ls_spmv(const BProb *_
                 dot += (double)pi * (double)s;
             });
     }
-    const double v[1] = {dot};
-    double tot[1];
-    if (ls_member_sum<1>(v, part, NE, e, L, &S.t1, tot) && threadIdx.x == 0) {
-        if (!(tot[0] > 0.0)) {
-            S.breakdown = 1;
-            ls_finish(S, active);
-        } else {
-            S.alpha = S.rz / tot[0];
-        }
-    }
+    // the entry's share of p.Ap; the update's blocks add up the member's
+    dot = ls_block_sum<BB>(dot);
+    if (threadIdx.x == 0) part[2 * (size_t)NE + e] = dot;
 }
 
 // r -= alpha Ap, (x or d) += alpha p, z = inv r; ||r||^2 and r.z; then the member's stopping
@@ -1232,7 +1250,7 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
     const LBlock L = blks[e];
     const BProb P = probs[L.m];
     LState &S = st[L.m];
-    if (S.done) return;
+    if (S.done || (MIXED && S.want_ru)) return;
     F *r = MIXED ? (F *)P.r32 : (F *)P.r64;
     F *z = MIXED ? (F *)P.z32 : (F *)P.z64;
     const int it = S.it;
@@ -1240,13 +1258,12 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
     const F *Ap = MIXED ? (const F *)P.Ap32 : (const F *)P.Ap64;
     const F *inv = MIXED ? (const F *)P.inv32 : (const F *)P.inv64;
     F *acc = MIXED ? (F *)P.d32 : (F *)P.x;
-    const F alpha = (F)S.alpha;
-    double v[2] = {0.0, 0.0};
     // UU rows per thread and round (rows i, i + LS_BB, ...: the order of the sums is that of a
-    // row at a time), every load of the round issued before its stores
+    // row at a time), every load of the round issued before its stores, the first round's before alpha is
+    // known
     constexpr int UU = 4;
-    for (int i0 = L.r0 + (int)threadIdx.x; i0 < L.r1; i0 += UU * LS_BB) {
-        F rv[UU], av[UU], iv[UU], cv[UU], pv[UU];
+    F rv[UU], av[UU], iv[UU], cv[UU], pv[UU];
+    auto load = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < UU; ++u) {
             const int i = i0 + u * LS_BB;
@@ -1257,6 +1274,25 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
             cv[u] = ok ? acc[i] : F(0);
             pv[u] = ok ? p[i] : F(0);
         }
+    };
+    load(L.r0 + (int)threadIdx.x);
+    // alpha, by every block of the member from the SpMV's entries in one fixed tree (a last block that
+    // did it at the SpMV's end put 3 us behind every one)
+    const double rz0 = S.rz;
+    double pAp = 0.0;
+    for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += LS_BB) pAp += __ldcg(part + 2 * (size_t)NE + b);
+    pAp = ls_block_sum<LS_BB>(pAp);
+    if (!(pAp > 0.0)) {
+        if (e == L.b0 && threadIdx.x == 0) {
+            S.breakdown = 1;
+            ls_finish(S, active);
+        }
+        return;
+    }
+    const F alpha = (F)(rz0 / pAp);
+    double v[2] = {0.0, 0.0};
+    for (int i0 = L.r0 + (int)threadIdx.x; i0 < L.r1; i0 += UU * LS_BB) {
+        if (i0 != L.r0 + (int)threadIdx.x) load(i0);
 #pragma unroll
         for (int u = 0; u < UU; ++u) {
             const int i = i0 + u * LS_BB;
@@ -1272,7 +1308,7 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
         }
     }
     double tot[2];
-    if (!ls_member_sum<2>(v, part, NE, e, L, &S.t2, tot)) return;
+    if (!ls_member_sum<LS_BB, 2>(v, part, NE, e, L, &S.t2, tot)) return;
     if (threadIdx.x == 0) {
         s_ru = 0;
         const int it1 = it + 1;
@@ -1341,7 +1377,7 @@ __global__ void __launch_bounds__(LS_BB, 5) k_ls_resid(const BProb *__restrict__
         F *pb = MIXED ? (F *)P.pb32 : (F *)P.pb64;
         const double *x = P.x;
         double v[3] = {0.0, 0.0, 0.0};
-        ls_spmv_entry<double, double>(
+        ls_spmv_entry<LS_BB, double, double>(
             P, P.A64, L, [&](int j) { return x[j]; },
             [&](int i) { return make_double2(P.b[i], MODE == 2 ? 0.0 : P.inv64[i]); },
             [&](int i, double s, double2 own) {
@@ -1368,7 +1404,7 @@ __global__ void __launch_bounds__(LS_BB, 5) k_ls_resid(const BProb *__restrict__
                 }
             });
         double tot[3];
-        if (!ls_member_sum<3>(v, part, NE, e, L, &S.t3, tot) || threadIdx.x != 0) continue;
+        if (!ls_member_sum<LS_BB, 3>(v, part, NE, e, L, &S.t3, tot) || threadIdx.x != 0) continue;
         const double rn = sqrt(tot[0]);
         if (MODE == 0) {
             const double nb = sqrt(tot[2]);
@@ -2271,18 +2307,21 @@ static int ls_run(femd_ctx ctx, femd_batch_s *B, const std::vector<int> &ids, bo
     if (mx) FEMD_TRY_CUDA(cudaFuncSetAttribute(k_ls_spmv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)(CL_WIN_MAX * sizeof(float))));
     const int C = std::max(1, B->ls_chunk);
-    const long long max_chunks = (long long)max_it / C + 4;
+    // (a member may wait LS_RU - 1 iterations for each reliable update)
+    const long long max_chunks = (long long)max_it * (mx ? LS_RU : 1) / C + 4;
     int aborted = 0;
     for (long long j = 0; j <= max_chunks; ++j) {
         for (int c = 0; c < C; ++c) {
             if (mx) {
-                k_ls_spmv<true><<<NE, LS_BB, win_b, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_count);
+                k_ls_spmv<true><<<NE, LS_BB, win_b, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_count,
+                                                                  c % LS_RU == 0);
                 k_ls_update<true><<<NE, LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_list, ru_count);
+                if (c % LS_RU != LS_RU - 1 && c != C - 1) continue;
                 k_ls_flush<false><<<std::min(G1, NE), LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, ru_list, ru_count);
                 k_ls_resid<true, 1><<<std::min(G1, NE), LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active,
                                                                                  ru_list, ru_count);
             } else {
-                k_ls_spmv<false><<<NE, LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_count);
+                k_ls_spmv<false><<<NE, LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_count, 0);
                 k_ls_update<false><<<NE, LS_BB, 0, counted(s)>>>(d_desc.p, d_tab.p, NE, d_state.p, d_part.p, active, ru_list,
                                                                    ru_count);
             }
@@ -2573,16 +2612,18 @@ static int ls_advance(femd_ctx ctx, femd_batch_s *B, bool mx, int chunks, int *n
         for (int c = 0; c < C; ++c) {
             if (NE32) {
                 k_ls_spmv<true><<<NE32, LS_BB, win_b, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p, L.d_part.p, active,
-                                                                   ru_count);
+                                                                   ru_count, c % LS_RU == 0);
                 k_ls_update<true><<<NE32, LS_BB, 0, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p, L.d_part.p, active, ru_list,
                                                                  ru_count);
-                k_ls_flush<false><<<std::min(G1, NE32), LS_BB, 0, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p, ru_list,
-                                                                                ru_count);
-                k_ls_resid<true, 1><<<std::min(G1, NE32), LS_BB, 0, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p, L.d_part.p,
-                                                                                  active, ru_list, ru_count);
+                if (c % LS_RU == LS_RU - 1 || c == C - 1) {
+                    k_ls_flush<false><<<std::min(G1, NE32), LS_BB, 0, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p, ru_list,
+                                                                                    ru_count);
+                    k_ls_resid<true, 1><<<std::min(G1, NE32), LS_BB, 0, counted(s)>>>(L.d_desc.p, T32, NE32, L.d_state.p,
+                                                                                      L.d_part.p, active, ru_list, ru_count);
+                }
             }
             if (NE64) {
-                k_ls_spmv<false><<<NE64, LS_BB, 0, counted(s)>>>(L.d_desc.p, T64, NE64, L.d_state.p, L.d_part.p, active, ru_count);
+                k_ls_spmv<false><<<NE64, LS_BB, 0, counted(s)>>>(L.d_desc.p, T64, NE64, L.d_state.p, L.d_part.p, active, ru_count, 0);
                 k_ls_update<false><<<NE64, LS_BB, 0, counted(s)>>>(L.d_desc.p, T64, NE64, L.d_state.p, L.d_part.p, active, ru_list,
                                                                   ru_count);
             }
