@@ -872,17 +872,28 @@ __global__ void __launch_bounds__(128) k_pair_offsets(const int *__restrict__ rc
             const int *d = dofs + (size_t)(rc_code[c] / nloc) * nloc;
             for (int w = 0; w < offs / 4; ++w) {
                 unsigned word = 0xffffffffu;
+                int J[4], at[4];                              // four searches in step
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const int j = 4 * w + k, J = j < nloc ? d[j] : -1;
-                    if (J < 0) continue;
-                    int lo = 0, hi = len;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (row[mid] < J) lo = mid + 1; else hi = mid;
-                    }
-                    if (lo == len || row[lo] != J) atomicOr(status, ST_OUTSIDE);
-                    else word = (word & ~(0xffu << (8 * k))) | (unsigned)lo << (8 * k);
+                    J[k] = 4 * w + k < nloc ? d[4 * w + k] : -1;
+                    at[k] = 0;
+                }
+                for (int n = len; n > 1;) {
+                    const int h = n >> 1;
+                    int x[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) x[k] = row[at[k] + h - 1];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (x[k] < J[k]) at[k] += h;
+                    n -= h;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (J[k] < 0) continue;
+                    if (len && row[at[k]] < J[k]) ++at[k];
+                    if (at[k] == len || row[at[k]] != J[k]) atomicOr(status, ST_OUTSIDE);
+                    else word = (word & ~(0xffu << (8 * k))) | (unsigned)at[k] << (8 * k);
                 }
                 off[(size_t)c * (offs / 4) + w] = word;
             }
@@ -1103,7 +1114,6 @@ static int prepare_terms(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     return FEMD_OK;
 }
 
-static constexpr size_t ASM_SHARED = 32u << 20;   // doubles (256 MB) of the context's workspace
 static constexpr int FAST_MAX_ROW = 96;   // longest row the shared-memory accumulator holds
 
 // FAST assembly of a matrix (K non-null) or a vector (f non-null).  Tables and factors live in
@@ -1145,8 +1155,8 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     // the cells' factors, vectors or matrices: in the context's workspace up to its bound (the
     // context's stream orders the assemblies that share it), else in the pattern's own
     const size_t cells = (size_t)ne * per_cell + 1;
-    DevBuf<double> &W = cells <= ASM_SHARED ? ctx->asm_scratch : p->ws_factors;
-    if (W.n < cells) FEMD_TRY(W.alloc(std::min(cells + cells / 4, std::max(cells, ASM_SHARED))));
+    DevBuf<double> &W = cells <= CTX_SCRATCH ? ctx->asm_scratch : p->ws_factors;
+    if (W.n < cells) FEMD_TRY(W.alloc(std::min(cells + cells / 4, std::max(cells, CTX_SCRATCH))));
     // the slot holding these tables, else the least recently used one, refilled (stream-ordered,
     // so kernels still reading the slot's old tables finish first)
     femd_pattern_s::TableSlot *slot = nullptr;

@@ -86,6 +86,10 @@ struct DevBuf {
 
 }  // namespace femd
 
+namespace femd {
+static constexpr size_t CTX_SCRATCH = 32u << 20;   // doubles (256 MB)
+}
+
 struct femd_ctx_s {
     // handles that keep the context (patterns, matrices, batches) hold a reference each;
     // femd_cuda_ctx_destroy drops the creator's, and the last one frees the stream
@@ -100,7 +104,8 @@ struct femd_ctx_s {
     // most), pinned room for its result, and the events that time it
     femd::DevBuf<double> res_scratch;
     void *res_host = nullptr;
-    // the cells' factors, vectors or matrices of an assembly, up to 256 MB; a larger one's belong to its pattern
+    // scratch of an assembly (the cells' factors, vectors or matrices) and of a pattern's build, up to
+    // CTX_SCRATCH doubles; the context's stream orders what shares it
     femd::DevBuf<double> asm_scratch;
     cudaEvent_t res_e0 = nullptr, res_e1 = nullptr;
 };

@@ -43,20 +43,34 @@ __global__ void k_fill_rows(const int *__restrict__ dofs, long long total, int n
     }
 }
 
-// Sort each row's list (a handful of entries) by insertion: the fill order above is not
-// deterministic, the sorted order is.
-__global__ void k_sort_rows(const int *__restrict__ rc_ptr, int *__restrict__ rc_code, int nrows, int *__restrict__ maxcells)
+// Put a row's list in increasing order: the fill order above is not deterministic, the sorted order
+// is.  Up to 8 entries (a vertex has 6 cells in a regular mesh) by an odd-even exchange in registers,
+// more by insertion.
+__device__ __forceinline__ void sort_row(int *__restrict__ v, int m)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrows) return;
-    const int lo = rc_ptr[i], hi = rc_ptr[i + 1];
-    for (int a = lo + 1; a < hi; ++a) {
-        const int v = rc_code[a];
-        int b = a - 1;
-        while (b >= lo && rc_code[b] > v) { rc_code[b + 1] = rc_code[b]; --b; }
-        rc_code[b + 1] = v;
+    if (m <= 8) {
+        int r[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) r[k] = k < m ? v[k] : INT_MAX;
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+#pragma unroll
+            for (int k = s & 1; k + 1 < 8; k += 2) {
+                const int lo = min(r[k], r[k + 1]), hi = max(r[k], r[k + 1]);
+                r[k] = lo;
+                r[k + 1] = hi;
+            }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < m) v[k] = r[k];
+        return;
     }
-    atomicMax(maxcells, hi - lo);
+    for (int a = 1; a < m; ++a) {
+        const int x = v[a];
+        int b = a - 1;
+        while (b >= 0 && v[b] > x) { v[b + 1] = v[b]; --b; }
+        v[b + 1] = x;
+    }
 }
 
 // ---- K1, short rows: one thread per row -----------------------------------------------------
@@ -66,26 +80,73 @@ __global__ void k_sort_rows(const int *__restrict__ rc_ptr, int *__restrict__ rc
 // different banks whatever entry each one is at. A row with more than PT_CAP columns is put on a
 // list for the warp-per-row kernel below (counting pass); the filling pass skips it, since its
 // length (from indptr) is then known to be above PT_CAP.
+//
+// The counting pass also sorts the row's cells and, where there is room for it (tmp: a row's place is
+// rc_ptr[i] nloc, its candidates before it), keeps the row, so that the columns only have to be moved
+// together (k_pattern_compact) instead of being inserted a second time: 512^2 P2, 88 + 96 us for two
+// insertions, 32 for the sort and 13 for the diagonal (229 us), against 103 for this pass and 32 for moving (135 us).
 static constexpr int PT_THREADS = 128;
+static constexpr int PT_SORT = 16;  // candidates sorted in registers
 static constexpr int PT_CAP = 40;   // P1..P3 rows of a 6-valent mesh have 7, 19, 37 columns
 
 template <bool FILL>
 __global__ void __launch_bounds__(PT_THREADS) k_pattern_rows_t(const int *__restrict__ dofs, int nloc,
                                                                const int *__restrict__ rc_ptr,
-                                                               const int *__restrict__ rc_code, int nrows,
+                                                               int *__restrict__ rc_code, int nrows,
                                                                int *__restrict__ rowlen, const int *__restrict__ indptr,
-                                                               int *__restrict__ indices, int *__restrict__ list,
-                                                               int *__restrict__ nlist, int *__restrict__ status)
+                                                               int *__restrict__ indices, int *__restrict__ tmp,
+                                                               int *__restrict__ list, int *__restrict__ counts,
+                                                               int *__restrict__ status)
 {
+    // counts: the most cells of a row, the rows without an entry, the listed rows
     __shared__ int sbuf[PT_CAP * PT_THREADS];
     int *buf = sbuf + threadIdx.x;
     // every thread of a block takes the same number of turns, so the warp reduction below has all lanes
     for (int base = blockIdx.x * PT_THREADS; base < nrows; base += gridDim.x * PT_THREADS) {
         const int i = base + threadIdx.x;
-        int len = 0;
+        int len = 0, cells = 0;
+        if (!FILL && i < nrows) {
+            cells = rc_ptr[i + 1] - rc_ptr[i];
+            sort_row(rc_code + rc_ptr[i], cells);
+        }
         if (i < nrows && !(FILL && indptr[i + 1] - indptr[i] > PT_CAP)) {
             const int lo = rc_ptr[i], hi = rc_ptr[i + 1];
             bool over = false;
+            if ((hi - lo) * nloc <= PT_SORT) {
+                // few candidates (an edge's two cells): sorted in registers, the repeats left out
+                int v[PT_SORT], a = lo, j = 0;
+                const int *cd = dofs;
+#pragma unroll
+                for (int k = 0; k < PT_SORT; ++k) {
+                    v[k] = INT_MAX;
+                    if (a < hi) {
+                        if (j == 0) cd = dofs + (size_t)(rc_code[a] / nloc) * nloc;
+                        const int d = cd[j];
+                        if (d >= 0) v[k] = d;
+                        if (++j == nloc) { j = 0; ++a; }
+                    }
+                }
+                // Batcher's odd-even merge exchange
+#pragma unroll
+                for (int lq = 0; lq < 4; ++lq)
+#pragma unroll
+                    for (int lh = lq; lh >= 0; --lh)
+#pragma unroll
+                        for (int x = 0; x < PT_SORT; ++x) {
+                            const int h = 1 << lh, off = lh == lq ? 0 : h;
+                            if (x >= off && ((x - off) & (2 * h - 1)) < h && x + h < PT_SORT && x >> (lq + 1) == (x + h) >> (lq + 1)) {
+                                const int l = min(v[x], v[(x + h) & (PT_SORT - 1)]), m = max(v[x], v[(x + h) & (PT_SORT - 1)]);
+                                v[x] = l;
+                                v[(x + h) & (PT_SORT - 1)] = m;
+                            }
+                        }
+#pragma unroll
+                for (int k = 0; k < PT_SORT; ++k)
+                    if (v[k] != INT_MAX && (k == 0 || v[k] != v[k ? k - 1 : 0])) {
+                        buf[len * PT_THREADS] = v[k];
+                        ++len;
+                    }
+            } else
             for (int a = lo; a < hi && !over; ++a) {
                 const int *cd = dofs + (size_t)(rc_code[a] / nloc) * nloc;
                 for (int j = 0; j < nloc; ++j) {
@@ -106,18 +167,27 @@ __global__ void __launch_bounds__(PT_THREADS) k_pattern_rows_t(const int *__rest
             }
             if (over) {
                 // only the counting pass gets here: the warp kernel counts and later fills this row
-                if (!FILL) list[atomicAdd(nlist, 1)] = i;
+                if (!FILL) list[atomicAdd(counts + 2, 1)] = i;
                 len = 0;
             } else if (FILL) {
                 int *out = indices + indptr[i];
                 for (int c = 0; c < len; ++c) out[c] = buf[c * PT_THREADS];
             } else {
                 rowlen[i] = len;
+                if (tmp) {
+                    int *out = tmp + (size_t)rc_ptr[i] * nloc;
+                    for (int c = 0; c < len; ++c) out[c] = buf[c * PT_THREADS];
+                }
             }
         }
         if (!FILL) {
-            const int m = __reduce_max_sync(0xffffffffu, len);
-            if ((threadIdx.x & 31) == 0 && m) atomicMax(status + 2, m);
+            const int m = __reduce_max_sync(0xffffffffu, len), mc = __reduce_max_sync(0xffffffffu, cells);
+            const unsigned none = __ballot_sync(0xffffffffu, i < nrows && cells == 0);
+            if ((threadIdx.x & 31) == 0) {
+                if (m) atomicMax(status + 2, m);
+                if (mc > *(volatile int *)counts) atomicMax(counts, mc);
+                if (none) atomicAdd(counts + 1, __popc(none));
+            }
         }
     }
 }
@@ -133,7 +203,8 @@ __global__ void __launch_bounds__(PAT_WARPS * 32) k_pattern_rows(const int *__re
                                                                   const int *__restrict__ list,
                                                                   const int *__restrict__ nlist,
                                                                   int *__restrict__ rowlen, const int *__restrict__ indptr,
-                                                                  int *__restrict__ indices, int *__restrict__ status)
+                                                                  int *__restrict__ indices, int *__restrict__ diag,
+                                                                  int *__restrict__ status)
 {
     __shared__ int sbuf[PAT_WARPS][PAT_CAP];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -180,10 +251,56 @@ __global__ void __launch_bounds__(PAT_WARPS * 32) k_pattern_rows(const int *__re
             const int v = buf[t];
             const bool keep = v != INT_MAX && (t == 0 || buf[t - 1] != v);
             const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (FILL && keep) indices[base + count + __popc(bal & ((1u << lane) - 1u))] = v;
+            if (FILL && keep) {
+                const int p = base + count + __popc(bal & ((1u << lane) - 1u));
+                indices[p] = v;
+                if (v == i) diag[i] = p;
+            }
             count += __popc(bal);
         }
         if (!FILL && lane == 0) { rowlen[i] = count; atomicMax(status + 2, count); }
+        __syncwarp();
+    }
+}
+
+// Move the kept rows together, a warp to 32 rows (the columns of consecutive rows are one range, so
+// the stores are contiguous), and note each row's diagonal.  A row of cells holds its own dof; a row
+// without cells has none.  Rows above PT_CAP are the warp kernel's.
+__global__ void __launch_bounds__(256) k_pattern_compact(const int *__restrict__ indptr, const int *__restrict__ rc_ptr, int nloc,
+                                                         const int *__restrict__ tmp, int nrows, int *__restrict__ indices,
+                                                         int *__restrict__ diag)
+{
+    __shared__ int s_first[8][33], s_src[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int r0 = (blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += gridDim.x * 256) {
+        const int i = r0 + lane, end = indptr[min(r0 + 32, nrows)];
+        s_first[w][lane] = i < nrows ? indptr[i] : end;
+        s_src[w][lane] = i < nrows ? rc_ptr[i] : 0;
+        if (lane == 0) s_first[w][32] = end;
+        __syncwarp();
+        if (i < nrows && s_first[w][lane] == s_first[w][lane + 1]) diag[i] = -1;
+        constexpr int U = 4;                                 // positions of a lane in flight
+        for (int p0 = s_first[w][0] + lane; p0 < end; p0 += 32 * U) {
+            int t[U], c[U];
+            bool in[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int p = p0 + 32 * u;
+                t[u] = 0;                                    // the last row that starts at or before p
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (s_first[w][t[u] + o] <= p) t[u] += o;
+                const int b = s_first[w][t[u]];
+                in[u] = p < end && s_first[w][t[u] + 1] - b <= PT_CAP;
+                c[u] = in[u] ? __ldcs(&tmp[(size_t)s_src[w][t[u]] * nloc + (p - b)]) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (in[u]) {
+                    indices[p0 + 32 * u] = c[u];
+                    if (c[u] == r0 + t[u]) diag[r0 + t[u]] = p0 + 32 * u;
+                }
+        }
         __syncwarp();
     }
 }
@@ -204,9 +321,15 @@ __global__ void k_diag_pos(const int *__restrict__ indptr, const int *__restrict
 }
 
 // ---- K2: scatter map ------------------------------------------------------------------------
-__global__ void k_scatter_map(const int *__restrict__ dofs, long long ne_nloc, int nloc, const int *__restrict__ indptr,
-                              const int *__restrict__ indices, int *__restrict__ map, int *__restrict__ status)
+// One thread per (cell, i).  NLOC > 0: the row is read once, every column compared with the cell's
+// NLOC dofs in registers (P2: 12 loads on average; a binary search for each dof, as for other nloc,
+// takes 30, and the loads of 32 rows at once are what bounds this: 86 us at 512^2 P2, 67 so).
+template <int NLOC>
+__global__ void __launch_bounds__(256) k_scatter_map(const int *__restrict__ dofs, long long ne_nloc, int nloc_, const int *__restrict__ indptr,
+                                                     const int *__restrict__ indices, int *__restrict__ map,
+                                                     int *__restrict__ status)
 {
+    const int nloc = NLOC ? NLOC : nloc_;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < ne_nloc; t += (long long)gridDim.x * blockDim.x) {
         const long long e = t / nloc;
         const int *d = dofs + e * nloc;
@@ -217,6 +340,27 @@ __global__ void k_scatter_map(const int *__restrict__ dofs, long long ne_nloc, i
             continue;
         }
         const int rlo = indptr[I], rhi = indptr[I + 1];
+        if (NLOC) {
+            int J[NLOC ? NLOC : 1], pos[NLOC ? NLOC : 1];
+#pragma unroll
+            for (int j = 0; j < NLOC; ++j) {
+                J[j] = d[j];
+                pos[j] = -1;
+            }
+#pragma unroll 4
+            for (int q = rlo; q < rhi; ++q) {
+                const int c = indices[q];
+#pragma unroll
+                for (int j = 0; j < NLOC; ++j)
+                    if (c == J[j]) pos[j] = q;
+            }
+#pragma unroll
+            for (int j = 0; j < NLOC; ++j) {
+                if (J[j] >= 0 && pos[j] < 0) atomicOr(status, ST_OUTSIDE);
+                out[j] = pos[j];
+            }
+            continue;
+        }
         for (int j = 0; j < nloc; ++j) {
             const int J = d[j];
             int pos = -1;
@@ -244,9 +388,11 @@ int build_scatter_map(femd_ctx ctx, femd_pattern p)
     const long long tot = (long long)p->ncells * p->nloc;
     FEMD_TRY(p->map.alloc((size_t)tot * p->nloc));
     FEMD_TRY(reset_status(ctx));
-    if (tot > 0)
-        k_scatter_map<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(ctx->stream)>>>(
-            p->cell_dofs.p, tot, p->nloc, p->indptr.p, p->indices.p, p->map.p, ctx->status_dev);
+    if (tot > 0) {
+        const unsigned grid = grid_for((size_t)tot, 256, 1u << 20);
+        auto k = p->nloc == 3 ? k_scatter_map<3> : p->nloc == 6 ? k_scatter_map<6> : p->nloc == 10 ? k_scatter_map<10> : k_scatter_map<0>;
+        k<<<grid, 256, 0, counted(ctx->stream)>>>(p->cell_dofs.p, tot, p->nloc, p->indptr.p, p->indices.p, p->map.p, ctx->status_dev);
+    }
     FEMD_TRY_CUDA(cudaGetLastError());
     int flags = 0;
     FEMD_TRY(read_status(ctx, &flags, nullptr));
@@ -288,85 +434,96 @@ int femd_cuda_pattern_from_cells(femd_ctx ctx, int nrows, int ncells, int nloc, 
     p->nloc = nloc;
     auto fail = [&](int st) { delete p; return st; };
     const long long tot = (long long)ncells * nloc;
+    // Scratch, one block of ints: the counts (the scan's input, then the fill positions and the long
+    // rows), the row lengths, the scan's own, three counters, and the kept rows.  In the context's
+    // workspace where it fits (its stream orders the builds), else of this call, without the kept rows.
+    const size_t nr = (size_t)nrows + 1, nscan = scan_tmp_ints(nr), base_ints = 2 * nr + nscan + 4;
+    const size_t with_rows = base_ints + (size_t)tot * nloc;
+    const bool keep = with_rows <= 2 * CTX_SCRATCH, shared = keep || base_ints <= 2 * CTX_SCRATCH;
+    const size_t ints = keep ? with_rows : base_ints;
+    DevBuf<double> own;
+    DevBuf<double> &scratch = shared ? ctx->asm_scratch : own;
     int st;
-    if ((st = p->cell_dofs.alloc((size_t)tot)) != FEMD_OK) return fail(st);
+    if (scratch.n < (ints + 1) / 2 && (st = scratch.alloc((ints + 1) / 2))) return fail(st);
+    int *const cnt = reinterpret_cast<int *>(scratch.p), *const rowlen = cnt + nr, *const tmp = rowlen + nr,
+              *const counts = tmp + nscan, *const rows_kept = keep ? counts + 4 : nullptr;
+    if ((st = p->cell_dofs.alloc((size_t)tot)) || (st = p->rc_ptr.alloc(nr)) || (st = p->indptr.alloc(nr)) ||
+        (st = p->diag_pos.alloc(nr)))
+        return fail(st);
+    cudaError_t e = cudaSuccess;
+    auto failed = [&]() { set_error(std::string("cell_pattern: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); };
     if (tot) {
-        cudaError_t e = cudaMemcpyAsync(p->cell_dofs.p, cell_dofs_dev, (size_t)tot * sizeof(int), cudaMemcpyDefault, s);
+        e = cudaMemcpyAsync(p->cell_dofs.p, cell_dofs_dev, (size_t)tot * sizeof(int), cudaMemcpyDefault, s);
         if (e != cudaSuccess) { set_error(std::string("cell_pattern: copy of cell_dofs: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); }
     }
-    DevBuf<int> cnt, tmp, fill, rowlen;
-    DevBuf<int> maxc;
-    if ((st = cnt.alloc((size_t)nrows + 1)) || (st = tmp.alloc(scan_tmp_ints((size_t)nrows + 1))) ||
-        (st = p->rc_ptr.alloc((size_t)nrows + 1)) || (st = p->indptr.alloc((size_t)nrows + 1)) ||
-        (st = fill.alloc((size_t)nrows + 1)) || (st = rowlen.alloc((size_t)nrows + 1)) || (st = maxc.alloc(3)))
-        return fail(st);
+    // an array's last entry and the status words, by one wait
+    int *const last = static_cast<int *>(ctx->res_host);
+    auto read = [&](const int *at, int *flags, int *bad) {
+        e = cudaMemcpyAsync(last, at, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(last + 1, counts, 3 * sizeof(int), cudaMemcpyDeviceToHost, s);
+        return e == cudaSuccess ? read_status(ctx, flags, bad) : FEMD_OK;
+    };
     if ((st = reset_status(ctx))) return fail(st);
-    cudaMemsetAsync(cnt.p, 0, ((size_t)nrows + 1) * sizeof(int), s);
-    // the most cells of a row, the rows without a diagonal, the rows on the long-row list
-    cudaMemsetAsync(maxc.p, 0, 3 * sizeof(int), s);
-    if (tot) k_count_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, cnt.p, ctx->status_dev);
-    if ((st = exclusive_scan_int(cnt.p, p->rc_ptr.p, (size_t)nrows + 1, tmp.p, s))) return fail(st);
-    int flags = 0;
-    if ((st = read_status(ctx, &flags, nullptr))) return fail(st);
+    cudaMemsetAsync(cnt, 0, nr * sizeof(int), s);
+    cudaMemsetAsync(counts, 0, 3 * sizeof(int), s);
+    if (tot) k_count_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, cnt, ctx->status_dev);
+    if ((st = exclusive_scan_int(cnt, p->rc_ptr.p, nr, tmp, s))) return fail(st);
+    int flags = 0, bad = 0;
+    st = read(p->rc_ptr.p + nrows, &flags, nullptr);
+    if (e != cudaSuccess) return failed();
+    if (st) return fail(st);
     if (flags & ST_BADDOF) { set_error("cell_pattern: a cell dof is >= nrows"); return fail(FEMD_EINVAL); }
-    int total_rc = 0;
-    cudaError_t e = cudaMemcpyAsync(&ctx->status_host[2], p->rc_ptr.p + nrows, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_error(std::string("cell_pattern: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); }
-    total_rc = ctx->status_host[2];
-    if ((st = p->rc_code.alloc((size_t)total_rc + 1))) return fail(st);
-    cudaMemcpyAsync(fill.p, p->rc_ptr.p, ((size_t)nrows + 1) * sizeof(int), cudaMemcpyDeviceToDevice, s);
-    if (tot) k_fill_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, nloc, fill.p, p->rc_code.p);
-    if (nrows) k_sort_rows<<<grid_for((size_t)nrows, 256), 256, 0, counted(s)>>>(p->rc_ptr.p, p->rc_code.p, nrows, maxc.p);
-    // K1: row lengths, scan, fill. Rows of up to PT_CAP columns take a thread each; the longer
-    // ones go on a list (in `fill`, free again by now) that a warp per row takes.
-    cudaMemsetAsync(rowlen.p + nrows, 0, sizeof(int), s);
+    if ((st = p->rc_code.alloc((size_t)last[0] + 1))) return fail(st);
+    cudaMemcpyAsync(cnt, p->rc_ptr.p, nr * sizeof(int), cudaMemcpyDeviceToDevice, s);
+    if (tot) k_fill_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, nloc, cnt, p->rc_code.p);
+    // K1: row lengths, scan, columns. Rows of up to PT_CAP columns take a thread each; the longer
+    // ones go on a list (in cnt, free again by now) that a warp per row takes.
+    cudaMemsetAsync(rowlen + nrows, 0, sizeof(int), s);
     const unsigned tgrid = grid_for((size_t)nrows, PT_THREADS, 1u << 20);
     const unsigned lgrid = std::min(grid_for((size_t)nrows, PAT_WARPS, 1u << 20), 1184u);
-    int *const long_rows = fill.p, *const nlong = maxc.p + 2;
+    int *const long_rows = cnt;
     if (nrows) {
-        k_pattern_rows_t<false><<<tgrid, PT_THREADS, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, nrows,
-                                                                     rowlen.p, nullptr, nullptr, long_rows, nlong,
+        k_pattern_rows_t<false><<<tgrid, PT_THREADS, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, nrows, rowlen,
+                                                                     nullptr, nullptr, rows_kept, long_rows, counts,
                                                                      ctx->status_dev);
-        k_pattern_rows<false><<<lgrid, PAT_WARPS * 32, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p,
-                                                                long_rows, nlong, rowlen.p, nullptr, nullptr,
-                                                                ctx->status_dev);
+        k_pattern_rows<false><<<lgrid, PAT_WARPS * 32, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, long_rows,
+                                                                       counts + 2, rowlen, nullptr, nullptr, nullptr,
+                                                                       ctx->status_dev);
     }
-    if ((st = exclusive_scan_int(rowlen.p, p->indptr.p, (size_t)nrows + 1, tmp.p, s))) return fail(st);
-    int nnz = 0;
-    e = cudaMemcpyAsync(&ctx->status_host[2], p->indptr.p + nrows, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_error(std::string("cell_pattern: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); }
-    nnz = ctx->status_host[2];
-    int bad = 0;
-    if ((st = read_status(ctx, &flags, &bad))) return fail(st);
+    if ((st = exclusive_scan_int(rowlen, p->indptr.p, nr, tmp, s))) return fail(st);
+    st = read(p->indptr.p + nrows, &flags, &bad);
+    if (e != cudaSuccess) return failed();
+    if (st) return fail(st);
+    p->nnz = last[0];
+    p->max_row_cells = last[1];
+    p->all_diag = last[2] == 0;
     p->max_row_len = ctx->status_host[2];
     if (flags & ST_ROW_TOO_LONG) {
         set_error("cell_pattern: row " + std::to_string(bad) + " couples more than " + std::to_string(PAT_CAP) +
                   " cell dofs (too many cells around one node)");
         return fail(FEMD_EINVAL);
     }
-    p->nnz = nnz;
-    if ((st = p->indices.alloc((size_t)nnz + 1))) return fail(st);
+    if ((st = p->indices.alloc((size_t)p->nnz + 1))) return fail(st);
     if (nrows) {
-        k_pattern_rows_t<true><<<tgrid, PT_THREADS, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, nrows,
-                                                                    nullptr, p->indptr.p, p->indices.p, nullptr, nullptr,
-                                                                    ctx->status_dev);
-        k_pattern_rows<true><<<lgrid, PAT_WARPS * 32, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p,
-                                                               long_rows, nlong, nullptr, p->indptr.p, p->indices.p,
-                                                               ctx->status_dev);
+        if (keep) {
+            k_pattern_compact<<<grid_for((size_t)nrows, 256, 1u << 20), 256, 0, counted(s)>>>(p->indptr.p, p->rc_ptr.p, nloc, rows_kept,
+                                                                                             nrows, p->indices.p, p->diag_pos.p);
+        } else {
+            k_pattern_rows_t<true><<<tgrid, PT_THREADS, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, nrows,
+                                                                        nullptr, p->indptr.p, p->indices.p, nullptr, nullptr,
+                                                                        nullptr, ctx->status_dev);
+        }
+        if (last[3])
+            k_pattern_rows<true><<<lgrid, PAT_WARPS * 32, 0, counted(s)>>>(p->cell_dofs.p, nloc, p->rc_ptr.p, p->rc_code.p, long_rows,
+                                                                          counts + 2, nullptr, p->indptr.p, p->indices.p,
+                                                                          p->diag_pos.p, ctx->status_dev);
+        if (!keep)
+            k_diag_pos<<<grid_for((size_t)nrows, 256), 256, 0, counted(s)>>>(p->indptr.p, p->indices.p, nrows, nrows, p->diag_pos.p,
+                                                                             nullptr);
     }
-    if ((st = p->diag_pos.alloc((size_t)nrows + 1))) return fail(st);
-    if (nrows)
-        k_diag_pos<<<grid_for((size_t)nrows, 256), 256, 0, counted(s)>>>(p->indptr.p, p->indices.p, nrows, nrows, p->diag_pos.p,
-                                                                          maxc.p + 1);
     e = cudaGetLastError();
-    if (e != cudaSuccess) { set_error(std::string("cell_pattern: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); }
-    e = cudaMemcpyAsync(&ctx->status_host[2], maxc.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_error(std::string("cell_pattern: ") + cudaGetErrorString(e)); return fail(FEMD_ECUDA); }
-    p->max_row_cells = ctx->status_host[2];
-    p->all_diag = ctx->status_host[3] == 0;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);      // the pattern may be used on any stream from here on
+    if (e != cudaSuccess) return failed();
     *out = p;
     return FEMD_OK;
 }
