@@ -410,7 +410,7 @@ def kernel_rates(fb, torch, pr, hbm):
     pr.assemble(jacobi=True)
     us = C.c_double()
     for kern, name, alg, txt in (
-            (0, "K5 k_spmv (FP64 SpMV fused with p.Ap)", 12 * nnz + 4 * (n + 1) + 16 * n,
+            (0, "K5 k_spmv_slices (FP64 SpMV fused with p.Ap)", 12 * nnz + 4 * (n + 1) + 16 * n,
              "12 nnz + 4 (n+1) + 8 n (p, counted once) + 8 n (Ap)"),
             (1, "K6 k_cg_update (x += a p, r -= a Ap, ||r||^2, r.D^-1 r)", 56 * n, "40 n read + 16 n written")):
         fb.core.check(fb.lib.femd_cuda_kernel_time(ctx.h, pr.K.h, kern, 50, C.byref(us)))

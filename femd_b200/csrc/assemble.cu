@@ -1116,6 +1116,35 @@ static int prepare_terms(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
 
 static constexpr int FAST_MAX_ROW = 96;   // longest row the shared-memory accumulator holds
 
+// Where the cells' factors, vectors or matrices go: the context's workspace up to its bound (the
+// context's stream orders the assemblies that share it), else, and where the work is being captured (a
+// graph keeps the address), the pattern's own, which is not given back once a capture has used it.
+static int cell_workspace(femd_ctx ctx, femd_pattern p, size_t cells, DevBuf<double> **W)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    FEMD_TRY_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (!captured && cells <= CTX_SCRATCH) {
+        *W = &ctx->asm_scratch;
+        return (*W)->n < cells ? (*W)->alloc(std::min(cells + cells / 4, CTX_SCRATCH)) : FEMD_OK;
+    }
+    *W = &p->ws_factors;
+    if ((*W)->n < cells) {
+        if (p->ws_captured) {
+            p->ws_kept.emplace_back(new DevBuf<double>());
+            std::swap(p->ws_kept.back()->p, (*W)->p);
+            std::swap(p->ws_kept.back()->n, (*W)->n);
+        }
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the allocation is not part of the capture
+        FEMD_TRY_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const int st = (*W)->alloc(cells);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        FEMD_TRY(st);
+    }
+    p->ws_captured |= captured;
+    return FEMD_OK;
+}
+
 // FAST assembly of a matrix (K non-null) or a vector (f non-null).  Tables and factors live in
 // the pattern's workspace; no allocation once the workspace has its size.
 static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule *rule, femd_pattern p, int nterms,
@@ -1152,11 +1181,15 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
                 }
     }
     const size_t per_cell = vector ? (size_t)nl : element ? (size_t)nl2 : (size_t)fs.nf;
-    // the cells' factors, vectors or matrices: in the context's workspace up to its bound (the
-    // context's stream orders the assemblies that share it), else in the pattern's own
+    if (!vector) {
+        const bool by_pairs = (nl == 3 || nl == 6 || nl == 10) && (element || listed);
+        FEMD_TRY(by_pairs ? build_pair_offsets(ctx, p) : build_scatter_map(ctx, p));
+    }
     const size_t cells = (size_t)ne * per_cell + 1;
-    DevBuf<double> &W = cells <= CTX_SCRATCH ? ctx->asm_scratch : p->ws_factors;
-    if (W.n < cells) FEMD_TRY(W.alloc(std::min(cells + cells / 4, std::max(cells, CTX_SCRATCH))));
+    std::unique_lock<std::mutex> guard(ctx->shared);
+    DevBuf<double> *Wp = nullptr;
+    FEMD_TRY(cell_workspace(ctx, p, cells, &Wp));
+    DevBuf<double> &W = *Wp;
     // the slot holding these tables, else the least recently used one, refilled (stream-ordered,
     // so kernels still reading the slot's old tables finish first)
     femd_pattern_s::TableSlot *slot = nullptr;
@@ -1213,8 +1246,6 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
             mesh->points_dev, mesh->tris_dev, ne, nq, nl, p->cell_dofs.p, d_tab, fs, W.p);
     }
     FEMD_TRY_CUDA(cudaGetLastError());
-    const bool by_pairs = (nl == 3 || nl == 6 || nl == 10) && (element || listed);
-    FEMD_TRY(by_pairs ? build_pair_offsets(ctx, p) : build_scatter_map(ctx, p));
     FEMD_TRY(reset_status(ctx));
     double *inv = nullptr;
     if (want_inv) {
@@ -1240,13 +1271,14 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
         FEMD_ROWS_OFF(6, 0) FEMD_ROWS_OFF(6, 1) FEMD_ROWS_OFF(6, 3) FEMD_ROWS_OFF(6, 4) FEMD_ROWS_OFF(6, 5)
         FEMD_ROWS_OFF(10, 0) FEMD_ROWS_OFF(10, 1) FEMD_ROWS_OFF(10, 3) FEMD_ROWS_OFF(10, 4) FEMD_ROWS_OFF(10, 5)
 #undef FEMD_ROWS_OFF
-        if (!by_pairs) {
+        if (!((nl == 3 || nl == 6 || nl == 10) && (element || listed))) {
             cudaFuncSetAttribute(k_assemble_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
             k_assemble_rows<<<grid, FAST_BLOCK, shm, counted(s)>>>(p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->map.p,
                                                                    p->diag_pos.p, n, nl, nq, W.p, d_S, d_ref,
                                                                    fs, maxlen, K->data.p, inv, ctx->status_dev);
         }
     }
+    guard.unlock();
     FEMD_TRY_CUDA(cudaGetLastError());
     K->f32_valid = false;
     if (want_inv) {

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 #include <atomic>
+#include <memory>
+#include <mutex>
 #include <stdint.h>
 
 #include <string>
@@ -97,15 +99,19 @@ struct femd_ctx_s {
     int device = 0;
     cudaStream_t stream = nullptr;
     int sm_count = 0;
-    // a small device status block: [0] error flags, [1] first bad row, [2..] spare
+    // a small device status block: [0] error flags, [1] first bad row, [2..3] spare, [4] the slices' width
     int *status_dev = nullptr;
     int *status_host = nullptr;   // pinned
+    // several host threads may use patterns and matrices of one context: held while what follows is in
+    // use, by an assembly until its last kernel is queued (the stream then orders the next), by a
+    // pattern's build and an on-chip solve until they have read their results
+    std::mutex shared;
     // the on-chip solve (resident.cu): device scratch, grown to the largest such system (a few MB at
     // most), pinned room for its result, and the events that time it
     femd::DevBuf<double> res_scratch;
     void *res_host = nullptr;
     // scratch of an assembly (the cells' factors, vectors or matrices) and of a pattern's build, up to
-    // CTX_SCRATCH doubles; the context's stream orders what shares it
+    // CTX_SCRATCH doubles (not for work that is being captured: a graph would keep the address)
     femd::DevBuf<double> asm_scratch;
     cudaEvent_t res_e0 = nullptr, res_e1 = nullptr;
 };
@@ -135,8 +141,11 @@ struct femd_pattern_s : femd::HandleBase {
     femd::DevBuf<int> diag_pos;        // position of (i, i), -1 when absent
     bool all_diag = false;             // every row i holds the position (i, i)
     int max_row_cells = 0, max_row_len = 0;
-    // assembly workspace past the context's shared one, grown on demand and reused across calls
+    // assembly workspace past the context's shared one and under capture, grown on demand and reused
+    // across calls; what a capture has used is kept until the pattern goes (ws_kept)
     femd::DevBuf<double> ws_factors;
+    bool ws_captured = false;
+    std::vector<std::unique_ptr<femd::DevBuf<double>>> ws_kept;
     // the rule's tables (weights, points, reference values, the pair tensors) of the last few
     // forms, each with the host copy it was uploaded from: a repeated assembly of the same form
     // uploads nothing (a pageable upload can wait for the stream)
@@ -167,7 +176,9 @@ struct femd_pattern_s : femd::HandleBase {
     // the single solve's layout (krylov.cu): slices of 32 consecutive rows, entry j of every row side by
     // side, filled up to the slice's longest row (column -1).  sl_state: 0 not looked at, 1 suitable, -1
     // too much filling; sl_slots entries in all; the slices' first entries (in 32) and the columns, built
-    // at the first solve that uses them
+    // at the first solve that uses them, under sl_lock (matrices of one pattern may be solved by
+    // several threads)
+    std::mutex sl_lock;
     int sl_state = 0;
     long long sl_slots = 0;
     femd::DevBuf<int> sl_ptr, sl_col;

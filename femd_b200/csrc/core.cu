@@ -264,7 +264,7 @@ int femd_cuda_ctx_create(int device, femd_ctx *out)
     c->device = dev;
     c->sm_count = prop.multiProcessorCount;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, 4 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, 8 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, 4 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&c->res_host, sizeof(femd::ResidentOut));
     if (e == cudaSuccess) e = cudaEventCreate(&c->res_e0);

@@ -1,6 +1,7 @@
-// krylov.cu -- K5: CSR SpMV (sub-warp per row) fused with p^T A p; K6: the fused Jacobi-PCG
-// update (x += a p, r -= a Ap, ||r||^2 and r^T D^-1 r in one pass) and direction update; the
-// whole CG loop runs on the device with no host round trip per iteration.
+// krylov.cu -- K5: SpMV (slices of 32 rows, or CSR with a sub-warp per row) fused with p^T A p; K6: the
+// fused Jacobi-PCG update (x += a p, r -= a Ap, ||r||^2 and r^T D^-1 r in one pass) and direction
+// update; the whole CG loop runs on the device with no host round trip per iteration.  Systems that fit
+// the SMs' shared memory are solved by the one kernel of resident.cu.
 //
 // Reference: krylov::cg_jacobi (include/femd/krylov/cg.hpp:296-350), cg_update_chunk_jacobi
 // (:99-171), detail_cg::finish (:222-237), CSRMatrix::apply (include/femd/sparse/csr.hpp:203-215).
@@ -843,13 +844,16 @@ static int use_slices(femd_ctx ctx, femd_matrix K, bool *use)
     const int n = P->nrows, nsl = (n + 31) / 32;
     *use = false;
     if (K->spmv_tpr || n == 0) return FEMD_OK;
+    std::lock_guard<std::mutex> guard(P->sl_lock);
     if (P->sl_state == 0) {
-        FEMD_TRY(reset_status(ctx));
-        k_slice_widths<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(P->indptr.p, n, nsl,
-                                                                                                     ctx->status_dev + 2, nullptr);
+        std::lock_guard<std::mutex> word(ctx->shared);
+        int *const sum = ctx->status_dev + 4, width = 0;
+        FEMD_TRY_CUDA(cudaMemsetAsync(sum, 0, sizeof(int), ctx->stream));
+        k_slice_widths<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(P->indptr.p, n, nsl, sum, nullptr);
         FEMD_TRY_CUDA(cudaGetLastError());
-        FEMD_TRY(read_status(ctx, nullptr, nullptr));
-        P->sl_slots = 32ll * ctx->status_host[2];
+        FEMD_TRY_CUDA(cudaMemcpyAsync(&width, sum, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        FEMD_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+        P->sl_slots = 32ll * width;
         P->sl_state = P->sl_slots <= P->nnz + P->nnz / 5 + 4096 ? 1 : -1;
     }
     *use = P->sl_state == 1;
@@ -859,6 +863,7 @@ static int use_slices(femd_ctx ctx, femd_matrix K, bool *use)
 // The slices' places and columns, once per pattern.
 static int slice_layout(femd_ctx ctx, femd_pattern P)
 {
+    std::lock_guard<std::mutex> guard(P->sl_lock);
     if (P->sl_col.p) return FEMD_OK;
     const int n = P->nrows, nsl = (n + 31) / 32;
     cudaStream_t s = ctx->stream;
@@ -1052,7 +1057,7 @@ static int cg_resident(femd_ctx ctx, femd_matrix K, bool jac, const double *b, d
     femd_pattern P = K->pattern;
     cudaStream_t s = ctx->stream;
     *ran = false;
-    if (timed) FEMD_TRY_CUDA(cudaEventRecord(ctx->res_e0, s));
+    if (timed) FEMD_TRY_CUDA(cudaEventRecord(ctx->res_e0, s));   // the caller holds ctx->shared
     const cudaError_t e = resident_launch(plan, P->indptr.p, P->indices.p, K->data.p, jac ? K->inv.p : nullptr, b, x, P->nrows,
                                           max_iter, tol, zx, slots, out, s);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {
@@ -1094,6 +1099,7 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     cudaStream_t s = ctx->stream;
     ResidentPlan plan;
     if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+        std::lock_guard<std::mutex> guard(ctx->shared);
         const size_t need = (size_t)n + 1 + RES_SLOT_DOUBLES + RES_OUT_DOUBLES;
         if (ctx->res_scratch.n < need) FEMD_TRY(ctx->res_scratch.alloc(need + need / 4));
         double *slots = ctx->res_scratch.p, *out = slots + RES_SLOT_DOUBLES;
@@ -2019,6 +2025,7 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
                   "the on-chip solve's scratch fits the fixed array");
     ResidentPlan plan;
     if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+        std::lock_guard<std::mutex> guard(ctx->shared);
         bool ran = false;
         FEMD_TRY(cg_resident(ctx, K, jac, b_dev, x_dev, max_iter, tol, plan, r, part, reinterpret_cast<ResidentOut *>(st),
                              false, &ran, res));

@@ -436,12 +436,13 @@ int femd_cuda_pattern_from_cells(femd_ctx ctx, int nrows, int ncells, int nloc, 
     const long long tot = (long long)ncells * nloc;
     // Scratch, one block of ints: the counts (the scan's input, then the fill positions and the long
     // rows), the row lengths, the scan's own, three counters, and the kept rows.  In the context's
-    // workspace where it fits (its stream orders the builds), else of this call, without the kept rows.
+    // workspace where it fits, else of this call, without the kept rows.
     const size_t nr = (size_t)nrows + 1, nscan = scan_tmp_ints(nr), base_ints = 2 * nr + nscan + 4;
     const size_t with_rows = base_ints + (size_t)tot * nloc;
     const bool keep = with_rows <= 2 * CTX_SCRATCH, shared = keep || base_ints <= 2 * CTX_SCRATCH;
     const size_t ints = keep ? with_rows : base_ints;
     DevBuf<double> own;
+    std::lock_guard<std::mutex> guard(ctx->shared);
     DevBuf<double> &scratch = shared ? ctx->asm_scratch : own;
     int st;
     if (scratch.n < (ints + 1) / 2 && (st = scratch.alloc((ints + 1) / 2))) return fail(st);

@@ -291,6 +291,8 @@ FEMD_API int femd_cuda_combine(femd_ctx ctx, double alpha, femd_matrix A, double
  * with the same stopping rule, final true residual, 10 tol acceptance and breakdown tests
  * (cg.hpp:222-237).  The reductions are deterministic (fixed order, the same bits on every
  * run) but not the reference's chunk order, so iteration counts may differ by a few.
+ * A system whose matrix fits the SMs' shared memory is solved in one launch, whose blocks wait for
+ * each other with a bound (FEMD_ETIMEOUT past it); on-chip solves of one context run one at a time.
  * ====================================================================================== */
 typedef struct {
     int converged;
