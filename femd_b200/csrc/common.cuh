@@ -62,6 +62,7 @@ template <class T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
+    bool part = false;   // of another buffer, which gives the memory back
     int alloc(size_t count)
     {
         release();
@@ -79,9 +80,17 @@ struct DevBuf {
     }
     void release()
     {
-        if (p) dev_free(p);
+        if (p && !part) dev_free(p);
         p = nullptr;
         n = 0;
+        part = false;
+    }
+    void place(T *at, size_t count)
+    {
+        release();
+        p = at;
+        n = count;
+        part = true;
     }
     ~DevBuf() { release(); }
 };
@@ -134,6 +143,7 @@ struct femd_pattern_s : femd::HandleBase {
     femd_ctx ctx = nullptr;
     int nrows = 0, ncols = 0, ncells = 0, nloc = 0;
     long long nnz = 0;
+    femd::DevBuf<int> block;           // one allocation for the arrays of a build whose sizes are known at its start
     femd::DevBuf<int> indptr, indices;
     femd::DevBuf<int> cell_dofs;       // ncells x nloc (copy)
     femd::DevBuf<int> rc_ptr, rc_code; // row -> (cell nloc + local), increasing cell order
