@@ -232,10 +232,10 @@ __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
-// exclusive scan of n ints in place on the stream; n+1 entries are written when total is
-// requested (out[n] = total).  Uses tmp (device) of scan_tmp_size(n) ints.
+// The exclusive scan of n ints on the stream, in to out (which may be in) and, where given, to copy (which
+// may be in too).  tmp: scan_tmp_ints(n) device ints.
 size_t scan_tmp_ints(size_t n);
-int exclusive_scan_int(const int *in, int *out, size_t n, int *tmp, cudaStream_t s);
+int exclusive_scan_int(const int *in, int *out, size_t n, int *tmp, cudaStream_t s, int *copy = nullptr);
 
 // Kernel launches issued by this library in this process (graph launches count their nodes).
 void add_launches(long long n);

@@ -107,26 +107,66 @@ void dev_free(void *p)
     if (dev != cur) cudaSetDevice(cur);
 }
 
-// ---- exclusive scan of int32 (three phases: tile scans, scan of tile sums, add) ------------
+// ---- exclusive scan of int32 -----------------------------------------------------------------
+// The tiles' sums, then the tiles, each with its offset: two readings of the input (the second from
+// L2) and one writing, all of them 32 consecutive ints of a warp.  1 M ints: 3.6 + 5.0 us
+// (4.2 M: 5.6 + 10.4); scanning the tiles by threads of 8 consecutive ints in global memory (4.2 M:
+// 23 us), then the tiles' sums, then adding the offsets took 8.6 + 5 + 7.1 us.
 static constexpr int SCAN_THREADS = 512;
 static constexpr int SCAN_ITEMS = 8;
 static constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int *__restrict__ in, int *__restrict__ out,
-                                                            size_t n, int *__restrict__ tile_sums)
+// The sum of a block's v, in every thread
+__device__ __forceinline__ int scan_block_sum(int v, int *warp_tot)
+{
+    static_assert(SCAN_THREADS / 32 == 16, "a half-warp holds the warps' sums");
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < 16 ? warp_tot[threadIdx.x & 15] : 0);
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restrict__ in, size_t n, int *__restrict__ sums)
 {
     __shared__ int warp_tot[SCAN_THREADS / 32];
-    const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
-    int v[SCAN_ITEMS];
-    int run = 0;
+    const size_t base = (size_t)blockIdx.x * SCAN_TILE + threadIdx.x;
+    int v = 0;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) v += base + i * SCAN_THREADS < n ? in[base + i * SCAN_THREADS] : 0;
+    v = scan_block_sum(v, warp_tot);
+    if (threadIdx.x == 0) sums[blockIdx.x] = v;
+}
+
+// A tile's scan from its offset, to out and (where given) copy; either may be in, of which a block reads
+// its own tile before it writes.  tiles: null: one tile; DIRECT: the tiles' sums, of which every block
+// adds up those before its own; else their scan.
+template <bool DIRECT>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int *in, int *out, int *copy, size_t n, const int *__restrict__ tiles)
+{
+    __shared__ int buf[SCAN_TILE + SCAN_TILE / 32];   // entry k at k + k / 32: 8 consecutive ones of 32 threads meet no bank twice
+    __shared__ int before[SCAN_THREADS / 32], warp_tot[SCAN_THREADS / 32];
+    const size_t base = (size_t)blockIdx.x * SCAN_TILE + threadIdx.x;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const size_t g = base + i;
-        const int x = g < n ? in[g] : 0;
-        v[i] = run;
-        run += x;
+        const int k = threadIdx.x + i * SCAN_THREADS;
+        buf[k + k / 32] = base + i * SCAN_THREADS < n ? in[base + i * SCAN_THREADS] : 0;
     }
-    // inclusive warp scan of the per-thread totals
+    int off = 0;
+    if (DIRECT) {
+        for (unsigned t = threadIdx.x; t < blockIdx.x; t += SCAN_THREADS) off += tiles[t];
+        off = scan_block_sum(off, before);            // its barrier is also the one behind buf
+    } else {
+        if (tiles) off = tiles[blockIdx.x];
+        __syncthreads();
+    }
+    int v[SCAN_ITEMS], run = 0;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) {
+        const int k = threadIdx.x * SCAN_ITEMS + i;
+        v[i] = run;
+        run += buf[k + k / 32];
+    }
+    // the threads before, in the warp and in the warps before
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int inc = run;
 #pragma unroll
@@ -136,30 +176,22 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int *__restri
     }
     if (lane == 31) warp_tot[wid] = inc;
     __syncthreads();
-    if (wid == 0) {
-        int w = lane < SCAN_THREADS / 32 ? warp_tot[lane] : 0;
-        int wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += t;
-        }
-        if (lane < SCAN_THREADS / 32) warp_tot[lane] = wi - w;   // exclusive warp offsets
-        if (lane == SCAN_THREADS / 32 - 1 && tile_sums) tile_sums[blockIdx.x] = wi;
-    }
-    __syncthreads();
-    const int off = warp_tot[wid] + inc - run;
+    off += inc - run + __reduce_add_sync(0xffffffffu, lane < wid ? warp_tot[lane & 15] : 0);
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const size_t g = base + i;
-        if (g < n) out[g] = v[i] + off;
+        const int k = threadIdx.x * SCAN_ITEMS + i;
+        buf[k + k / 32] = v[i] + off;
     }
-}
-
-__global__ void k_scan_add(int *__restrict__ out, size_t n, const int *__restrict__ tile_off)
-{
-    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < n) out[g] += tile_off[g / SCAN_TILE];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) {
+        const int k = threadIdx.x + i * SCAN_THREADS;
+        const size_t g = base + i * SCAN_THREADS;
+        if (g < n) {
+            out[g] = buf[k + k / 32];
+            if (copy) copy[g] = buf[k + k / 32];
+        }
+    }
 }
 
 size_t scan_tmp_ints(size_t n)
@@ -173,20 +205,29 @@ size_t scan_tmp_ints(size_t n)
     return total + 1;
 }
 
-int exclusive_scan_int(const int *in, int *out, size_t n, int *tmp, cudaStream_t s)
+// Up to this many tiles their sums are added up by every block of the last kernel instead of being
+// scanned by a launch between: 1,024 tiles 10.4 us against 3.0 + 9.7 and the gap; at 4,095 the blocks'
+// reads, tiles^2 / 2, have used the gain up (33 against 3.4 + 30).
+static constexpr size_t SCAN_DIRECT = 1024;
+
+int exclusive_scan_int(const int *in, int *out, size_t n, int *tmp, cudaStream_t s, int *copy)
 {
     if (n == 0) return FEMD_OK;
     const size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (tiles == 1) {
-        k_scan_tiles<<<1, SCAN_THREADS, 0, counted(s)>>>(in, out, n, nullptr);
+        k_scan_tiles<false><<<1, SCAN_THREADS, 0, counted(s)>>>(in, out, copy, n, nullptr);
         FEMD_TRY_CUDA(cudaGetLastError());
         return FEMD_OK;
     }
     int *sums = tmp;
-    k_scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, counted(s)>>>(in, out, n, sums);
+    k_scan_sums<<<(unsigned)tiles, SCAN_THREADS, 0, counted(s)>>>(in, n, sums);
     FEMD_TRY_CUDA(cudaGetLastError());
-    FEMD_TRY(exclusive_scan_int(sums, sums, tiles, tmp + tiles + 1, s));
-    k_scan_add<<<grid_for(n, 256), 256, 0, counted(s)>>>(out, n, sums);
+    if (tiles <= SCAN_DIRECT) {
+        k_scan_tiles<true><<<(unsigned)tiles, SCAN_THREADS, 0, counted(s)>>>(in, out, copy, n, sums);
+    } else {
+        FEMD_TRY(exclusive_scan_int(sums, sums, tiles, tmp + tiles + 1, s));
+        k_scan_tiles<false><<<(unsigned)tiles, SCAN_THREADS, 0, counted(s)>>>(in, out, copy, n, sums);
+    }
     FEMD_TRY_CUDA(cudaGetLastError());
     return FEMD_OK;
 }

@@ -469,8 +469,7 @@ int femd_cuda_pattern_from_cells(femd_ctx ctx, int nrows, int ncells, int nloc, 
     if ((st = reset_status(ctx))) return fail(st);
     cudaMemsetAsync(rowlen + nrows, 0, (1 + 4 + nr) * sizeof(int), s);   // the scan's last length, the counters, the counts
     if (tot) k_count_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, cnt, ctx->status_dev);
-    if ((st = exclusive_scan_int(cnt, p->rc_ptr.p, nr, tmp, s))) return fail(st);
-    cudaMemcpyAsync(cnt, p->rc_ptr.p, nr * sizeof(int), cudaMemcpyDeviceToDevice, s);
+    if ((st = exclusive_scan_int(cnt, p->rc_ptr.p, nr, tmp, s, cnt))) return fail(st);   // cnt: the fill positions
     if (tot) k_fill_rows<<<grid_for((size_t)tot, 256, 1u << 20), 256, 0, counted(s)>>>(p->cell_dofs.p, tot, nrows, nloc, cnt, p->rc_code.p);
     // K1: row lengths, scan, columns. Rows of up to PT_CAP columns take a thread each; the longer
     // ones go on a list (in cnt, free again by now) that a warp per row takes.
