@@ -232,7 +232,6 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(
 // ---- K4 ---------------------------------------------------------------------------------------
 // One thread per row; f_i = sum over the row's cells (increasing order) of fe(l), with
 // fe(l) = sum_t sum_q (w_q c_t) row_a(q, l) (assemble_vector_2d, assembly_2d.hpp:188-207).
-template <int MODE>
 __global__ void __launch_bounds__(256) k_assemble_vector(
     const double *__restrict__ pts, const int *__restrict__ tris, const int *__restrict__ rc_ptr,
     const int *__restrict__ rc_code, int nrows, int nloc, int nq, const double *__restrict__ g_ref,
@@ -611,7 +610,7 @@ __global__ void __launch_bounds__(256) k_elem_factors(const double *__restrict__
                     for (int t = 0; t < fs.nterms; ++t) {
                         if (fs.kind[t] == FEMD_COEF_CONST) continue;
                         const double ar = amat(fs.a[t], fs.pr[k], Ji0, Ji1, Ji2, Ji3);
-                        const double bs = fs.vector ? 1.0 : amat(fs.b[t], fs.ps[k], Ji0, Ji1, Ji2, Ji3);
+                        const double bs = amat(fs.b[t], fs.ps[k], Ji0, Ji1, Ji2, Ji3);
                         acc += c[t] * ar * bs;
                     }
                     F[o++] = wq * acc;
@@ -1369,15 +1368,9 @@ int femd_cuda_assemble_vector(femd_ctx ctx, const femd_mesh2d *mesh, const femd_
     const int nl = rule->nloc, nq = rule->nq, n = p->nrows;
     const size_t shm = ((size_t)nq * 3 * nl + nq) * sizeof(double);
     if (n > 0) {
-        if (mode == FEMD_ASM_EXACT) {
-            cudaFuncSetAttribute(k_assemble_vector<FEMD_ASM_EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-            k_assemble_vector<FEMD_ASM_EXACT><<<grid_for((size_t)n, 256, 1u << 22), 256, shm, counted(s)>>>(
-                mesh->points_dev, mesh->tris_dev, p->rc_ptr.p, p->rc_code.p, n, nl, nq, R.ref.p, R.rw.p, ts, f_dev);
-        } else {
-            cudaFuncSetAttribute(k_assemble_vector<FEMD_ASM_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-            k_assemble_vector<FEMD_ASM_FAST><<<grid_for((size_t)n, 256, 1u << 22), 256, shm, counted(s)>>>(
-                mesh->points_dev, mesh->tris_dev, p->rc_ptr.p, p->rc_code.p, n, nl, nq, R.ref.p, R.rw.p, ts, f_dev);
-        }
+        cudaFuncSetAttribute(k_assemble_vector, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+        k_assemble_vector<<<grid_for((size_t)n, 256, 1u << 22), 256, shm, counted(s)>>>(
+            mesh->points_dev, mesh->tris_dev, p->rc_ptr.p, p->rc_code.p, n, nl, nq, R.ref.p, R.rw.p, ts, f_dev);
         FEMD_TRY_CUDA(cudaGetLastError());
     }
     FEMD_TRY_CUDA(cudaStreamSynchronize(s));   // R and scratch are released on return
