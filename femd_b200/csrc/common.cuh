@@ -207,7 +207,8 @@ struct femd_matrix_s : femd::HandleBase {
     // femd_cuda_matrix_set_inv_diag, or the host upload of femd_cuda_cg_solve_host); until then
     // every preconditioned solve refuses the matrix instead of reading uninitialised memory
     bool inv_valid = false;
-    int spmv_tpr = 0;                    // autotuned threads per row (0: not tuned)
+    int spmv_tpr = 0;                    // threads per row and loads per lane, tuned or set (0: the heuristic)
+    bool spmv_tuned = false;             // by the autotuner
     bool resident_unfit = false;         // the on-chip solve has found that a block's rows do not fit
     // the solver workspace of this matrix (vectors, pinned state, captured CUDA graphs), kept
     // between solves so that a solve allocates nothing once it has run once

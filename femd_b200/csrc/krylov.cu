@@ -837,13 +837,15 @@ static unsigned slices_grid(femd_ctx ctx, int n)
 }
 
 // Whether the solves on this matrix use the slices: not where they would be filled up by over a fifth
-// (very uneven rows), nor where a shape of the lane groups was chosen for the matrix.
+// (very uneven rows), nor where the caller set a shape of the lane groups for the matrix.  A shape that
+// the autotuner found is the best of the lane groups, not better than the slices (1024^2 P2: 148-164 us
+// an SpMV against 108): it is for products, and for the solves on uneven rows.
 static int use_slices(femd_ctx ctx, femd_matrix K, bool *use)
 {
     femd_pattern P = K->pattern;
     const int n = P->nrows, nsl = (n + 31) / 32;
     *use = false;
-    if (K->spmv_tpr || n == 0) return FEMD_OK;
+    if ((K->spmv_tpr && !K->spmv_tuned) || n == 0) return FEMD_OK;
     std::lock_guard<std::mutex> guard(P->sl_lock);
     if (P->sl_state == 0) {
         std::lock_guard<std::mutex> word(ctx->shared);
@@ -1691,7 +1693,10 @@ int femd_cuda_spmv_autotune(femd_ctx ctx, femd_matrix K, int set, int *tpr_out, 
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (set) K->spmv_tpr = best;
+    if (set) {
+        K->spmv_tpr = best;
+        K->spmv_tuned = true;
+    }
     if (tpr_out) *tpr_out = best;
     if (us_out) *us_out = best_ms * 1e3;
     return FEMD_OK;
@@ -1706,6 +1711,7 @@ int femd_cuda_spmv_set_tpr(femd_matrix K, int tpr)
     FEMD_CHECK_ARG(tpr == 0 || ((t == 2 || t == 4 || t == 8 || t == 16 || t == 32) && (u == 0 || u == 1 || u == 2 || u == 4)),
                    "spmv_set_tpr: shape = threads per row (0 heuristic, 2..32) | loads per lane (1, 2, 4) << 8");
     K->spmv_tpr = tpr;
+    K->spmv_tuned = false;
     return FEMD_OK;
 }
 

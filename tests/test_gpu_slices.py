@@ -77,3 +77,15 @@ def test_solves(fb, kind, bound):
     K.set_spmv_tpr(4 | 4 << 8)
     again = fb.cg_solve(K, M, b, None, 100000, 1e-12)[0]
     assert np.linalg.norm((again - half).cpu().numpy()) <= bound * np.linalg.norm(x)
+
+
+def test_a_tuned_shape_leaves_the_slices(fb):
+    """The autotuner's shape is for products: the solve keeps the slices, and so its bits."""
+    import torch
+    K, A = system(fb, "band")
+    b = torch.as_tensor(np.random.default_rng(3).standard_normal(K.nrows)).cuda()
+    M = fb.JacobiPreconditioner(K)
+    x = fb.cg_solve(K, M, b, None, 1000, 1e-10)[0]
+    shape, us = K.autotune_spmv(True)
+    assert shape != 0 and us > 0.0
+    assert torch.equal(fb.cg_solve(K, M, b, None, 1000, 1e-10)[0], x)
