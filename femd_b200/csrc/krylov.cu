@@ -8,9 +8,11 @@
 //
 // Reductions.  Every kernel that produces a dot product writes one partial per block; every block
 // of the next kernel adds them all in one fixed tree and so knows alpha, or beta and the stopping
-// test, without a word from the others (its first block writes the state down).  A last block that
-// adds the partials at the end of a kernel (an atomic ticket; the start and finish kernels, which
-// run once, do that) put 3 to 6 us behind every SpMV and update.  The grid of each kernel depends
+// test, without a word from the others (its first block writes the state down).  What a kernel tests
+// at its start, done and want_ru, it changes in its last block alone (an atomic ticket, taken where the
+// loop stops or pauses): every thread of the launch has made the test by then, so a block that starts late
+// never finds half of itself gone.  A last block that adds the partials at the end of every kernel
+// (the start and finish kernels, which run once, do that) put 3 to 6 us behind every SpMV and update.  The grid of each kernel depends
 // only on n, so the sums -- and the iterates -- have the same bits on every run.  Kernels of an
 // iteration that starts after the stopping test has fired return at once, so whole chunks of
 // iterations are queued (captured in a CUDA graph) and the host only polls between chunks.
@@ -83,6 +85,17 @@ __device__ __forceinline__ bool last_block(unsigned *ticket)
     }
     __syncthreads();
     return amlast;
+}
+
+// p.Ap is not positive, as every block of the launch has found: the last one ends the solve.
+template <class T>
+__device__ __forceinline__ void stop_breakdown(CGState<T> *st)
+{
+    if (last_block(&st->ticket) && threadIdx.x == 0) {
+        st->ticket = 0;
+        st->breakdown = 1;
+        st->done = 1;
+    }
 }
 
 // Sum of NV partial arrays (each gridDim.x long, stride ld) in a fixed order by one block.
@@ -343,7 +356,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_cg_update(T *__restrict__ x, T *_
     double tot[1];
     all_partials<1>(pap, npap, 0, tot, sh);
     if (!(tot[0] > 0.0)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) { st->breakdown = 1; st->done = 1; }
+        stop_breakdown(st);
         return;
     }
     const T a = (T)(rz0 / tot[0]);
@@ -404,22 +417,26 @@ __global__ void __launch_bounds__(RED_BLOCK) k_cg_direction(T *__restrict__ p, c
         // mixed precision: ask for a reliable update when the recurrence residual has dropped by a
         // decade since the last one, or looks converged
         const bool pause = MIXED && (rn <= 0.1 * maxr || stop || bad);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const bool leave = MIXED ? pause : stop || bad;                // the same in every block
+        if ((!leave || last_block(&st->ticket)) && (leave || blockIdx.x == 0) && threadIdx.x == 0) {
             st->rr = tot[0];
             st->it = it;
             st->itn[place ^ 1] = it;
             st->rn = rn;
-            if (MIXED) {
-                st->rz_prev = rz0;
-                if (pause) st->want_ru = 1;
-            } else if (stop || bad) {
-                if (!stop) st->breakdown = 1;
-                st->done = 1;
-            }
+            if (MIXED) st->rz_prev = rz0;
             st->beta = beta;
             st->rz[place ^ 1] = rzn;
+            if (leave) {
+                st->ticket = 0;
+                if (MIXED) {
+                    st->want_ru = 1;
+                } else {
+                    if (!stop) st->breakdown = 1;
+                    st->done = 1;
+                }
+            }
         }
-        if (MIXED ? pause : stop || bad) return;
+        if (leave) return;
     }
     const T b = (T)beta;
     const int step = gridDim.x * RED_BLOCK;
@@ -583,7 +600,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_pc_update(double *__restrict__ x,
     double pAp[1];
     all_partials<1>(pap, npap, 0, pAp, sh);
     if (!(pAp[0] > 0.0)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) { st->breakdown = 1; st->done = 1; }
+        stop_breakdown(st);
         return;
     }
     const double a = st->rz[0] / pAp[0];
