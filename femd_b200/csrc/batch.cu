@@ -1282,15 +1282,17 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
     double pAp = 0.0;
     for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += LS_BB) pAp += __ldcg(part + 2 * (size_t)NE + b);
     pAp = ls_block_sum<LS_BB>(pAp);
+    double v[2] = {0.0, 0.0}, tot[2];
     if (!(pAp > 0.0)) {
-        if (e == L.b0 && threadIdx.x == 0) {
+        // every block of the member finds this; the last one says so, when all threads have made the
+        // test above
+        if (ls_member_sum<LS_BB, 2>(v, part, NE, e, L, &S.t2, tot) && threadIdx.x == 0) {
             S.breakdown = 1;
             ls_finish(S, active);
         }
         return;
     }
     const F alpha = (F)(rz0 / pAp);
-    double v[2] = {0.0, 0.0};
     for (int i0 = L.r0 + (int)threadIdx.x; i0 < L.r1; i0 += UU * LS_BB) {
         if (i0 != L.r0 + (int)threadIdx.x) load(i0);
 #pragma unroll
@@ -1307,7 +1309,6 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
             }
         }
     }
-    double tot[2];
     if (!ls_member_sum<LS_BB, 2>(v, part, NE, e, L, &S.t2, tot)) return;
     if (threadIdx.x == 0) {
         s_ru = 0;
