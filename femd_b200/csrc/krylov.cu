@@ -938,11 +938,11 @@ struct SolverWS {
     size_t nodesm = 0;
     int chm = 0;
     // CG with a general preconditioner: z, and the graph of a chunk for the preconditioner it was
-    // captured with
+    // captured with (by its number: another one may come to lie at a released one's address)
     DevBuf<double> z;
     cudaGraphExec_t xpc = nullptr;
     size_t nodespc = 0;
-    femd_precond pc_for = nullptr;
+    unsigned long long pc_for = 0;
     int chpc = 0;
     ~SolverWS()
     {
@@ -1440,10 +1440,10 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
     if (!W.z.p) FEMD_TRY(W.z.alloc((size_t)n + 1));
     const unsigned gs = W.gs, gr = W.gr;
     const int *done = &W.st.p->done;
-    if (W.pc_for != P) {
+    if (W.pc_for != precond_id(P)) {
         if (W.xpc) cudaGraphExecDestroy(W.xpc);
         W.xpc = nullptr;
-        W.pc_for = P;
+        W.pc_for = precond_id(P);
         W.chpc = n > (1 << 18) ? 2 : 8;
         cudaGraph_t graph = nullptr;
         FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1457,9 +1457,9 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
             k_pc_direction<<<gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.z.p, n, W.st.p);
         }
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
-        if (st != FEMD_OK) { if (graph) cudaGraphDestroy(graph); W.pc_for = nullptr; return st; }
+        if (st != FEMD_OK) { if (graph) cudaGraphDestroy(graph); W.pc_for = 0; return st; }
         if (ce != cudaSuccess) {
-            W.pc_for = nullptr;
+            W.pc_for = 0;
             set_error(std::string("cg: graph capture: ") + cudaGetErrorString(ce));
             return FEMD_ECUDA;
         }
@@ -1468,7 +1468,7 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
         cudaGraphDestroy(graph);
         if (ce != cudaSuccess) {
             W.xpc = nullptr;
-            W.pc_for = nullptr;
+            W.pc_for = 0;
             set_error(std::string("cg: graph instantiate: ") + cudaGetErrorString(ce));
             return FEMD_ECUDA;
         }

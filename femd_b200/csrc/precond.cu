@@ -17,6 +17,7 @@
 // parallelism to give; a faster preconditioner would be a different one (another ordering), with
 // other iterates.
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <limits>
@@ -30,6 +31,7 @@
 struct femd_precond_s : femd::HandleBase {
     femd_ctx ctx = nullptr;
     femd_pattern pattern = nullptr;
+    const unsigned long long id;         // of no other preconditioner of the process, before or after
     int pc_kind = 0;                     // FEMD_PC_ILU0 / FEMD_PC_SSOR
     double omega = 1.0, min_pivot = 0.0;
     int n = 0, nlf = 0, nlb = 0;
@@ -39,7 +41,12 @@ struct femd_precond_s : femd::HandleBase {
     femd::DevBuf<int2> places;
     int threads = 0, slot = 0, zs = 0, ring = 0;
     size_t smem = 0;
-    femd_precond_s() : HandleBase(femd::KIND_PRECOND) {}
+    static unsigned long long next_id()
+    {
+        static std::atomic<unsigned long long> count{0};
+        return ++count;
+    }
+    femd_precond_s() : HandleBase(femd::KIND_PRECOND), id(next_id()) {}
     ~femd_precond_s() override { femd::ctx_release(ctx); }
 };
 
@@ -452,6 +459,7 @@ int precond_enqueue(femd_precond P, const double *r, double *z, const int *skip,
     return FEMD_OK;
 }
 
+unsigned long long precond_id(femd_precond P) { return P->id; }
 int precond_rows(femd_precond P) { return P->n; }
 femd_ctx precond_ctx(femd_precond P) { return P->ctx; }
 femd_pattern precond_pattern(femd_precond P) { return P->pattern; }
