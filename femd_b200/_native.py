@@ -103,6 +103,7 @@ SIGNATURES = {
     "femd_cuda_precond_create": (_I, [_P, _P, _I, _D, C.POINTER(_P)]),
     "femd_cuda_precond_info": (_I, [_P, _PI, _PI, _PI, C.POINTER(C.c_double)]),
     "femd_cuda_precond_apply": (_I, [_P, _P, _P, _P]),
+    "femd_cuda_precond_debug": (_I, [_P, _I]),
     "femd_cuda_cg_precond": (_I, [_P, _P, _P, _P, _P, _I, _D, C.POINTER(femd_cg_result)]),
     "femd_cuda_pcg_mixed": (_I, [_P, _P, _P, _P, _I, _D, C.POINTER(femd_cg_result)]),
     "femd_cuda_cg_jacobi_noalloc": (_I, [_P, _P, _I, _P, _P, _I, _D, C.POINTER(femd_cg_result)]),

@@ -511,6 +511,10 @@ class _PCBase(_Handle):
         self.ctx.leave()
         return z
 
+    def debug(self, spin_limit=-1):
+        """Bound the applications' waits (tests of the failure path); negative: the built-in bound."""
+        check(lib.femd_cuda_precond_debug(self.h, int(spin_limit)))
+
 
 class ILU0Preconditioner(_PCBase):
     """Incomplete LU with no fill on the pattern of K, natural ordering (ILU0Preconditioner,

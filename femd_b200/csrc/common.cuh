@@ -131,6 +131,7 @@ void ctx_release(femd_ctx ctx);
 // the preconditioners of precond.cu: z = M^{-1} r enqueued on s (skipped when *skip is set)
 int precond_enqueue(femd_precond P, const double *r, double *z, const int *skip, cudaStream_t s);
 unsigned long long precond_id(femd_precond P);   // of no other preconditioner of the process
+int precond_take_late(femd_precond P, bool *late, cudaStream_t s);
 int precond_rows(femd_precond P);
 // The FP32 copy of a matrix in row-sum form (the mixed-precision inner iteration): position q of
 // the original CSR goes to a32[dst ? dst[q] : q] as (float) a[q], except each row's diagonal

@@ -1505,6 +1505,15 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
         if (ce != cudaSuccess) { set_error(std::string("cg: ") + cudaGetErrorString(ce)); status = FEMD_ECUDA; }
     }
+    if (status == FEMD_OK && W.st_host->breakdown) {
+        // an application whose wait ran out gives NaN, and so a breakdown
+        bool late = false;
+        FEMD_TRY(precond_take_late(P, &late, s));
+        if (late) {
+            set_error("cg: an application of the preconditioner waited too long for its copies");
+            status = FEMD_ETIMEOUT;
+        }
+    }
     if (status == FEMD_OK) {
         const CGState<double> &S = *W.st_host;
         if (S.nb == 0.0) {

@@ -31,7 +31,7 @@
 struct femd_precond_s : femd::HandleBase {
     femd_ctx ctx = nullptr;
     femd_pattern pattern = nullptr;
-    const unsigned long long id;         // of no other preconditioner of the process, before or after
+    unsigned long long id;               // of no other preconditioner of the process, before or after
     int pc_kind = 0;                     // FEMD_PC_ILU0 / FEMD_PC_SSOR
     double omega = 1.0, min_pivot = 0.0;
     int n = 0, nlf = 0, nlb = 0;
@@ -40,6 +40,9 @@ struct femd_precond_s : femd::HandleBase {
     femd::DevBuf<uint4> chunks;
     femd::DevBuf<int2> places;
     int threads = 0, slot = 0, zs = 0, ring = 0;
+    // the bound of a wait for the ring's copies, and the word an application sets where one ran out
+    int spins = 0;
+    femd::DevBuf<int> late;
     size_t smem = 0;
     static unsigned long long next_id()
     {
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(PC_BLOCK) k_ilu0_factor(const int *__restrict_
 // level also hands them over), a row's first entries are in registers before the barrier that
 // frees it, and z itself lies in shared memory (ZS) while it fits; all of it at 32-bit places in
 // shared memory with constant strides.  One application at P2 64 x 64 (16,129 rows, 254 + 254
-// levels): 935 us with rows read from CSR through the level lists by two launches, 272 here; of
+// levels): 935 us with rows read from CSR through the level lists by two launches, 282 here; of
 // that the division takes 6 %, the subtractions 20 %, loading the next level's rows 24 %.
 //
 // A chunk that no slot holds (the inner nodes of all cells at P3 are one level) is read where it lies.
@@ -158,7 +161,11 @@ __global__ void k_pc_pack(const int *__restrict__ ip, const int *__restrict__ ix
     }
 }
 
-// The ring's copies: one mbarrier a slot, waited on by the copying warp alone.  A wait is bounded.
+// The ring's copies: one mbarrier a slot, waited on by the copying warp alone.  A wait is bounded: past
+// it the block leaves at the next barrier, before anything is read from the slot, gives z back as NaN
+// (so CG ends, by its breakdown test) and sets *late_out, which the solve reports.  The word that every
+// thread reads for it takes 10 us of an application's 282 at P2 64 x 64; a barrier that carries it
+// (__syncthreads_or) 14, a chunk of zeros in the slot's place 21.
 static constexpr int PC_SPINS = 1 << 22;
 
 __device__ __forceinline__ void pc_copy(char *dst, const uint4 *src, int n16, uint64_t *bar)
@@ -169,9 +176,9 @@ __device__ __forceinline__ void pc_copy(char *dst, const uint4 *src, int n16, ui
                  :: "r"(d), "l"(src), "r"(16u * n16), "r"(b) : "memory");
 }
 
-__device__ __forceinline__ bool pc_wait(uint64_t *bar, unsigned parity)
+__device__ __forceinline__ bool pc_wait(uint64_t *bar, unsigned parity, int spins)
 {
-    for (int spin = 0; spin < PC_SPINS; ++spin) {
+    for (int spin = 0; spin < spins; ++spin) {
         unsigned ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
@@ -183,11 +190,11 @@ __device__ __forceinline__ bool pc_wait(uint64_t *bar, unsigned parity)
 // z = M^{-1} r.  ILU(0): z_i = r_i - sum_{p < d_i} v_p z_col, then z_i = (z_i - sum_{p > d_i} v_p
 // z_col) / v_ii (precond.hpp:193-204).  SSOR: (r_i - sum) w / v_ii; z_i c v_ii / w with c = (2 -
 // w) / w; (z_i - sum) w / v_ii (:127-142).  ZS: z in shared memory; RING: the ring's slots; places: the
-// chunks' places and sizes in 16 B (size 0: read where it lies).
+// chunks' places and sizes in 16 B (size 0: read where it lies); spins: the bound of a wait.
 template <bool SSOR, bool ZS, int RING>
 __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__restrict__ chunks, const int2 *__restrict__ places, int nlf,
                                                       int nl, int slot, int n, double w, const double *__restrict__ r,
-                                                      double *z, const int *__restrict__ skip)
+                                                      double *z, const int *__restrict__ skip, int spins, int *late_out)
 {
     extern __shared__ __align__(16) char dyn[];
     if (skip && *skip) return;
@@ -210,12 +217,13 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
         if (tid == 0) z_at(n) = 0.0;
     }
     __shared__ uint64_t bar[RING];
-    __shared__ int s_late;                                   // a copy did not arrive: z is given back as NaN
+    // the level whose barrier followed a wait that ran out (-1: the first barrier): a thread past the barrier
+    // of level L leaves where that is L or before; a later barrier's word may already be there
+    __shared__ volatile int s_late;
     if (tid >= T) {
         // the copying warp: chunk L + 2 is in when level L ends (its threads then load from it)
         const bool lead = tid == T;
         int issued = 0, arrived = 0;
-        bool late = false;
         // chunk k into its slot; one that no slot holds only counts as arrived
         auto issue = [&](int2 c) {
             if (c.y) pc_copy(dyn + ring0 + issued % RING * slot, chunks + c.x, c.y, &bar[issued % RING]);
@@ -224,7 +232,7 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
         };
         int2 next = make_int2(0, 0);                         // the chunk issued after the next barrier
         if (lead) {
-            s_late = 0;
+            s_late = nl;
             for (int k = 0; k < RING; ++k)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((unsigned)__cvta_generic_to_shared(&bar[k])) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -232,20 +240,24 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
             if (issued < nl) next = places[issued];
         }
         for (int L = -1; L < nl; ++L) {
-            if (lead) {
-                for (; arrived < min(L + 3, issued) && !late; ++arrived)
-                    late = !pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u);
-                if (late) s_late = 1;
-            }
+            if (lead)
+                while (arrived < min(L + 3, issued)) {
+                    if (!pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u, spins)) {
+                        s_late = L;
+                        break;
+                    }
+                    ++arrived;
+                }
             __syncwarp();
             __syncthreads();                                 // the level's rows are final, its slot is free
-            if (lead && L >= 0 && issued < nl && !late) {
+            if (s_late <= L) break;
+            if (lead && L >= 0 && issued < nl) {
                 issue(next);
                 if (issued < nl) next = places[issued];
             }
         }
-        if (lead && late)                                    // leave no copy in flight
-            for (; arrived < issued; ++arrived) pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u);
+        if (lead && s_late < nl)                                  // leave no copy in flight
+            for (; arrived < issued; ++arrived) pc_wait(&bar[arrived % RING], (unsigned)(arrived / RING) & 1u, PC_SPINS);
         __syncwarp();
     } else {
         __syncthreads();
@@ -330,13 +342,16 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
         // rows of this level and the next, and whether this level is read where it lies
         int4 head = make_int4(0, 0, -1, 0);
         bool at = places[0].y == 0;
-        if (at) chunk = reinterpret_cast<const char *>(chunks + places[0].x);
+        const bool none = s_late < 0;                        // the first chunks are not here
+        if (none) at = false;
+        else if (at) chunk = reinterpret_cast<const char *>(chunks + places[0].x);
         else {
             head = get4(ringed, 0);
             load(ringed, tid, head.x);
         }
         auto levels = [&](auto forward, int L0, int L1) {
             for (int L = L0; L < L1; ++L) {
+                const int late = s_late;                     // covers the next level's chunk
                 if (at) {
                     head = get4(lies, 0);
                     for (int u = tid; u < head.x; u += T) {
@@ -350,6 +365,7 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
                         row(ringed, forward);
                     }
                 }
+                if (late < L) return;
                 // the next level's rows: its chunk was handed over by the last barrier
                 place = (L + 1) % RING ? place + slot : dyn0 + ring0;
                 at = head.z >= 0;
@@ -361,15 +377,19 @@ __global__ void __launch_bounds__(PC_ROWS + PC_COPY) k_pc_apply(const uint4 *__r
                 __syncthreads();                             // the level's rows are final
             }
         };
-        levels(std::true_type(), 0, nlf);
-        levels(std::false_type(), nlf, nl);
+        if (!none) levels(std::true_type(), 0, nlf);
+        if (s_late >= nlf) levels(std::false_type(), nlf, nl);
     }
-    const bool late = s_late;
-    if (ZS || late)
-        for (int i = tid; i < n; i += blockDim.x) z[i] = late ? __longlong_as_double(0x7ff8000000000000ll) : z_at(i);
+    const bool left = s_late < nl;
+    if (left) {                                              // every thread left at the same barrier
+        __syncthreads();                                     // a last level's rows may just have been stored
+        if (tid == 0) *late_out = 1;
+    }
+    if (ZS || left)
+        for (int i = tid; i < n; i += blockDim.x) z[i] = left ? __longlong_as_double(0x7ff8000000000000ll) : z_at(i);
 }
 
-using PcKernel = void (*)(const uint4 *, const int2 *, int, int, int, int, double, const double *, double *, const int *);
+using PcKernel = void (*)(const uint4 *, const int2 *, int, int, int, int, double, const double *, double *, const int *, int, int *);
 
 template <bool SSOR>
 static PcKernel pc_kernel(bool zs, int ring)
@@ -454,12 +474,27 @@ int precond_enqueue(femd_precond P, const double *r, double *z, const int *skip,
     if (P->n == 0) return FEMD_OK;
     PcKernel k = P->pc_kind == FEMD_PC_ILU0 ? pc_kernel<false>(P->zs, P->ring) : pc_kernel<true>(P->zs, P->ring);
     FEMD_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC_SMEM));
-    k<<<1, P->threads, P->smem, counted(s)>>>(P->chunks.p, P->places.p, P->nlf, P->nlf + P->nlb, P->slot, P->n, P->omega, r, z, skip);
+    k<<<1, P->threads, P->smem, counted(s)>>>(P->chunks.p, P->places.p, P->nlf, P->nlf + P->nlb, P->slot, P->n, P->omega, r, z, skip,
+                                               P->spins, P->late.p);
     FEMD_TRY_CUDA(cudaGetLastError());
     return FEMD_OK;
 }
 
 unsigned long long precond_id(femd_precond P) { return P->id; }
+
+// Whether a wait of an application on s ran out since the last call; waits for s.
+int precond_take_late(femd_precond P, bool *late, cudaStream_t s)
+{
+    int word = 0;
+    *late = false;
+    if (P->n == 0) return FEMD_OK;
+    FEMD_TRY_CUDA(cudaMemcpyAsync(&word, P->late.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FEMD_TRY_CUDA(cudaMemsetAsync(P->late.p, 0, sizeof(int), s));
+    FEMD_TRY_CUDA(cudaStreamSynchronize(s));
+    *late = word != 0;
+    return FEMD_OK;
+}
+
 int precond_rows(femd_precond P) { return P->n; }
 femd_ctx precond_ctx(femd_precond P) { return P->ctx; }
 femd_pattern precond_pattern(femd_precond P) { return P->pattern; }
@@ -549,8 +584,10 @@ int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, double omega
         (st = frows.alloc((size_t)std::max(n, 1))) || (st = fptr.alloc(fp.size())) ||
         (st = brows.alloc((size_t)std::max(n, 1))) || (st = bptr.alloc(bp.size())) || (st = fe.alloc(feoff.size() + 1)) ||
         (st = be.alloc(beoff.size() + 1)) || (st = et.alloc(etot.size() + 1)) || (st = rt.alloc(rtot.size())) ||
-        (st = plc.alloc(place.size())) || (st = P->chunks.alloc((size_t)pl.back() + 1)) || (st = P->places.alloc(first.size())))
+        (st = plc.alloc(place.size())) || (st = P->chunks.alloc((size_t)pl.back() + 1)) || (st = P->places.alloc(first.size())) || (st = P->late.alloc(1)))
         return st;
+    P->spins = PC_SPINS;
+    FEMD_TRY_CUDA(cudaMemsetAsync(P->late.p, 0, sizeof(int), s));
     auto up = [&](void *d, const void *h, size_t bytes) { return bytes ? cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess; };
     if (nnz) FEMD_TRY_CUDA(cudaMemcpyAsync(v.p, K->data.p, (size_t)nnz * sizeof(double), cudaMemcpyDeviceToDevice, s));
     FEMD_TRY_CUDA(up(diag.p, dg.data(), (size_t)n * sizeof(int)));
@@ -606,6 +643,16 @@ int femd_cuda_precond_info(femd_precond handle, int *kind, int *levels_forward, 
     if (levels_forward) *levels_forward = P->nlf;
     if (levels_backward) *levels_backward = P->nlb;
     if (min_pivot) *min_pivot = P->pc_kind == FEMD_PC_ILU0 ? P->min_pivot : 0.0;
+    return FEMD_OK;
+}
+
+int femd_cuda_precond_debug(femd_precond handle, int spin_limit)
+{
+    clear_error();
+    femd_precond_s *P = as_precond(handle);
+    FEMD_CHECK_ARG(P, "preconditioner: not a preconditioner handle");
+    P->spins = spin_limit >= 0 ? spin_limit : PC_SPINS;
+    P->id = femd_precond_s::next_id();   // a chunk captured before has the old bound
     return FEMD_OK;
 }
 

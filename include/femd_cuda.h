@@ -45,7 +45,7 @@ extern "C" {
 #define FEMD_ECUDA       3   /* a CUDA runtime error; femd_cuda_last_error() has its text */
 #define FEMD_EOUTSIDE    4   /* an element entry outside the pattern (reference: std::logic_error) */
 #define FEMD_EZERODIAG   5   /* Jacobi: zero diagonal entry (reference: std::invalid_argument) */
-#define FEMD_ETIMEOUT    6   /* a bounded device-side wait ran out (batched / served solves) */
+#define FEMD_ETIMEOUT    6   /* a bounded device-side wait ran out (batched, served, on-chip, preconditioned solves) */
 #define FEMD_EABORT      7   /* a host-requested abort stopped a batched solve */
 #define FEMD_EPIVOT      8   /* ILU(0): a zero pivot (reference: std::runtime_error -> RuntimeError) */
 
@@ -342,6 +342,9 @@ FEMD_API int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, dou
 FEMD_API int femd_cuda_precond_info(femd_precond P, int *kind, int *levels_forward, int *levels_backward, double *min_pivot);
 /* z = M^{-1} r (r and z device vectors of nrows, distinct), asynchronous on the context's stream. */
 FEMD_API int femd_cuda_precond_apply(femd_ctx ctx, femd_precond P, const double *r_dev, double *z_dev);
+/* For tests of the failure path: bound every wait of an application by spin_limit polls (negative: the
+ * built-in bound).  Where a wait runs out, z is all NaN, and a solve returns FEMD_ETIMEOUT. */
+FEMD_API int femd_cuda_precond_debug(femd_precond P, int spin_limit);
 /* krylov::cg(A, M, x, b, max_iter, tol) with M = P (built on K's pattern): the stopping rule, final true
  * residual, 10 tol acceptance and breakdown tests of cg.hpp:245-290 and 222-237. */
 FEMD_API int femd_cuda_cg_precond(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b_dev, double *x_dev,
