@@ -212,7 +212,8 @@ __global__ void __launch_bounds__(RED_BLOCK) k_spmv(const int *__restrict__ indp
 // blocks: one leaves the last slices uneven (P3 216^2 22.6 us), of four every block of the update
 // adds up twice the partials (mixed P2 512^2: 37.3 us an iteration against 35.0).
 // A lane sums its row in entry order, as the CSR form below does, so both give the same bits.
-// FP32 values: row-sum form, as k_spmv.
+// FP32 values: row-sum form, as k_spmv, and in four chains (entry j in chain j % 4) that are added as
+// its four lanes are: one chain of a row's 19 or 37 terms made the mixed solve's error 1.6 times as large.
 static constexpr int SL_U64 = 5, SL_U32 = 8, SL_BLOCKS = 5;
 
 template <class V, class T, bool DOT>
@@ -223,7 +224,8 @@ __global__ void __launch_bounds__(RED_BLOCK, SL_BLOCKS) k_spmv_slices(const int 
 {
     __shared__ double sh[32];
     constexpr bool ROWSUM = std::is_same<V, float>::value;
-    constexpr int U = ROWSUM ? SL_U32 : SL_U64;
+    constexpr int U = ROWSUM ? SL_U32 : SL_U64, CHAINS = ROWSUM ? 4 : 1;
+    static_assert(U % CHAINS == 0 && (CHAINS == 1 || CHAINS == 4), "entry j is of chain j % CHAINS");
     if (DOT && (st->done || st->want_ru)) return;
     const int lane = threadIdx.x & 31, nsl = (n + 31) >> 5;
     const int gwarp = (blockIdx.x * RED_BLOCK + threadIdx.x) >> 5, nwarp = (gridDim.x * RED_BLOCK) >> 5;
@@ -233,7 +235,9 @@ __global__ void __launch_bounds__(RED_BLOCK, SL_BLOCKS) k_spmv_slices(const int 
         const int *cp = cols + (size_t)32 * b + lane;
         const V *vp = vals + (size_t)32 * b + lane;
         const T xi = (ROWSUM || DOT) && i < n ? __ldg(&x[i]) : T(0);
-        T acc = T(0);
+        T acc[CHAINS];
+#pragma unroll
+        for (int k = 0; k < CHAINS; ++k) acc[k] = T(0);
         for (int j0 = 0; j0 < width; j0 += U) {
             int c[U];
             V v[U];
@@ -248,11 +252,12 @@ __global__ void __launch_bounds__(RED_BLOCK, SL_BLOCKS) k_spmv_slices(const int 
             for (int u = 0; u < U; ++u) xv[u] = c[u] >= 0 ? __ldg(&x[c[u]]) : T(0);
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (c[u] >= 0) acc = fma((T)v[u], ROWSUM && c[u] != i ? xv[u] - xi : xv[u], acc);
+                if (c[u] >= 0) acc[u % CHAINS] = fma((T)v[u], ROWSUM && c[u] != i ? xv[u] - xi : xv[u], acc[u % CHAINS]);
         }
+        const T sum = CHAINS == 4 ? (acc[0] + acc[2 % CHAINS]) + (acc[1 % CHAINS] + acc[3 % CHAINS]) : acc[0];
         if (i < n) {
-            y[i] = acc;
-            if (DOT) dot += (double)xi * (double)acc;
+            y[i] = sum;
+            if (DOT) dot += (double)xi * (double)sum;
         }
     }
     if (DOT) write_partial(dot, part, sh);
