@@ -900,6 +900,18 @@ __global__ void __launch_bounds__(128) k_pair_offsets(const int *__restrict__ rc
     }
 }
 
+// Cells that name a dof twice: k_assemble_rows_off takes a pair's columns as distinct.
+__global__ void __launch_bounds__(128) k_repeated_dofs(const int *__restrict__ dofs, int ne, int nloc, int *__restrict__ status)
+{
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
+        const int *d = dofs + (size_t)e * nloc;
+        bool twice = false;
+        for (int j = 1; j < nloc; ++j)
+            for (int l = 0; l < j; ++l) twice |= d[j] >= 0 && d[j] == d[l];
+        if (twice) atomicOr(status, ST_REPEAT);
+    }
+}
+
 static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
 {
     if (p->pair_off.p) return FEMD_OK;
@@ -911,6 +923,9 @@ static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
         k_pair_offsets<<<grid_for((size_t)p->nrows, 128, 1u << 20), 128, 0, counted(ctx->stream)>>>(
             p->rc_ptr.p, p->rc_code.p, p->indptr.p, p->indices.p, p->cell_dofs.p, p->nrows, p->nloc, offs,
             reinterpret_cast<unsigned *>(p->pair_off.p), ctx->status_dev);
+    if (p->ncells)
+        k_repeated_dofs<<<grid_for((size_t)p->ncells, 128, 1u << 20), 128, 0, counted(ctx->stream)>>>(p->cell_dofs.p, p->ncells,
+                                                                                                    p->nloc, ctx->status_dev);
     FEMD_TRY_CUDA(cudaGetLastError());
     int flags = 0;
     FEMD_TRY(read_status(ctx, &flags, nullptr));
@@ -919,6 +934,7 @@ static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
         set_error("assemble_matrix_2d: entry outside the pattern");
         return FEMD_EOUTSIDE;
     }
+    p->pair_repeat = (flags & ST_REPEAT) != 0;
     return FEMD_OK;
 }
 
@@ -1159,7 +1175,14 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     // element matrices where a coefficient varies, and for constant forms whose factors the row
     // kernel below has no instance for; factors per cell else (P2: 24-32 B a cell against 288)
     const bool listed = fs.npair == 1 || fs.npair == 3 || fs.npair == 4 || fs.npair == 5;
-    const bool element = !vector && (nl == 3 || nl == 6 || nl == 10) && (fs.has_var || !listed);
+    // the row kernel over the pair offsets: P1 to P3, unless a cell names a dof twice
+    bool pairs = !vector && (nl == 3 || nl == 6 || nl == 10);
+    if (pairs) {
+        FEMD_TRY(build_pair_offsets(ctx, p));
+        pairs = !p->pair_repeat;
+    }
+    if (!vector && !pairs) FEMD_TRY(build_scatter_map(ctx, p));
+    const bool element = pairs && (fs.has_var || !listed);
     const bool tensors = !vector && !element;
     const size_t nS = tensors ? (size_t)fs.npair * nl2 : 0;
     std::vector<double> tab(3 * (size_t)nq + nref + nS, 0.0);
@@ -1180,10 +1203,6 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
                 }
     }
     const size_t per_cell = vector ? (size_t)nl : element ? (size_t)nl2 : (size_t)fs.nf;
-    if (!vector) {
-        const bool by_pairs = (nl == 3 || nl == 6 || nl == 10) && (element || listed);
-        FEMD_TRY(by_pairs ? build_pair_offsets(ctx, p) : build_scatter_map(ctx, p));
-    }
     const size_t cells = (size_t)ne * per_cell + 1;
     std::unique_lock<std::mutex> guard(ctx->shared);
     DevBuf<double> *Wp = nullptr;
@@ -1260,7 +1279,7 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
         const size_t sho = ((size_t)np * nl2 + (size_t)maxlen * FAST_BLOCK) * sizeof(double) +
                            (FAST_BLOCK / 32) * 33 * sizeof(int) + (size_t)FAST_BLOCK * maxlen;
 #define FEMD_ROWS_OFF(NL, NP)                                                                                          \
-        if (nl == NL && np == NP) {                                                                                    \
+        if (pairs && nl == NL && np == NP) {                                                                                  \
             cudaFuncSetAttribute(k_assemble_rows_off<NL, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sho); \
             k_assemble_rows_off<NL, NP><<<grid, FAST_BLOCK, sho, counted(s)>>>(                                        \
                 p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->pair_off.p, p->diag_pos.p, n, W.p, d_S, maxlen, \
@@ -1270,7 +1289,7 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
         FEMD_ROWS_OFF(6, 0) FEMD_ROWS_OFF(6, 1) FEMD_ROWS_OFF(6, 3) FEMD_ROWS_OFF(6, 4) FEMD_ROWS_OFF(6, 5)
         FEMD_ROWS_OFF(10, 0) FEMD_ROWS_OFF(10, 1) FEMD_ROWS_OFF(10, 3) FEMD_ROWS_OFF(10, 4) FEMD_ROWS_OFF(10, 5)
 #undef FEMD_ROWS_OFF
-        if (!((nl == 3 || nl == 6 || nl == 10) && (element || listed))) {
+        if (!pairs) {
             cudaFuncSetAttribute(k_assemble_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
             k_assemble_rows<<<grid, FAST_BLOCK, shm, counted(s)>>>(p->indptr.p, p->rc_ptr.p, p->rc_code.p, p->map.p,
                                                                    p->diag_pos.p, n, nl, nq, W.p, d_S, d_ref,

@@ -173,6 +173,7 @@ struct femd_pattern_s : femd::HandleBase {
     // columns (uint8, 255 = constrained): the scatter map in the rows' own order, a quarter of
     // its size (built on the first FAST assembly of P1 to P3)
     femd::DevBuf<unsigned char> pair_off;
+    bool pair_repeat = false;                 // a cell names a dof twice (known with pair_off)
     // the batched engine's compact layout of the pattern, built on first use: a reverse
     // Cuthill-McKee order with the rows of every 256 sorted by length (iperm: original row ->
     // reordered row); the entries in slices of 32 reordered rows, column-major within a slice
@@ -268,7 +269,7 @@ inline unsigned grid_for(size_t work, unsigned block, unsigned cap = 1u << 30)
 }
 
 // status flags written by kernels into ctx->status_dev[0]
-enum StatusFlag : int { ST_OUTSIDE = 1, ST_ZERODIAG = 2, ST_ROW_TOO_LONG = 4, ST_TIMEOUT = 8, ST_ABORT = 16 };
+enum StatusFlag : int { ST_OUTSIDE = 1, ST_ZERODIAG = 2, ST_ROW_TOO_LONG = 4, ST_TIMEOUT = 8, ST_ABORT = 16, ST_REPEAT = 32 };
 
 int read_status(femd_ctx ctx, int *flags, int *bad_row);
 int reset_status(femd_ctx ctx);
