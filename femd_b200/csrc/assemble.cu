@@ -146,75 +146,78 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(
                 const double x0 = __shfl_sync(gmask, vx, gbase + 0), y0 = __shfl_sync(gmask, vy, gbase + 0);
                 const double x1 = __shfl_sync(gmask, vx, gbase + 1), y1 = __shfl_sync(gmask, vy, gbase + 1);
                 const double x2 = __shfl_sync(gmask, vx, gbase + 2), y2 = __shfl_sync(gmask, vy, gbase + 2);
-                int myj = -1;
+                unsigned mine = 0;                           // the cell's columns at p: one, or more where it repeats a dof
                 for (int j = 0; j < nloc; ++j) {
                     const int pj = __shfl_sync(gmask, mj, gbase + j);
-                    if (pj == p) myj = j;
+                    if (pj == p) mine |= 1u << j;
                 }
-                if (!valid || myj < 0) continue;
+                if (!valid || !mine) continue;
                 const double J0 = __dsub_rn(x1, x0), J1 = __dsub_rn(x2, x0);
                 const double J2 = __dsub_rn(y1, y0), J3 = __dsub_rn(y2, y0);
                 const double d = __dsub_rn(__dmul_rn(J0, J3), __dmul_rn(J1, J2));
                 const double ad = fabs(d);
-                double Ke = 0.0;
-                if (MODE == FEMD_ASM_EXACT) {
-                    const double Ji0 = __ddiv_rn(J3, d), Ji1 = __ddiv_rn(-J1, d);
-                    const double Ji2 = __ddiv_rn(-J2, d), Ji3 = __ddiv_rn(J0, d);
-                    for (int t = 0; t < ts.nterms; ++t) {
-                        const int ma = ts.a[t], mb = ts.b[t];
-                        for (int q = 0; q < nq; ++q) {
-                            const double w = __dmul_rn(srw[q], ad);
-                            const double ct = ts.is_const[t] ? ts.cval[t] : ts.cpts[t][(size_t)e * nq + q];
-                            const double s = __dmul_rn(w, ct);
-                            if (s == 0.0) continue;
-                            const double *R = sref + q * 3 * nloc;
-                            double ra, rb;
-                            if (ma == 0) ra = R[l];
-                            else {
-                                const double aa = ma == 1 ? Ji0 : Ji1, bb = ma == 1 ? Ji2 : Ji3;
-                                ra = __dadd_rn(__dmul_rn(aa, R[nloc + l]), __dmul_rn(bb, R[2 * nloc + l]));
-                            }
-                            const double sa = __dmul_rn(s, ra);
-                            if (sa == 0.0) continue;
-                            if (mb == 0) rb = R[myj];
-                            else {
-                                const double aa = mb == 1 ? Ji0 : Ji1, bb = mb == 1 ? Ji2 : Ji3;
-                                rb = __dadd_rn(__dmul_rn(aa, R[nloc + myj]), __dmul_rn(bb, R[2 * nloc + myj]));
-                            }
-                            Ke = __dadd_rn(Ke, __dmul_rn(sa, rb));
-                        }
-                    }
-                    acc = __dadd_rn(acc, Ke);
-                } else {
-                    const double rd = 1.0 / d;
-                    // A[m][r]: code m of the physical row in terms of reference row r (value, xi, eta)
-                    const double A[3][3] = {{1.0, 0.0, 0.0}, {0.0, J3 * rd, -J2 * rd}, {0.0, -J1 * rd, J0 * rd}};
-                    double G9[9];
-#pragma unroll
-                    for (int r = 0; r < 9; ++r) G9[r] = 0.0;
-                    for (int t = 0; t < ts.nterms; ++t) {
-                        const int ma = ts.a[t], mb = ts.b[t];
-                        if (ts.is_const[t]) {
-                            const double cs = ts.cval[t] * ad;
-#pragma unroll
-                            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                                for (int s = 0; s < 3; ++s) G9[3 * r + s] += cs * A[ma][r] * A[mb][s];
-                        } else {
-                            const double *cp = ts.cpts[t] + (size_t)e * nq;
+                for (; mine; mine &= mine - 1) {
+                    const int myj = __ffs(mine) - 1;
+                    double Ke = 0.0;
+                    if (MODE == FEMD_ASM_EXACT) {
+                        const double Ji0 = __ddiv_rn(J3, d), Ji1 = __ddiv_rn(-J1, d);
+                        const double Ji2 = __ddiv_rn(-J2, d), Ji3 = __ddiv_rn(J0, d);
+                        for (int t = 0; t < ts.nterms; ++t) {
+                            const int ma = ts.a[t], mb = ts.b[t];
                             for (int q = 0; q < nq; ++q) {
+                                const double w = __dmul_rn(srw[q], ad);
+                                const double ct = ts.is_const[t] ? ts.cval[t] : ts.cpts[t][(size_t)e * nq + q];
+                                const double s = __dmul_rn(w, ct);
+                                if (s == 0.0) continue;
                                 const double *R = sref + q * 3 * nloc;
-                                const double ra = A[ma][0] * R[l] + A[ma][1] * R[nloc + l] + A[ma][2] * R[2 * nloc + l];
-                                const double rb = A[mb][0] * R[myj] + A[mb][1] * R[nloc + myj] + A[mb][2] * R[2 * nloc + myj];
-                                Ke += (srw[q] * ad * cp[q]) * ra * rb;
+                                double ra, rb;
+                                if (ma == 0) ra = R[l];
+                                else {
+                                    const double aa = ma == 1 ? Ji0 : Ji1, bb = ma == 1 ? Ji2 : Ji3;
+                                    ra = __dadd_rn(__dmul_rn(aa, R[nloc + l]), __dmul_rn(bb, R[2 * nloc + l]));
+                                }
+                                const double sa = __dmul_rn(s, ra);
+                                if (sa == 0.0) continue;
+                                if (mb == 0) rb = R[myj];
+                                else {
+                                    const double aa = mb == 1 ? Ji0 : Ji1, bb = mb == 1 ? Ji2 : Ji3;
+                                    rb = __dadd_rn(__dmul_rn(aa, R[nloc + myj]), __dmul_rn(bb, R[2 * nloc + myj]));
+                                }
+                                Ke = __dadd_rn(Ke, __dmul_rn(sa, rb));
                             }
                         }
-                    }
-                    const int lj = l * nloc + myj;
+                        acc = __dadd_rn(acc, Ke);
+                    } else {
+                        const double rd = 1.0 / d;
+                        // A[m][r]: code m of the physical row in terms of reference row r (value, xi, eta)
+                        const double A[3][3] = {{1.0, 0.0, 0.0}, {0.0, J3 * rd, -J2 * rd}, {0.0, -J1 * rd, J0 * rd}};
+                        double G9[9];
 #pragma unroll
-                    for (int r = 0; r < 9; ++r)
-                        if (G9[r] != 0.0) Ke += G9[r] * sS[r * nloc * nloc + lj];
-                    acc += Ke;
+                        for (int r = 0; r < 9; ++r) G9[r] = 0.0;
+                        for (int t = 0; t < ts.nterms; ++t) {
+                            const int ma = ts.a[t], mb = ts.b[t];
+                            if (ts.is_const[t]) {
+                                const double cs = ts.cval[t] * ad;
+#pragma unroll
+                                for (int r = 0; r < 3; ++r)
+#pragma unroll
+                                    for (int s = 0; s < 3; ++s) G9[3 * r + s] += cs * A[ma][r] * A[mb][s];
+                            } else {
+                                const double *cp = ts.cpts[t] + (size_t)e * nq;
+                                for (int q = 0; q < nq; ++q) {
+                                    const double *R = sref + q * 3 * nloc;
+                                    const double ra = A[ma][0] * R[l] + A[ma][1] * R[nloc + l] + A[ma][2] * R[2 * nloc + l];
+                                    const double rb = A[mb][0] * R[myj] + A[mb][1] * R[nloc + myj] + A[mb][2] * R[2 * nloc + myj];
+                                    Ke += (srw[q] * ad * cp[q]) * ra * rb;
+                                }
+                            }
+                        }
+                        const int lj = l * nloc + myj;
+#pragma unroll
+                        for (int r = 0; r < 9; ++r)
+                            if (G9[r] != 0.0) Ke += G9[r] * sS[r * nloc * nloc + lj];
+                        acc += Ke;
+                    }
                 }
             }
             if (valid) {

@@ -1,4 +1,4 @@
-"""Cells that name a dof twice (a mesh one cell wide with its sides identified): the FAST assembly adds
+"""Cells that name a dof twice (a mesh one cell wide with its sides identified): the assembly adds
 all their contributions, G^T A G with A the matrix before the sides are identified.
 
 Tolerance: an entry is a sum of at most 8 cells x 9 repeats x 3 terms x 36 points products, each formed
@@ -34,9 +34,10 @@ def pattern(fb, n, dofs):
     return P
 
 
+@pytest.mark.parametrize("exact", [False, True])
 @pytest.mark.parametrize("form", ["constant", "varying", "unsymmetric"])
 @pytest.mark.parametrize("k", [1, 2, 3, 4])
-def test_fast_adds_all(fb, k, form):
+def test_all_are_added(fb, k, form, exact):
     m = fb.rectangle_mesh(0, 0, 1, 1, 1, 9)
     V = fb.LagrangeSpace2D(m, k)
     # the vertices of the side x = 1 become those of x = 0
@@ -56,7 +57,7 @@ def test_fast_adds_all(fb, k, form):
                "unsymmetric": ([0], [1], [one])}[form]
     def assembled(P):
         K = fb.CSRMatrix(P)
-        fb.assemble_matrix_2d(Q, Q, a, b, c, K, jacobi=False)
+        fb.assemble_matrix_2d(Q, Q, a, b, c, K, jacobi=False, exact=exact)
         ip, ix = P.to_host()
         return sp.csr_matrix((K.data, ix, ip), shape=(V.dim, V.dim))
 
