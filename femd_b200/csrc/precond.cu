@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "precond_host.h"
 
 struct femd_precond_s : femd::HandleBase {
     femd_ctx ctx = nullptr;
@@ -34,7 +35,8 @@ struct femd_precond_s : femd::HandleBase {
     unsigned long long id;               // of no other preconditioner of the process, before or after
     int pc_kind = 0;                     // FEMD_PC_ILU0 / FEMD_PC_SSOR
     double omega = 1.0, min_pivot = 0.0;
-    int n = 0, nlf = 0, nlb = 0;
+    int n = 0, levels_f = 0, levels_b = 0;
+    int nlf = 0, nlb = 0;                // chunks: one a level, more where a level is very large
     // the sweeps' chunks, one per forward and backward level in order (k_pc_apply), their places and
     // sizes, and the launch
     femd::DevBuf<uint4> chunks;
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(PC_BLOCK) k_ilu0_factor(const int *__restrict_
 // slice's 128 B together).  The 32 rows of a warp are filled up to the same number of entries, a
 // multiple of 4, with the value +0 on column n, whose z is +0: s - (+0 * +0) is s, bit for bit, so
 // no lane needs a test in the chain.  With z in shared memory a column is its place there in bytes.
-static constexpr int PC_AHEAD = 8, PC_SLICE = 8;
+static constexpr int PC_AHEAD = 8;
 static constexpr int PC_ROWS = 256, PC_COPY = 32;    // threads that take rows (at most), and that copy
 static constexpr size_t PC_SMEM = 220 * 1024;
 
@@ -116,10 +118,7 @@ struct __align__(16) PcRow {
     double diag, pad;
 };
 
-__host__ __device__ inline size_t pc_chunk_bytes(int m, int E)
-{
-    return 16 + sizeof(PcRow) * (size_t)m + 12 * (size_t)E;   // E: a multiple of 4 PC_SLICE
-}
+static_assert(sizeof(PcRow) == PC_RECORD && sizeof(int4) == PC_HEAD, "as the host lays the chunks out");
 
 // Fill the chunks: one thread per row in level order (rows; lptr: the levels' first).
 __global__ void k_pc_pack(const int *__restrict__ ip, const int *__restrict__ ix, const int *__restrict__ diag,
@@ -413,55 +412,6 @@ __global__ void k_pc_min_diag(int n, const int *__restrict__ diag, const double 
     }
 }
 
-// rows grouped by level: level(i) = 1 + max level over the rows that row i reads (its lower part
-// for the forward sweep, its upper part for the backward one, taken from the last row down)
-static void level_schedule(int n, const std::vector<int> &ip, const std::vector<int> &ix, const std::vector<int> &dg,
-                           bool forward, std::vector<int> &rows, std::vector<int> &ptr)
-{
-    std::vector<int> lev((size_t)n, 0);
-    int nl = 0;
-    for (int s = 0; s < n; ++s) {
-        const int i = forward ? s : n - 1 - s;
-        int l = 0;
-        if (forward)
-            for (int p = ip[i]; p < dg[i]; ++p) l = std::max(l, lev[ix[p]] + 1);
-        else
-            for (int p = dg[i] + 1; p < ip[i + 1]; ++p) l = std::max(l, lev[ix[p]] + 1);
-        lev[i] = l;
-        nl = std::max(nl, l + 1);
-    }
-    ptr.assign((size_t)nl + 1, 0);
-    for (int i = 0; i < n; ++i) ++ptr[lev[i] + 1];
-    for (int l = 0; l < nl; ++l) ptr[l + 1] += ptr[l];
-    rows.assign((size_t)n, 0);
-    std::vector<int> fill(ptr.begin(), ptr.end() - 1);
-    for (int i = 0; i < n; ++i) rows[fill[lev[i]]++] = i;
-}
-
-// The chunks of one sweep's levels: per row (in level order) its first entry, per level its entries;
-// the chunks' sizes are appended to place (in 16 B, running).
-static void chunk_layout(const std::vector<int> &ip, const std::vector<int> &dg, bool forward, std::vector<int> &rows,
-                         const std::vector<int> &ptr, std::vector<int> &eoff, std::vector<int> &etot, std::vector<int> &rtot,
-                         std::vector<long long> &place)
-{
-    const int nl = (int)ptr.size() - 1;
-    auto length = [&](int i) { return forward ? dg[i] - ip[i] : ip[i + 1] - dg[i] - 1; };
-    eoff.assign(rows.size(), 0);
-    for (int l = 0; l < nl; ++l) {
-        std::stable_sort(rows.begin() + ptr[l], rows.begin() + ptr[l + 1], [&](int a, int b) { return length(a) > length(b); });
-        const int m = ptr[l + 1] - ptr[l];
-        int E = 0;
-        for (int u = 0; u < m; u += PC_SLICE) {
-            for (int j = 0; j < std::min(PC_SLICE, m - u); ++j) eoff[ptr[l] + u + j] = E;
-            E += PC_SLICE * ((length(rows[ptr[l] + (u & ~31)]) + 3) & ~3);
-        }
-        etot.push_back(E);
-        rtot.push_back(m);
-        const size_t bytes = pc_chunk_bytes(m, E);
-        place.push_back(place.back() + (long long)(bytes / 16));
-    }
-}
-
 static femd_precond_s *as_precond(void *h)
 {
     femd_precond_s *p = static_cast<femd_precond_s *>(h);
@@ -546,13 +496,17 @@ int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, double omega
     std::vector<int> fr, fp, br, bp;
     level_schedule(n, ip, ix, dg, true, fr, fp);
     level_schedule(n, ip, ix, dg, false, br, bp);
-    P->nlf = (int)fp.size() - 1;
-    P->nlb = (int)bp.size() - 1;
+    P->levels_f = (int)fp.size() - 1;
+    P->levels_b = (int)bp.size() - 1;
     std::vector<int> feoff, beoff, etot, rtot;
     std::vector<long long> pl(1, 0);
-    chunk_layout(ip, dg, true, fr, fp, feoff, etot, rtot, pl);
-    chunk_layout(ip, dg, false, br, bp, beoff, etot, rtot, pl);
-    FEMD_CHECK_ARG(pl.back() < INT_MAX, std::string(what) + ": the matrix is too large");
+    chunk_layout(ip, dg, true, PC_CHUNK_MAX, fr, fp, feoff, etot, rtot, pl);
+    chunk_layout(ip, dg, false, PC_CHUNK_MAX, br, bp, beoff, etot, rtot, pl);
+    P->nlf = (int)fp.size() - 1;
+    P->nlb = (int)bp.size() - 1;
+    bool large = pl.back() >= INT_MAX;
+    for (size_t k = 0; k + 1 < pl.size(); ++k) large |= 16 * (pl[k + 1] - pl[k]) > INT_MAX;
+    FEMD_CHECK_ARG(!large, std::string(what) + ": the matrix is too large");
     std::vector<int> place(pl.begin(), pl.end());
     const int nch = P->nlf + P->nlb;
     rtot.push_back(0);                   // the chunk after the last
@@ -640,8 +594,8 @@ int femd_cuda_precond_info(femd_precond handle, int *kind, int *levels_forward, 
     femd_precond_s *P = as_precond(handle);
     FEMD_CHECK_ARG(P, "preconditioner: not a preconditioner handle");
     if (kind) *kind = P->pc_kind;
-    if (levels_forward) *levels_forward = P->nlf;
-    if (levels_backward) *levels_backward = P->nlb;
+    if (levels_forward) *levels_forward = P->levels_f;
+    if (levels_backward) *levels_backward = P->levels_b;
     if (min_pivot) *min_pivot = P->pc_kind == FEMD_PC_ILU0 ? P->min_pivot : 0.0;
     return FEMD_OK;
 }

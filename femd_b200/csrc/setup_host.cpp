@@ -11,6 +11,7 @@
 
 #include "../../include/femd_cuda.h"
 #include "compact_host.h"
+#include "precond_host.h"
 
 namespace femd {
 void set_error(const std::string &msg);
@@ -151,6 +152,64 @@ void compact_layout(int n, const std::vector<int> &ip, const std::vector<int> &i
     }
     L.bw = bw;
     L.ok = bw <= 32767;
+}
+
+// ---- the rows' order of ILU(0) and SSOR (precond_host.h) ------------------------------------
+void level_schedule(int n, const std::vector<int> &ip, const std::vector<int> &ix, const std::vector<int> &dg, bool forward,
+                    std::vector<int> &rows, std::vector<int> &ptr)
+{
+    std::vector<int> lev((size_t)n, 0);
+    int nl = 0;
+    for (int s = 0; s < n; ++s) {
+        const int i = forward ? s : n - 1 - s;
+        int l = 0;
+        if (forward)
+            for (int p = ip[i]; p < dg[i]; ++p) l = std::max(l, lev[ix[p]] + 1);
+        else
+            for (int p = dg[i] + 1; p < ip[i + 1]; ++p) l = std::max(l, lev[ix[p]] + 1);
+        lev[i] = l;
+        nl = std::max(nl, l + 1);
+    }
+    ptr.assign((size_t)nl + 1, 0);
+    for (int i = 0; i < n; ++i) ++ptr[lev[i] + 1];
+    for (int l = 0; l < nl; ++l) ptr[l + 1] += ptr[l];
+    rows.assign((size_t)n, 0);
+    std::vector<int> fill(ptr.begin(), ptr.end() - 1);
+    for (int i = 0; i < n; ++i) rows[fill[lev[i]]++] = i;
+}
+
+void chunk_layout(const std::vector<int> &ip, const std::vector<int> &dg, bool forward, long long limit, std::vector<int> &rows,
+                  std::vector<int> &ptr, std::vector<int> &eoff, std::vector<int> &etot, std::vector<int> &rtot,
+                  std::vector<long long> &place)
+{
+    auto length = [&](int i) { return forward ? dg[i] - ip[i] : ip[i + 1] - dg[i] - 1; };
+    auto filled = [&](int at) { return (length(rows[at]) + 3) & ~3; };       // the entries of the warp of rows that starts here
+    eoff.assign(rows.size(), 0);
+    std::vector<int> first(1, 0);
+    for (size_t l = 0; l + 1 < ptr.size(); ++l) {
+        std::stable_sort(rows.begin() + ptr[l], rows.begin() + ptr[l + 1], [&](int a, int b) { return length(a) > length(b); });
+        for (int r0 = ptr[l], m; r0 < ptr[l + 1]; r0 += m) {
+            const int left = ptr[l + 1] - r0;
+            long long bytes = PC_HEAD;
+            for (m = 0; m < left;) {
+                const int take = std::min(PC_WARP, left - m);
+                bytes += (long long)take * PC_RECORD + 12ll * ((take + PC_SLICE - 1) / PC_SLICE * PC_SLICE) * filled(r0 + m);
+                if (bytes > limit) break;
+                m += take;
+            }
+            if (m == 0) m = std::min(PC_SLICE, left);
+            int E = 0;
+            for (int u = 0; u < m; u += PC_SLICE) {
+                for (int j = 0; j < std::min(PC_SLICE, m - u); ++j) eoff[r0 + u + j] = E;
+                E += PC_SLICE * filled(r0 + u / PC_WARP * PC_WARP);
+            }
+            etot.push_back(E);
+            rtot.push_back(m);
+            place.push_back(place.back() + (long long)(pc_chunk_bytes(m, E) / 16));
+            first.push_back(r0 + m);
+        }
+    }
+    ptr = first;
 }
 
 }  // namespace femd
@@ -435,6 +494,35 @@ int femd_host_rcm_order(int n, const int *indptr, const int *indices, int *order
     std::vector<int> ip(indptr, indptr + n + 1), ix(indices, indices + nnz), out;
     femd::rcm_order(n, ip, ix, out);
     std::copy(out.begin(), out.end(), order);
+    return FEMD_OK;
+}
+
+// The order in which a preconditioner's sweep does the rows (femd::level_schedule, femd::chunk_layout).
+int femd_host_precond_chunks(int n, const int *indptr, const int *indices, int forward, long long limit, int *nchunks, int *rows,
+                             int *first, long long *bytes)
+{
+    femd::clear_error();
+    if (n < 0 || !indptr || (indptr[n] && !indices) || !nchunks || limit < 0) {
+        femd::set_error("precond_chunks: bad arguments");
+        return FEMD_EINVAL;
+    }
+    std::vector<int> ip(indptr, indptr + n + 1), ix(indices, indices + indptr[n]), dg((size_t)n), r, p, eoff, etot, rtot;
+    for (int i = 0; i < n; ++i) {
+        const auto f = std::lower_bound(ix.begin() + ip[i], ix.begin() + ip[i + 1], i);
+        if (f == ix.begin() + ip[i + 1] || *f != i) {
+            femd::set_error("precond_chunks: zero diagonal entry in row " + std::to_string(i));
+            return FEMD_EINVAL;
+        }
+        dg[i] = (int)(f - ix.begin());
+    }
+    std::vector<long long> place(1, 0);
+    femd::level_schedule(n, ip, ix, dg, forward != 0, r, p);
+    femd::chunk_layout(ip, dg, forward != 0, limit ? limit : femd::PC_CHUNK_MAX, r, p, eoff, etot, rtot, place);
+    *nchunks = (int)p.size() - 1;
+    if (rows) std::copy(r.begin(), r.end(), rows);
+    if (first) std::copy(p.begin(), p.end(), first);
+    if (bytes)
+        for (size_t k = 0; k + 1 < place.size(); ++k) bytes[k] = 16 * (place[k + 1] - place[k]);
     return FEMD_OK;
 }
 

@@ -548,6 +548,13 @@ FEMD_API int femd_host_rcm_order(int n, const int *indptr, const int *indices, i
  * then nothing is filled.  No reference counterpart. */
 FEMD_API int femd_host_compact_layout(int n, const int *indptr, const int *indices, long long *nsell, int *bandwidth,
                                       int *iperm, int *rstart, int *dst, short *off, int *tile_lo, int *tile_hi);
+/* The order in which a preconditioner's forward (or backward) sweep does the rows of a square CSR
+ * pattern, computed on the host, here for inspection and tests: chunks of rows that do not depend on
+ * one another, each of rows of one level and of at most limit bytes (0: the built-in limit) or 8 rows.
+ * rows (n): the rows in order; first (*nchunks + 1): the chunks' first rows; bytes (*nchunks): their
+ * sizes; each of the three may be NULL.  No reference counterpart. */
+FEMD_API int femd_host_precond_chunks(int n, const int *indptr, const int *indices, int forward, long long limit,
+                                      int *nchunks, int *rows, int *first, long long *bytes);
 /* The equispaced P_k basis and its reference derivatives at points: out[q][3][nloc]. */
 FEMD_API int femd_host_tabulate(int k, int nq, const double *xi, const double *eta, double *out);
 
