@@ -212,7 +212,7 @@ struct femd_matrix_s : femd::HandleBase {
     bool inv_valid = false;
     int spmv_tpr = 0;                    // threads per row and loads per lane, tuned or set (0: the heuristic)
     bool spmv_tuned = false;             // by the autotuner
-    bool resident_unfit = false;         // the on-chip solve has found that a block's rows do not fit
+    int resident_unfit = 0;              // the forms of the on-chip solve that were found not to hold it
     // the solver workspace of this matrix (vectors, pinned state, captured CUDA graphs), kept
     // between solves so that a solve allocates nothing once it has run once
     void *solver_ws = nullptr;

@@ -1086,7 +1086,7 @@ static int cg_resident(femd_ctx ctx, femd_matrix K, bool jac, const double *b, d
                                           max_iter, tol, zx, slots, out, s);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {
         cudaGetLastError();                     // part of the device is taken away: the streaming loop needs no co-residency
-        K->resident_unfit = true;
+        K->resident_unfit |= plan.cluster ? RES_UNFIT_CLUSTER : RES_UNFIT_GRID;
         return FEMD_OK;
     }
     FEMD_TRY_CUDA(e);
@@ -1099,7 +1099,7 @@ static int cg_resident(femd_ctx ctx, femd_matrix K, bool jac, const double *b, d
         return FEMD_ETIMEOUT;
     }
     if (S->unfit) {
-        K->resident_unfit = true;
+        K->resident_unfit |= plan.cluster ? RES_UNFIT_CLUSTER : RES_UNFIT_GRID;
         return FEMD_OK;
     }
     *ran = true;
@@ -1122,7 +1122,7 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     const int n = P->nrows;
     cudaStream_t s = ctx->stream;
     ResidentPlan plan;
-    if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+    while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
         std::lock_guard<std::mutex> guard(ctx->shared);
         const size_t need = (size_t)n + 1 + RES_SLOT_DOUBLES + RES_OUT_DOUBLES;
         if (ctx->res_scratch.n < need) FEMD_TRY(ctx->res_scratch.alloc(need + need / 4));
@@ -2061,7 +2061,7 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     static_assert(sizeof(ResidentOut) <= sizeof(CGState<double>) && RES_SLOT_DOUBLES <= (size_t)NOALLOC_PART,
                   "the on-chip solve's scratch fits the fixed array");
     ResidentPlan plan;
-    if (!K->resident_unfit && resident_plan(ctx, n, P->nnz, plan)) {
+    while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
         std::lock_guard<std::mutex> guard(ctx->shared);
         bool ran = false;
         FEMD_TRY(cg_resident(ctx, K, jac, b_dev, x_dev, max_iter, tol, plan, r, part, reinterpret_cast<ResidentOut *>(st),

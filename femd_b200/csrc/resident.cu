@@ -488,7 +488,10 @@ using ResKernel = void (*)(ResArgs);
 //             14 / 3.2   15 / 4.5   15 / 4.4  15 / 5.5  17.9 / 6.0  20 / 7.0   24 / 7.2
 // One cluster is taken as long as 16 blocks hold the system: its sums take 0.7 to 1.0 us against
 // 2.0 us over the grid, more than the fewer SMs cost (16,129 rows: 4.4 us).
-bool resident_plan(femd_ctx ctx, int n, long long nnz, ResidentPlan &plan)
+// A lane group holds RES_SLOTS rows, so a block at most RES_SLOTS RES_THREADS: a matrix of few entries a
+// row goes to the grid where the cluster has room for its bytes but not for its rows.  Where a form did not
+// fit after all (rows of very uneven length), the next one is tried, and then the streaming loop.
+bool resident_plan(femd_ctx ctx, int n, long long nnz, int unfit, ResidentPlan &plan)
 {
     // a block's share: 10 B an entry, 4 B a row, and 12 B for each of its distinct columns; on P1-P3
     // meshes of 20 to 400 squares a side the fullest block takes 1.3 to 1.6 times its entries' and
@@ -496,10 +499,10 @@ bool resident_plan(femd_ctx ctx, int n, long long nnz, ResidentPlan &plan)
     const int smem = 220 * 1024;
     const double bytes = 1.6 * (10.0 * (double)nnz + 4.0 * n);
     plan.smem = smem;
-    plan.cluster = bytes <= (double)RES_MAX_CLUSTER * (smem - 20 * 1024);
+    const long long rows = RES_SLOTS * RES_THREADS;
+    plan.cluster = !(unfit & RES_UNFIT_CLUSTER) && bytes <= (double)RES_MAX_CLUSTER * (smem - 20 * 1024) && n <= RES_MAX_CLUSTER * rows;
     plan.blocks = plan.cluster ? RES_MAX_CLUSTER : std::min(ctx->sm_count, RES_MAX_BLOCKS);
-    if (!plan.cluster && bytes > (double)plan.blocks * smem) return false;
-    return true;
+    return plan.cluster || (!(unfit & RES_UNFIT_GRID) && bytes <= (double)plan.blocks * smem && n <= plan.blocks * rows);
 }
 
 cudaError_t resident_launch(const ResidentPlan &plan, const int *indptr, const int *indices, const double *data,

@@ -23,8 +23,10 @@ static constexpr int RES_MAX_BLOCKS = 256;
 static constexpr size_t RES_SUM_DOUBLES = 2 * 3 * RES_MAX_BLOCKS, RES_SLOT_DOUBLES = RES_SUM_DOUBLES + 2;
 static constexpr size_t RES_OUT_DOUBLES = (sizeof(ResidentOut) + sizeof(double) - 1) / sizeof(double);
 
-// Whether (and how) a system of n rows and nnz entries is solved on chip.
-bool resident_plan(femd_ctx ctx, int n, long long nnz, ResidentPlan &plan);
+// Whether (and how) a system of n rows and nnz entries is solved on chip; unfit: the forms that were found
+// not to hold it.
+static constexpr int RES_UNFIT_CLUSTER = 1, RES_UNFIT_GRID = 2;
+bool resident_plan(femd_ctx ctx, int n, long long nnz, int unfit, ResidentPlan &plan);
 
 // One solve on the stream: x is read as the start and holds the solution; inv may be null (no
 // preconditioner). zx: n doubles; slots: RES_SLOT_DOUBLES doubles; out: device.
