@@ -1137,18 +1137,15 @@ static constexpr int FAST_MAX_ROW = 96;   // longest row the shared-memory accum
 // Where the cells' factors, vectors or matrices go: the context's workspace up to its bound (the
 // context's stream orders the assemblies that share it), else, and where the work is being captured (a
 // graph keeps the address), the pattern's own, which is not given back once a capture has used it.
-static int cell_workspace(femd_ctx ctx, femd_pattern p, size_t cells, DevBuf<double> **W)
+static int cell_workspace(femd_ctx ctx, femd_pattern p, size_t cells, bool captured, DevBuf<double> **W)
 {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    FEMD_TRY_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
-    const bool captured = cap != cudaStreamCaptureStatusNone;
     if (!captured && cells <= CTX_SCRATCH) {
         *W = &ctx->asm_scratch;
         return (*W)->n < cells ? (*W)->alloc(std::min(cells + cells / 4, CTX_SCRATCH)) : FEMD_OK;
     }
     *W = &p->ws_factors;
     if ((*W)->n < cells) {
-        if (p->ws_captured) {
+        if (p->ws_captured || captured) {
             p->ws_kept.emplace_back(new DevBuf<double>());
             std::swap(p->ws_kept.back()->p, (*W)->p);
             std::swap(p->ws_kept.back()->n, (*W)->n);
@@ -1160,6 +1157,56 @@ static int cell_workspace(femd_ctx ctx, femd_pattern p, size_t cells, DevBuf<dou
         FEMD_TRY(st);
     }
     p->ws_captured |= captured;
+    return FEMD_OK;
+}
+
+// The slot of a form's tables: the one that holds them, else the least recently used one, refilled
+// (stream-ordered, so kernels still reading the slot's old tables finish first).  A captured assembly's
+// slot is kept as it is, and filled now where it is new: a copy in the graph would only run with it.
+static int table_slot(femd_ctx ctx, femd_pattern p, std::vector<double> &tab, bool captured, femd_pattern_s::TableSlot **out)
+{
+    using Slot = femd_pattern_s::TableSlot;
+    Slot *slot = nullptr, *oldest = nullptr;
+    int free_slots = 0;
+    for (auto &t : p->tables) {
+        if (t->host == tab) slot = t.get();
+        if (t->kept) continue;
+        ++free_slots;
+        if (!oldest || t->used < oldest->used) oldest = t.get();
+    }
+    if (!slot && captured) {
+        std::unique_ptr<Slot> fresh(new Slot());
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // none of this is part of the capture
+        FEMD_TRY_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        int st = fresh->dev.alloc(tab.size());
+        cudaStream_t side = nullptr;
+        cudaError_t e = cudaSuccess;
+        if (st == FEMD_OK) {
+            e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(fresh->dev.p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, side);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(side);
+            if (side) cudaStreamDestroy(side);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        FEMD_TRY(st);
+        FEMD_TRY_CUDA(e);
+        fresh->host = std::move(tab);
+        slot = fresh.get();
+        p->tables.push_back(std::move(fresh));
+    } else if (!slot) {
+        if (free_slots < femd_pattern_s::TABLE_SLOTS) {
+            p->tables.emplace_back(new Slot());
+            oldest = p->tables.back().get();
+        }
+        slot = oldest;
+        slot->host.clear();
+        if (slot->dev.n < tab.size()) FEMD_TRY(slot->dev.alloc(tab.size()));
+        FEMD_TRY_CUDA(cudaMemcpyAsync(slot->dev.p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+        slot->host = std::move(tab);
+    }
+    slot->used = ++p->table_clock;
+    slot->kept |= captured;
+    *out = slot;
     return FEMD_OK;
 }
 
@@ -1208,24 +1255,14 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     const size_t per_cell = vector ? (size_t)nl : element ? (size_t)nl2 : (size_t)fs.nf;
     const size_t cells = (size_t)ne * per_cell + 1;
     std::unique_lock<std::mutex> guard(ctx->shared);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    FEMD_TRY_CUDA(cudaStreamIsCapturing(s, &cap));
+    const bool captured = cap != cudaStreamCaptureStatusNone;
     DevBuf<double> *Wp = nullptr;
-    FEMD_TRY(cell_workspace(ctx, p, cells, &Wp));
+    FEMD_TRY(cell_workspace(ctx, p, cells, captured, &Wp));
     DevBuf<double> &W = *Wp;
-    // the slot holding these tables, else the least recently used one, refilled (stream-ordered,
-    // so kernels still reading the slot's old tables finish first)
     femd_pattern_s::TableSlot *slot = nullptr;
-    for (auto &t : p->tables)
-        if (t.host == tab) { slot = &t; break; }
-    if (!slot) {
-        slot = &p->tables[0];
-        for (auto &t : p->tables)
-            if (t.used < slot->used) slot = &t;
-        slot->host.clear();
-        if (slot->dev.n < tab.size()) FEMD_TRY(slot->dev.alloc(tab.size()));
-        FEMD_TRY_CUDA(cudaMemcpyAsync(slot->dev.p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        slot->host = std::move(tab);
-    }
-    slot->used = ++p->table_clock;
+    FEMD_TRY(table_slot(ctx, p, tab, captured, &slot));
     const double *d_tab = slot->dev.p;
     const double *d_ref = d_tab + 3 * nq, *d_S = d_ref + nref;
     const size_t tshm = (3 * (size_t)nq + nref) * sizeof(double);

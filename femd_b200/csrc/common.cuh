@@ -154,20 +154,22 @@ struct femd_pattern_s : femd::HandleBase {
     bool all_diag = false;             // every row i holds the position (i, i)
     int max_row_cells = 0, max_row_len = 0;
     // assembly workspace past the context's shared one and under capture, grown on demand and reused
-    // across calls; what a capture has used is kept until the pattern goes (ws_kept)
+    // across calls; what a capture has used or found is kept until the pattern goes (ws_kept)
     femd::DevBuf<double> ws_factors;
     bool ws_captured = false;
     std::vector<std::unique_ptr<femd::DevBuf<double>>> ws_kept;
     // the rule's tables (weights, points, reference values, the pair tensors) of the last few
     // forms, each with the host copy it was uploaded from: a repeated assembly of the same form
-    // uploads nothing (a pageable upload can wait for the stream)
+    // uploads nothing (a pageable upload can wait for the stream).  What a captured assembly reads is
+    // kept as it is until the pattern goes (kept), beside TABLE_SLOTS others
     struct TableSlot {
         femd::DevBuf<double> dev;
         std::vector<double> host;
         unsigned long long used = 0;
+        bool kept = false;
     };
     static constexpr int TABLE_SLOTS = 4;
-    TableSlot tables[TABLE_SLOTS];
+    std::vector<std::unique_ptr<TableSlot>> tables;
     unsigned long long table_clock = 0;
     // for every (row, cell) pair of the rc lists, the offsets within the row of the cell's nloc
     // columns (uint8, 255 = constrained): the scatter map in the rows' own order, a quarter of
