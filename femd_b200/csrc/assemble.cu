@@ -917,15 +917,17 @@ __global__ void __launch_bounds__(128) k_repeated_dofs(const int *__restrict__ d
 
 static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
 {
+    CtxLock guard(ctx->shared);
     if (p->pair_off.p) return FEMD_OK;
     const int offs = (p->nloc + 3) / 4 * 4;
     const size_t npairs = (size_t)p->ncells * p->nloc;
-    FEMD_TRY(p->pair_off.alloc(npairs * offs + 4));
+    DevBuf<unsigned char> pair_off;      // the pattern's when it is known to be good
+    FEMD_TRY(pair_off.alloc(npairs * offs + 4));
     FEMD_TRY(reset_status(ctx));
     if (p->nrows)
         k_pair_offsets<<<grid_for((size_t)p->nrows, 128, 1u << 20), 128, 0, counted(ctx->stream)>>>(
             p->rc_ptr.p, p->rc_code.p, p->indptr.p, p->indices.p, p->cell_dofs.p, p->nrows, p->nloc, offs,
-            reinterpret_cast<unsigned *>(p->pair_off.p), ctx->status_dev);
+            reinterpret_cast<unsigned *>(pair_off.p), ctx->status_dev);
     if (p->ncells)
         k_repeated_dofs<<<grid_for((size_t)p->ncells, 128, 1u << 20), 128, 0, counted(ctx->stream)>>>(p->cell_dofs.p, p->ncells,
                                                                                                     p->nloc, ctx->status_dev);
@@ -933,11 +935,11 @@ static int build_pair_offsets(femd_ctx ctx, femd_pattern p)
     int flags = 0;
     FEMD_TRY(read_status(ctx, &flags, nullptr));
     if (flags & ST_OUTSIDE) {
-        p->pair_off.release();
         set_error("assemble_matrix_2d: entry outside the pattern");
         return FEMD_EOUTSIDE;
     }
     p->pair_repeat = (flags & ST_REPEAT) != 0;
+    p->pair_off.swap(pair_off);
     return FEMD_OK;
 }
 
@@ -1254,7 +1256,7 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
     }
     const size_t per_cell = vector ? (size_t)nl : element ? (size_t)nl2 : (size_t)fs.nf;
     const size_t cells = (size_t)ne * per_cell + 1;
-    std::unique_lock<std::mutex> guard(ctx->shared);
+    CtxLock guard(ctx->shared);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     FEMD_TRY_CUDA(cudaStreamIsCapturing(s, &cap));
     const bool captured = cap != cudaStreamCaptureStatusNone;
@@ -1336,7 +1338,6 @@ static int fast_assemble(femd_ctx ctx, const femd_mesh2d *mesh, const femd_rule 
                                                                    fs, maxlen, K->data.p, inv, ctx->status_dev);
         }
     }
-    guard.unlock();
     FEMD_TRY_CUDA(cudaGetLastError());
     K->f32_valid = false;
     if (want_inv) {
@@ -1374,6 +1375,7 @@ int femd_cuda_assemble_matrix(femd_ctx ctx, const femd_mesh2d *mesh, const femd_
     DevBuf<double> scratch;
     TermSpec ts;
     FEMD_TRY(prepare_terms(ctx, mesh, rule, p, nterms, a, b, coef, R, scratch, ts));
+    CtxLock guard(ctx->shared);
     FEMD_TRY(reset_status(ctx));
     const int nl = rule->nloc, nq = rule->nq;
     size_t shm = ((size_t)nq * 3 * nl + nq + (mode == FEMD_ASM_FAST ? 9 * nl * nl : 0)) * sizeof(double);

@@ -92,6 +92,12 @@ struct DevBuf {
         n = count;
         part = true;
     }
+    void swap(DevBuf &o)
+    {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(part, o.part);
+    }
     ~DevBuf() { release(); }
 };
 
@@ -111,10 +117,11 @@ struct femd_ctx_s {
     // a small device status block: [0] error flags, [1] first bad row, [2..3] spare, [4] the slices' width
     int *status_dev = nullptr;
     int *status_host = nullptr;   // pinned
-    // several host threads may use patterns and matrices of one context: held while what follows is in
-    // use, by an assembly until its last kernel is queued (the stream then orders the next), by a
-    // pattern's build and an on-chip solve until they have read their results
-    std::mutex shared;
+    // held while the status words or what follows are in use, so that host threads on one context do not
+    // take them from each other: by an assembly until its last kernel is queued (the stream then orders
+    // the next) or its status is read, by a pattern's, map's, offsets' or preconditioner's build and an
+    // on-chip solve until they have read their results
+    std::recursive_mutex shared;
     // the on-chip solve (resident.cu): device scratch, grown to the largest such system (a few MB at
     // most), pinned room for its result, and the events that time it
     femd::DevBuf<double> res_scratch;
@@ -273,6 +280,8 @@ inline unsigned grid_for(size_t work, unsigned block, unsigned cap = 1u << 30)
 // status flags written by kernels into ctx->status_dev[0]
 enum StatusFlag : int { ST_OUTSIDE = 1, ST_ZERODIAG = 2, ST_ROW_TOO_LONG = 4, ST_TIMEOUT = 8, ST_ABORT = 16, ST_REPEAT = 32 };
 
+// (the caller holds ctx->shared from the one to the other)
+using CtxLock = std::unique_lock<std::recursive_mutex>;
 int read_status(femd_ctx ctx, int *flags, int *bad_row);
 int reset_status(femd_ctx ctx);
 

@@ -870,7 +870,7 @@ static int use_slices(femd_ctx ctx, femd_matrix K, bool *use)
     if ((K->spmv_tpr && !K->spmv_tuned) || n == 0) return FEMD_OK;
     std::lock_guard<std::mutex> guard(P->sl_lock);
     if (P->sl_state == 0) {
-        std::lock_guard<std::mutex> word(ctx->shared);
+        CtxLock word(ctx->shared);
         int *const sum = ctx->status_dev + 4, width = 0;
         FEMD_TRY_CUDA(cudaMemsetAsync(sum, 0, sizeof(int), ctx->stream));
         k_slice_widths<<<grid_for((size_t)nsl, RED_BLOCK / 32), RED_BLOCK, 0, counted(ctx->stream)>>>(P->indptr.p, n, nsl, sum, nullptr);
@@ -1123,7 +1123,7 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     cudaStream_t s = ctx->stream;
     ResidentPlan plan;
     while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
-        std::lock_guard<std::mutex> guard(ctx->shared);
+        CtxLock guard(ctx->shared);
         const size_t need = (size_t)n + 1 + RES_SLOT_DOUBLES + RES_OUT_DOUBLES;
         if (ctx->res_scratch.n < need) FEMD_TRY(ctx->res_scratch.alloc(need + need / 4));
         double *slots = ctx->res_scratch.p, *out = slots + RES_SLOT_DOUBLES;
@@ -1622,6 +1622,7 @@ int femd_cuda_matrix_jacobi(femd_ctx ctx, femd_matrix K)
     FEMD_CHECK_ARG(ctx && K, "Jacobi: NULL argument");
     FEMD_CHECK_ARG(K->pattern->nrows == K->pattern->ncols, "Jacobi: the matrix must be square");
     FEMD_TRY_CUDA(cudaSetDevice(ctx->device));
+    CtxLock guard(ctx->shared);
     FEMD_TRY(reset_status(ctx));
     const int n = K->pattern->nrows;
     if (n) k_jacobi_inv<<<grid_for((size_t)n, 256), 256, 0, counted(ctx->stream)>>>(K->pattern->diag_pos.p, K->data.p, K->inv.p, n,
@@ -2062,7 +2063,7 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
                   "the on-chip solve's scratch fits the fixed array");
     ResidentPlan plan;
     while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
-        std::lock_guard<std::mutex> guard(ctx->shared);
+        CtxLock guard(ctx->shared);
         bool ran = false;
         FEMD_TRY(cg_resident(ctx, K, jac, b_dev, x_dev, max_iter, tol, plan, r, part, reinterpret_cast<ResidentOut *>(st),
                              false, &ran, res));

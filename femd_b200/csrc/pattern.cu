@@ -380,27 +380,29 @@ __global__ void __launch_bounds__(256) k_scatter_map(const int *__restrict__ dof
 
 int build_scatter_map(femd_ctx ctx, femd_pattern p)
 {
+    CtxLock guard(ctx->shared);
     if (p->map.p) return FEMD_OK;
     if (p->cell_dofs.p == nullptr) {
         set_error("scatter map: the pattern was not built from cells");
         return FEMD_EINVAL;
     }
     const long long tot = (long long)p->ncells * p->nloc;
-    FEMD_TRY(p->map.alloc((size_t)tot * p->nloc));
+    DevBuf<int> map;                     // the pattern's when it is known to be good
+    FEMD_TRY(map.alloc((size_t)tot * p->nloc));
     FEMD_TRY(reset_status(ctx));
     if (tot > 0) {
         const unsigned grid = grid_for((size_t)tot, 256, 1u << 20);
         auto k = p->nloc == 3 ? k_scatter_map<3> : p->nloc == 6 ? k_scatter_map<6> : p->nloc == 10 ? k_scatter_map<10> : k_scatter_map<0>;
-        k<<<grid, 256, 0, counted(ctx->stream)>>>(p->cell_dofs.p, tot, p->nloc, p->indptr.p, p->indices.p, p->map.p, ctx->status_dev);
+        k<<<grid, 256, 0, counted(ctx->stream)>>>(p->cell_dofs.p, tot, p->nloc, p->indptr.p, p->indices.p, map.p, ctx->status_dev);
     }
     FEMD_TRY_CUDA(cudaGetLastError());
     int flags = 0;
     FEMD_TRY(read_status(ctx, &flags, nullptr));
     if (flags & ST_OUTSIDE) {
-        p->map.release();
         set_error("assemble_matrix_2d: entry outside the pattern");
         return FEMD_EOUTSIDE;
     }
+    p->map.swap(map);
     return FEMD_OK;
 }
 
@@ -442,7 +444,7 @@ int femd_cuda_pattern_from_cells(femd_ctx ctx, int nrows, int ncells, int nloc, 
     const bool keep = with_rows <= 2 * CTX_SCRATCH, shared = keep || base_ints <= 2 * CTX_SCRATCH;
     const size_t ints = keep ? with_rows : base_ints;
     DevBuf<double> own;
-    std::lock_guard<std::mutex> guard(ctx->shared);
+    CtxLock guard(ctx->shared);
     DevBuf<double> &scratch = shared ? ctx->asm_scratch : own;
     int st;
     if (scratch.n < (ints + 1) / 2 && (st = scratch.alloc((ints + 1) / 2))) return fail(st);

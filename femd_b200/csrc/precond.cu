@@ -556,6 +556,7 @@ int femd_cuda_precond_create(femd_ctx ctx, femd_matrix K, int kind, double omega
     FEMD_TRY_CUDA(up(plc.p, place.data(), place.size() * sizeof(int)));
     FEMD_TRY_CUDA(up(P->places.p, first.data(), first.size() * sizeof(int2)));
     if (kind == FEMD_PC_ILU0 && n) {
+        CtxLock status(ctx->shared);
         FEMD_TRY(reset_status(ctx));
         // status [1] holds the first row with a zero pivot (INT_MAX: none)
         k_ilu0_factor<<<1, PC_BLOCK, 0, counted(s)>>>(Q->indptr.p, Q->indices.p, diag.p, v.p, P->nlf, fptr.p, frows.p,
