@@ -1897,12 +1897,14 @@ static int launch_set(femd_ctx ctx, femd_batch_s *B, std::vector<int> order, int
     const int k = mx ? 1 : 0;
     if (B->graph_state[k] == 0) {
         cudaGraph_t g = nullptr;
+        CaptureScope capturing(capture_mutex());
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             const cudaError_t e2 = enqueue_step(B, mx, s);
             e = cudaStreamEndCapture(s, &g);
             if (e == cudaSuccess) e = e2;
         }
+        capturing.unlock();
         if (e == cudaSuccess) e = cudaGraphInstantiate(&B->exec[k], g, 0);
         if (g) cudaGraphDestroy(g);
         if (e == cudaSuccess) {
@@ -2637,11 +2639,13 @@ static int ls_advance(femd_ctx ctx, femd_batch_s *B, bool mx, int chunks, int *n
                           L.g_state == L.d_state.p && L.g_win == win_b && L.g_chunk == C;
         if (!same && !L.g_refused) {
             cudaGraph_t g = nullptr;
+            CaptureScope capturing(capture_mutex());
             cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
                 enqueue_chunk(NE32, NE64);
                 e = cudaStreamEndCapture(s, &g);
             }
+            capturing.unlock();
             if (e == cudaSuccess && L.gx) {
                 cudaGraphExecUpdateResultInfo info;
                 if (cudaGraphExecUpdate(L.gx, g, &info) != cudaSuccess) {

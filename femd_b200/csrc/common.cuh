@@ -6,6 +6,7 @@
 #include <atomic>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <stdint.h>
 
 #include <string>
@@ -252,6 +253,10 @@ int exclusive_scan_int(const int *in, int *out, size_t n, int *tmp, cudaStream_t
 
 // Kernel launches issued by this library in this process (graph launches count their nodes).
 void add_launches(long long n);
+// Held (shared) while a stream is captured: a device-wide wait in another thread, as a free makes, would
+// end the capture with an error, and would not have waited itself.
+std::shared_mutex &capture_mutex();
+using CaptureScope = std::shared_lock<std::shared_mutex>;
 // The launch-configuration stream argument of every kernel launch goes through counted(): it
 // counts the launch (unless the stream is being captured into a graph) and returns the stream.
 inline cudaStream_t counted(cudaStream_t s)

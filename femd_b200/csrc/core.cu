@@ -34,6 +34,19 @@ struct DevicePool {
 static std::mutex g_pool_mu;
 static DevicePool g_pools[POOL_DEVICES];
 
+std::shared_mutex &capture_mutex()
+{
+    static std::shared_mutex mu;
+    return mu;
+}
+
+// Wait for the device while no thread captures a stream.
+static void device_wait()
+{
+    std::unique_lock<std::shared_mutex> none(capture_mutex());
+    cudaDeviceSynchronize();
+}
+
 static cudaError_t device_pool(int dev, DevicePool **out)
 {
     if (dev < 0 || dev >= POOL_DEVICES) return cudaErrorInvalidDevice;
@@ -75,7 +88,7 @@ cudaError_t dev_alloc(void **p, size_t bytes)
     if (e == cudaErrorMemoryAllocation) {
         // give the pool's idle blocks back to the device and try once more
         cudaGetLastError();
-        cudaDeviceSynchronize();
+        device_wait();
         cudaMemPoolTrimTo(P->pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, P->pool, P->s);
     }
@@ -102,7 +115,7 @@ void dev_free(void *p)
     DevicePool *P = nullptr;
     if (device_pool(dev, &P) != cudaSuccess) return;
     if (dev != cur) cudaSetDevice(dev);
-    cudaDeviceSynchronize();
+    device_wait();
     cudaFreeAsync(p, P->s);
     if (dev != cur) cudaSetDevice(cur);
 }

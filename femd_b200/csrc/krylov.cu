@@ -1043,12 +1043,14 @@ static int capture_cg64(femd_ctx ctx, femd_matrix K, SolverWS &W, bool jac)
     cudaStream_t s = ctx->stream;
     const int n = W.n;
     cudaGraph_t graph = nullptr;
+    CaptureScope capturing(capture_mutex());
     FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < W.ch64; ++k) {
         solve_spmv<true>(K, W, W.p.p, W.Ap.p, s);
         update_direction(jac, W.wx.p, W.r.p, W.p.p, W.Ap.p, K->inv.p, n, W.part.p, W.npap(), W.upd(), W.gr, W.st.p, k & 1, s);
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
+    capturing.unlock();
     if (ce != cudaSuccess) { set_error(std::string("cg: graph capture: ") + cudaGetErrorString(ce)); return FEMD_ECUDA; }
     ce = cudaGraphInstantiate(&W.x64[jac], graph, 0);
     cudaGraphGetNodes(graph, nullptr, &W.nodes64[jac]);
@@ -1277,6 +1279,7 @@ static int prepare_mixed(femd_ctx ctx, femd_matrix K, SolverWS &W)
     W.chm = 32;
     const unsigned gs = W.gs, gr = W.gr;
     cudaGraph_t graph = nullptr;
+    CaptureScope capturing(capture_mutex());
     FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < W.chm; ++k) {
         if (W.slices)
@@ -1291,6 +1294,7 @@ static int prepare_mixed(femd_ctx ctx, femd_matrix K, SolverWS &W)
                                                                                   W.part32.p + W.upd(), gr, W.st32.p, k & 1);
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
+    capturing.unlock();
     if (ce != cudaSuccess) { set_error(std::string("pcg_mixed: graph capture: ") + cudaGetErrorString(ce)); return FEMD_ECUDA; }
     ce = cudaGraphInstantiate(&W.xm, graph, 0);
     cudaGraphGetNodes(graph, nullptr, &W.nodesm);
@@ -1451,6 +1455,7 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
         W.pc_for = precond_id(P);
         W.chpc = n > (1 << 18) ? 2 : 8;
         cudaGraph_t graph = nullptr;
+        CaptureScope capturing(capture_mutex());
         FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         int st = FEMD_OK;
         for (int k = 0; k < W.chpc && st == FEMD_OK; ++k) {
@@ -1462,6 +1467,7 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
             k_pc_direction<<<gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.z.p, n, W.st.p);
         }
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
+        capturing.unlock();
         if (st != FEMD_OK) { if (graph) cudaGraphDestroy(graph); W.pc_for = 0; return st; }
         if (ce != cudaSuccess) {
             W.pc_for = 0;
