@@ -1896,12 +1896,13 @@ static int launch_set(femd_ctx ctx, femd_batch_s *B, std::vector<int> order, int
     cudaError_t e = cudaSuccess;
     const int k = mx ? 1 : 0;
     if (B->graph_state[k] == 0) {
+        CtxLock guard(ctx->shared);
         cudaGraph_t g = nullptr;
         CaptureScope capturing(capture_mutex());
-        e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+        e = cudaStreamBeginCapture(ctx->capture, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            const cudaError_t e2 = enqueue_step(B, mx, s);
-            e = cudaStreamEndCapture(s, &g);
+            const cudaError_t e2 = enqueue_step(B, mx, ctx->capture);
+            e = cudaStreamEndCapture(ctx->capture, &g);
             if (e == cudaSuccess) e = e2;
         }
         capturing.unlock();
@@ -2610,7 +2611,7 @@ static int ls_advance(femd_ctx ctx, femd_batch_s *B, bool mx, int chunks, int *n
     LState *hsb[2] = {hs, hs + L.cap};
     LBlock *htb[2] = {reinterpret_cast<LBlock *>(hs + 2 * (size_t)L.cap), nullptr};
     htb[1] = htb[0] + L.tab_cap;
-    auto enqueue_chunk = [&](int NE32, int NE64) {
+    auto enqueue_chunk = [&](int NE32, int NE64, cudaStream_t s) {
         const LBlock *T32 = L.d_tab.p, *T64 = L.d_tab.p + NE32;
         for (int c = 0; c < C; ++c) {
             if (NE32) {
@@ -2639,11 +2640,12 @@ static int ls_advance(femd_ctx ctx, femd_batch_s *B, bool mx, int chunks, int *n
                           L.g_state == L.d_state.p && L.g_win == win_b && L.g_chunk == C;
         if (!same && !L.g_refused) {
             cudaGraph_t g = nullptr;
+            CtxLock guard(ctx->shared);
             CaptureScope capturing(capture_mutex());
-            cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+            cudaError_t e = cudaStreamBeginCapture(ctx->capture, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
-                enqueue_chunk(NE32, NE64);
-                e = cudaStreamEndCapture(s, &g);
+                enqueue_chunk(NE32, NE64, ctx->capture);
+                e = cudaStreamEndCapture(ctx->capture, &g);
             }
             capturing.unlock();
             if (e == cudaSuccess && L.gx) {
@@ -2674,7 +2676,7 @@ static int ls_advance(femd_ctx ctx, femd_batch_s *B, bool mx, int chunks, int *n
             }
         }
         if (L.gx && !L.g_refused) return launch_graph(L.gx, L.g_nodes, s);
-        enqueue_chunk(NE32, NE64);
+        enqueue_chunk(NE32, NE64, s);
         return cudaGetLastError();
     };
     // the table of the live members (their entries in admission order)

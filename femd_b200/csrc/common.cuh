@@ -114,6 +114,9 @@ struct femd_ctx_s {
     std::atomic<int> refs{1};
     int device = 0;
     cudaStream_t stream = nullptr;
+    // what the library captures (chunks of iterations) it captures on this stream, which nothing else
+    // uses, with `shared` held: work that another thread queues on `stream` meanwhile is not part of it
+    cudaStream_t capture = nullptr;
     int sm_count = 0;
     // a small device status block: [0] error flags, [1] first bad row, [2..3] spare, [4] the slices' width
     int *status_dev = nullptr;

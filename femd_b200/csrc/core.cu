@@ -287,6 +287,7 @@ void ctx_release(femd_ctx ctx)
     if (ctx->res_e0) cudaEventDestroy(ctx->res_e0);
     if (ctx->res_e1) cudaEventDestroy(ctx->res_e1);
     cudaStreamDestroy(ctx->stream);
+    cudaStreamDestroy(ctx->capture);
     delete ctx;
 }
 }  // namespace femd
@@ -318,6 +319,7 @@ int femd_cuda_ctx_create(int device, femd_ctx *out)
     c->device = dev;
     c->sm_count = prop.multiProcessorCount;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->capture, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, 8 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, 4 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&c->res_host, sizeof(femd::ResidentOut));
@@ -331,6 +333,7 @@ int femd_cuda_ctx_create(int device, femd_ctx *out)
         if (c->res_e0) cudaEventDestroy(c->res_e0);
         if (c->res_e1) cudaEventDestroy(c->res_e1);
         if (c->stream) cudaStreamDestroy(c->stream);
+        if (c->capture) cudaStreamDestroy(c->capture);
         delete c;
         return FEMD_ECUDA;
     }

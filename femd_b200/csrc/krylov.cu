@@ -1039,8 +1039,8 @@ static int take_values(femd_ctx ctx, femd_matrix K, SolverWS &W)
 static int capture_cg64(femd_ctx ctx, femd_matrix K, SolverWS &W, bool jac)
 {
     if (W.x64[jac]) return FEMD_OK;
-    femd_pattern P = K->pattern;
-    cudaStream_t s = ctx->stream;
+    CtxLock guard(ctx->shared);
+    cudaStream_t s = ctx->capture;
     const int n = W.n;
     cudaGraph_t graph = nullptr;
     CaptureScope capturing(capture_mutex());
@@ -1264,7 +1264,8 @@ static int prepare_mixed(femd_ctx ctx, femd_matrix K, SolverWS &W)
 {
     if (W.mixed_ready) return FEMD_OK;
     femd_pattern P = K->pattern;
-    cudaStream_t s = ctx->stream;
+    CtxLock guard(ctx->shared);
+    cudaStream_t s = ctx->capture;
     const int n = W.n;
     const size_t npart = 3 * (size_t)std::max({W.gs, W.gr, W.gl}) + 3;
     for (DevBuf<double> *b : {&W.Ax64, &W.r64}) FEMD_TRY(b->alloc((size_t)n + 1));
@@ -1454,19 +1455,21 @@ static int pc_run(femd_ctx ctx, femd_matrix K, femd_precond P, const double *b, 
         W.xpc = nullptr;
         W.pc_for = precond_id(P);
         W.chpc = n > (1 << 18) ? 2 : 8;
+        CtxLock guard(ctx->shared);
+        cudaStream_t cs = ctx->capture;
         cudaGraph_t graph = nullptr;
         CaptureScope capturing(capture_mutex());
-        FEMD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        FEMD_TRY_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         int st = FEMD_OK;
         for (int k = 0; k < W.chpc && st == FEMD_OK; ++k) {
-            launch_spmv<double, double, true>(W.shape, gs, s, Q->indptr.p, Q->indices.p, K->data.p, W.p.p, W.Ap.p, n, W.part.p,
+            launch_spmv<double, double, true>(W.shape, gs, cs, Q->indptr.p, Q->indices.p, K->data.p, W.p.p, W.Ap.p, n, W.part.p,
                                               W.st.p);
-            k_pc_update<<<gr, RED_BLOCK, 0, counted(s)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, n, W.part.p, gs, W.part.p + W.upd(), W.st.p);
-            st = precond_enqueue(P, W.r.p, W.z.p, done, s);
-            k_pc_rz<false><<<gr, RED_BLOCK, 0, counted(s)>>>(W.r.p, W.z.p, nullptr, n, W.part.p, W.st.p);
-            k_pc_direction<<<gr, RED_BLOCK, 0, counted(s)>>>(W.p.p, W.z.p, n, W.st.p);
+            k_pc_update<<<gr, RED_BLOCK, 0, counted(cs)>>>(W.wx.p, W.r.p, W.p.p, W.Ap.p, n, W.part.p, gs, W.part.p + W.upd(), W.st.p);
+            st = precond_enqueue(P, W.r.p, W.z.p, done, cs);
+            k_pc_rz<false><<<gr, RED_BLOCK, 0, counted(cs)>>>(W.r.p, W.z.p, nullptr, n, W.part.p, W.st.p);
+            k_pc_direction<<<gr, RED_BLOCK, 0, counted(cs)>>>(W.p.p, W.z.p, n, W.st.p);
         }
-        cudaError_t ce = cudaStreamEndCapture(s, &graph);
+        cudaError_t ce = cudaStreamEndCapture(cs, &graph);
         capturing.unlock();
         if (st != FEMD_OK) { if (graph) cudaGraphDestroy(graph); W.pc_for = 0; return st; }
         if (ce != cudaSuccess) {

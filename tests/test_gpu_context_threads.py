@@ -98,3 +98,50 @@ def test_zero_diagonals_are_told_to_their_thread(fb):
         return run
 
     assert not in_threads([job(b) for b in (3, -1, 77, -1)])
+
+
+def test_first_solves_beside_assemblies(fb):
+    """A solve's first call on a matrix captures its chunk of iterations; what other threads queue on the
+    context's stream meanwhile is not part of it."""
+    import torch
+    ctx = fb.context()
+    coef = fb.Coef.sinsin(1.0, 0.5, 2 * PI, 3 * PI)
+    V = fb.LagrangeSpace2D(fb.rectangle_mesh(0, 0, 1, 1, 24, 24), 2, bc="dirichlet")
+    V.cell_dofs_device(ctx)
+    P = fb.cell_pattern(V, V, ctx)
+    ip, ix = P.to_host()
+    data, inv = assembled(fb, ctx, V, P, coef)
+    b = torch.as_tensor(np.random.default_rng(0).standard_normal(V.dim)).cuda()
+
+    def fresh():
+        return fb.CSRMatrix.from_arrays(V.dim, V.dim, ip, ix, data, ctx=ctx)
+
+    def mixed():
+        K = fresh()
+        return fb.cg_solve(K, fb.JacobiPreconditioner(K), b, None, 5000, 1e-10, mixed=True)[0]
+
+    def ilu0():
+        K = fresh()
+        return fb.cg_solve(K, fb.ILU0Preconditioner(K), b, None, 5000, 1e-10)[0]
+
+    def lockstep():
+        mats = [fresh(), fresh()]
+        for K in mats:
+            fb.JacobiPreconditioner(K)
+        return fb.Batch(mats, ctx=ctx).solve([b, b], tol=1e-10, mixed=True, engine="lockstep")[0][1]
+
+    solves = [mixed, ilu0, lockstep]
+    refs = [s().cpu().numpy() for s in solves]
+
+    def solving(s, ref):
+        def run():
+            for _ in range(8):
+                assert np.array_equal(s().cpu().numpy(), ref)
+        return run
+
+    def assembling():
+        for _ in range(60):
+            d, i = assembled(fb, ctx, V, P, coef)
+            assert np.array_equal(d, data) and np.array_equal(i, inv)
+
+    assert not in_threads([solving(s, r) for s, r in zip(solves, refs)] + [assembling])
