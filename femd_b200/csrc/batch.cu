@@ -889,10 +889,10 @@ static constexpr int LS_BB = 256;
 static constexpr int LS_RU = 4;
 
 // y = A g on rows [r0, r1) with TPR lanes per row; out(row, sum) by the row's first lane
-template <int BB, int TPR, class V, class F, class Gather, class Pre, class Out>
+template <int TPR, class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_rows(const BProb &P, const V *A, int r0, int r1, Gather g, Pre pre, Out out)
 {
-    constexpr int U = 4, GPW = 32 / TPR, STEP = (BB / 32) * GPW;
+    constexpr int U = 4, GPW = 32 / TPR, STEP = (LS_BB / 32) * GPW;
     const int lane = threadIdx.x % TPR;
     const int sub = (int)(threadIdx.x & 31) / TPR;
     int i0 = r0 + (int)(threadIdx.x >> 5) * GPW;
@@ -985,23 +985,21 @@ __device__ __forceinline__ void sell_round(const BProb &P, const float *__restri
     }
 }
 
-template <int BB>
 __device__ __forceinline__ void sell_prime(const BProb &P, const float *__restrict__ A, int r0, int r1, SellCursor &c)
 {
     const int s0 = r0 + (int)(threadIdx.x >> 5) * 32;
     int end;
     sell_header(P, s0, r1, c.base, end, c.dl);
     c.width = (end - c.base) >> 5;
-    sell_header(P, s0 + BB, r1, c.base1, c.end1, c.dl1);
+    sell_header(P, s0 + LS_BB, r1, c.base1, c.end1, c.dl1);
     sell_round(P, A, c.base, c.width, 0, c.o, c.v);
 }
 
-template <int BB>
 __device__ __forceinline__ void ls_rows_sell(const BProb &P, const float *__restrict__ A, const float *win, int c0, int r0,
                                              int r1, float *__restrict__ Ap, double &dot, SellCursor &c)
 {
     const int lane = threadIdx.x & 31;
-    for (int s0 = r0 + (int)(threadIdx.x >> 5) * 32; s0 < r1; s0 += BB) {
+    for (int s0 = r0 + (int)(threadIdx.x >> 5) * 32; s0 < r1; s0 += LS_BB) {
         const int i = s0 + lane;
         const bool ok = i < r1;                                  // lanes past the member's last row: padding
         const float *wrow = win + (ok ? i - c0 : 0);
@@ -1022,21 +1020,21 @@ __device__ __forceinline__ void ls_rows_sell(const BProb &P, const float *__rest
         c.base = c.base1;
         c.width = (c.end1 - c.base1) >> 5;
         c.dl = c.dl1;
-        sell_header(P, s0 + 2 * BB, r1, c.base1, c.end1, c.dl1);
-        if (s0 + BB < r1) sell_round(P, A, c.base, c.width, 0, c.o, c.v);
+        sell_header(P, s0 + 2 * LS_BB, r1, c.base1, c.end1, c.dl1);
+        if (s0 + LS_BB < r1) sell_round(P, A, c.base, c.width, 0, c.o, c.v);
     }
 }
 
 // SpMV windows: whole rows with at most LS_W nonzeros each (a window's rows start within LS_W -
 // maxlen nonzeros of each other).  A window's column indices and values are read by coalesced
-// loads, LS_W / BB per thread, all issued before the gathers; the products go to shared memory
+// loads, LS_W / LS_BB per thread, all issued before the gathers; the products go to shared memory
 // (two buffers, one barrier per window) and each row is summed in order by one thread.
 static constexpr int LS_W = 1024;
 
-template <int BB, class V, class F, class Gather, class Pre, class Out>
+template <class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, int w1, Gather g, Pre pre, Out out)
 {
-    constexpr int LS_NPT = LS_W / BB;
+    constexpr int LS_NPT = LS_W / LS_BB;
     __shared__ F prod[2][LS_W];
     const int tid = (int)threadIdx.x;
     for (int w = w0; w < w1; ++w) {
@@ -1047,7 +1045,7 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
         V a[LS_NPT];
 #pragma unroll
         for (int t = 0; t < LS_NPT; ++t) {
-            const int q = qs + t * BB + tid;
+            const int q = qs + t * LS_BB + tid;
             col[t] = q < qe ? __ldcs(&P.indices[q]) : -1;
             a[t] = q < qe ? __ldcs(&A[q]) : V(0);
         }
@@ -1062,9 +1060,9 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
         for (int t = 0; t < LS_NPT; ++t) gv[t] = col[t] >= 0 ? g(col[t]) : F(0);
 #pragma unroll
         for (int t = 0; t < LS_NPT; ++t)
-            if (col[t] >= 0) pb[t * BB + tid] = (F)a[t] * gv[t];
+            if (col[t] >= 0) pb[t * LS_BB + tid] = (F)a[t] * gv[t];
         __syncthreads();
-        for (int row = row0; row < re; row += BB) {
+        for (int row = row0; row < re; row += LS_BB) {
             if (row != row0) {
                 lo = P.indptr[row];
                 hi = P.indptr[row + 1];
@@ -1077,33 +1075,32 @@ __device__ __forceinline__ void ls_windows(const BProb &P, const V *A, int w0, i
 }
 
 // y = A g over an entry: by windows when the member has a window table, else by row groups
-template <int BB, class V, class F, class Gather, class Pre, class Out>
+template <class V, class F, class Gather, class Pre, class Out>
 __device__ __forceinline__ void ls_spmv_entry(const BProb &P, const V *A, const LBlock &L, Gather g, Pre pre, Out out)
 {
     if (P.wrow) {
-        ls_windows<BB, V, F>(P, A, L.w0, L.w1, g, pre, out);
+        ls_windows<V, F>(P, A, L.w0, L.w1, g, pre, out);
         return;
     }
     switch (P.tpr) {
-    case 2: ls_rows<BB, 2, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 4: ls_rows<BB, 4, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 8: ls_rows<BB, 8, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    case 16: ls_rows<BB, 16, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
-    default: ls_rows<BB, 32, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 2: ls_rows<2, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 4: ls_rows<4, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 8: ls_rows<8, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    case 16: ls_rows<16, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
+    default: ls_rows<32, V, F>(P, A, L.r0, L.r1, g, pre, out); break;
     }
 }
 
 // the block's sum of v, in every thread
-template <int BB>
 __device__ __forceinline__ double ls_block_sum(double v)
 {
-    __shared__ double sh[BB / 32];
+    __shared__ double sh[LS_BB / 32];
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
     double t = 0.0;
 #pragma unroll
-    for (int w = 0; w < BB / 32; ++w) t += sh[w];
+    for (int w = 0; w < LS_BB / 32; ++w) t += sh[w];
     __syncthreads();
     return t;
 }
@@ -1111,11 +1108,11 @@ __device__ __forceinline__ double ls_block_sum(double v)
 // The member's totals of NV sums.  The block's sums go to part[k * NE + e]; in the member's last
 // block the function returns true (in every thread) with tot = the member's entry partials
 // summed in entry order, and resets the ticket.
-template <int BB, int NV>
+template <int NV>
 __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *part, int NE, int e, const LBlock &L,
                                               unsigned *ticket, double (&tot)[NV])
 {
-    __shared__ double sh[NV][BB / 32];
+    __shared__ double sh[NV][LS_BB / 32];
     __shared__ int last;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -1128,7 +1125,7 @@ __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *par
         for (int k = 0; k < NV; ++k) {
             double t = 0.0;
 #pragma unroll
-            for (int w = 0; w < BB / 32; ++w) t += sh[k][w];
+            for (int w = 0; w < LS_BB / 32; ++w) t += sh[k][w];
             part[(size_t)k * NE + e] = t;
         }
         __threadfence();
@@ -1141,14 +1138,14 @@ __device__ __forceinline__ bool ls_member_sum(const double (&v)[NV], double *par
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         double t = 0.0;
-        for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += BB) t += __ldcg(part + (size_t)k * NE + b);
+        for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += LS_BB) t += __ldcg(part + (size_t)k * NE + b);
         t = warp_sum(t);
         __syncthreads();
         if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = t;
         __syncthreads();
         double u = 0.0;
 #pragma unroll
-        for (int w = 0; w < BB / 32; ++w) u += sh[k][w];
+        for (int w = 0; w < LS_BB / 32; ++w) u += sh[k][w];
         tot[k] = u;
     }
     __syncthreads();
@@ -1173,7 +1170,6 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5)
     k_ls_spmv(const BProb *__restrict__ probs, const LBlock *__restrict__ blks, int NE, LState *st, double *part, int *active,
               int *ru_count, int clear)
 {
-    constexpr int BB = LS_BB;
     using F = typename std::conditional<MIXED, float, double>::type;
     extern __shared__ float ls_win[];
     if (MIXED && clear && blockIdx.x == 0 && threadIdx.x == 0) *ru_count = 0;
@@ -1203,18 +1199,18 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5)
         float *pn = (float *)pnew;
         const float bf = (float)beta;
         SellCursor cur;
-        sell_prime<BB>(P, (const float *)A, L.r0, L.r1, cur);
-        for (int w0 = c0 + (int)threadIdx.x; w0 < c1; w0 += WU * BB) {
+        sell_prime(P, (const float *)A, L.r0, L.r1, cur);
+        for (int w0 = c0 + (int)threadIdx.x; w0 < c1; w0 += WU * LS_BB) {
             float zv[WU], pv[WU];
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int w = w0 + u * BB;
+                const int w = w0 + u * LS_BB;
                 zv[u] = w < c1 ? zf[w] : 0.0f;
                 pv[u] = w < c1 ? pf[w] : 0.0f;
             }
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int w = w0 + u * BB;
+                const int w = w0 + u * LS_BB;
                 if (w < c1) {
                     const float pw = __fmaf_rn(bf, pv[u], zv[u]);
                     ls_win[w - c0] = pw;
@@ -1223,9 +1219,9 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5)
             }
         }
         __syncthreads();
-        ls_rows_sell<BB>(P, (const float *)A, ls_win, c0, L.r0, L.r1, (float *)Ap, dot, cur);
+        ls_rows_sell(P, (const float *)A, ls_win, c0, L.r0, L.r1, (float *)Ap, dot, cur);
     } else {
-        ls_spmv_entry<BB, F, F>(
+        ls_spmv_entry<F, F>(
             P, A, L, [&](int j) { return pdir(z, pold, beta, j); }, [&](int i) { return pdir(z, pold, beta, i); },
             [&](int i, F s, F pi) {
                 pnew[i] = pi;
@@ -1234,7 +1230,7 @@ __global__ void __launch_bounds__(LS_BB, MIXED ? 4 : 5)
             });
     }
     // the entry's share of p.Ap; the update's blocks add up the member's
-    dot = ls_block_sum<BB>(dot);
+    dot = ls_block_sum(dot);
     if (threadIdx.x == 0) part[2 * (size_t)NE + e] = dot;
 }
 
@@ -1281,12 +1277,12 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
     const double rz0 = S.rz;
     double pAp = 0.0;
     for (int b = L.b0 + (int)threadIdx.x; b < L.b1; b += LS_BB) pAp += __ldcg(part + 2 * (size_t)NE + b);
-    pAp = ls_block_sum<LS_BB>(pAp);
+    pAp = ls_block_sum(pAp);
     double v[2] = {0.0, 0.0}, tot[2];
     if (!(pAp > 0.0)) {
         // every block of the member finds this; the last one says so, when all threads have made the
         // test above
-        if (ls_member_sum<LS_BB, 2>(v, part, NE, e, L, &S.t2, tot) && threadIdx.x == 0) {
+        if (ls_member_sum<2>(v, part, NE, e, L, &S.t2, tot) && threadIdx.x == 0) {
             S.breakdown = 1;
             ls_finish(S, active);
         }
@@ -1309,7 +1305,7 @@ __global__ void __launch_bounds__(LS_BB) k_ls_update(const BProb *__restrict__ p
             }
         }
     }
-    if (!ls_member_sum<LS_BB, 2>(v, part, NE, e, L, &S.t2, tot)) return;
+    if (!ls_member_sum<2>(v, part, NE, e, L, &S.t2, tot)) return;
     if (threadIdx.x == 0) {
         s_ru = 0;
         const int it1 = it + 1;
@@ -1378,7 +1374,7 @@ __global__ void __launch_bounds__(LS_BB, 5) k_ls_resid(const BProb *__restrict__
         F *pb = MIXED ? (F *)P.pb32 : (F *)P.pb64;
         const double *x = P.x;
         double v[3] = {0.0, 0.0, 0.0};
-        ls_spmv_entry<LS_BB, double, double>(
+        ls_spmv_entry<double, double>(
             P, P.A64, L, [&](int j) { return x[j]; },
             [&](int i) { return make_double2(P.b[i], MODE == 2 ? 0.0 : P.inv64[i]); },
             [&](int i, double s, double2 own) {
@@ -1405,7 +1401,7 @@ __global__ void __launch_bounds__(LS_BB, 5) k_ls_resid(const BProb *__restrict__
                 }
             });
         double tot[3];
-        if (!ls_member_sum<LS_BB, 3>(v, part, NE, e, L, &S.t3, tot) || threadIdx.x != 0) continue;
+        if (!ls_member_sum<3>(v, part, NE, e, L, &S.t3, tot) || threadIdx.x != 0) continue;
         const double rn = sqrt(tot[0]);
         if (MODE == 0) {
             const double nb = sqrt(tot[2]);
