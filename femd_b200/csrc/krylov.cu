@@ -1116,6 +1116,13 @@ static int cg_resident(femd_ctx ctx, femd_matrix K, bool jac, const double *b, d
     return FEMD_OK;
 }
 
+// A shape of the SpMV that the caller set by hand is kept to: the solve streams with it.  So a program
+// that solves on many contexts at once can have its solves overlap, which those over the whole grid do
+// not.  Solves a second, one and eight threads: 25,281 rows 281 and 286 on chip, 107 and 583 streamed;
+// 67,081 rows 161 and 160, 56 and 195.  Up to some 17,000 rows (a cluster) nine overlap on chip: 6,241 rows
+// 884 and 3,553, 205 and 1,317.
+static bool on_chip(femd_matrix K) { return !K->spmv_tpr || K->spmv_tuned; }
+
 // One FP64 CG solve (cg.hpp:296-350): on chip where the system fits, else on the matrix's workspace.
 static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double *x, int max_iter, double tol,
                   femd_cg_result *res)
@@ -1124,7 +1131,7 @@ static int cg_run(femd_ctx ctx, femd_matrix K, bool jac, const double *b, double
     const int n = P->nrows;
     cudaStream_t s = ctx->stream;
     ResidentPlan plan;
-    while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
+    while (on_chip(K) && resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
         CtxLock guard(ctx->shared);
         const size_t need = (size_t)n + 1 + RES_SLOT_DOUBLES + RES_OUT_DOUBLES;
         if (ctx->res_scratch.n < need) FEMD_TRY(ctx->res_scratch.alloc(need + need / 4));
@@ -2071,7 +2078,7 @@ int femd_cuda_cg_jacobi_noalloc(femd_ctx ctx, femd_matrix K, int use_jacobi, con
     static_assert(sizeof(ResidentOut) <= sizeof(CGState<double>) && RES_SLOT_DOUBLES <= (size_t)NOALLOC_PART,
                   "the on-chip solve's scratch fits the fixed array");
     ResidentPlan plan;
-    while (resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
+    while (on_chip(K) && resident_plan(ctx, n, P->nnz, K->resident_unfit, plan)) {
         CtxLock guard(ctx->shared);
         bool ran = false;
         FEMD_TRY(cg_resident(ctx, K, jac, b_dev, x_dev, max_iter, tol, plan, r, part, reinterpret_cast<ResidentOut *>(st),

@@ -276,7 +276,8 @@ FEMD_API int femd_cuda_spmv(femd_ctx ctx, femd_matrix K, const double *x_dev, do
  * 1, 2, 4 (next byte) -- and returns the fastest (and, with set != 0, keeps it for K's SpMV and
  * CG).  Threads per row changes the summation order of a row, so a tuned matrix may give
  * results that differ from an untuned one in the last bits; loads per lane does not.  Solves that take
- * the sliced form of the matrix (even rows) keep to it; a shape set by hand (below) replaces it. */
+ * the sliced form of the matrix (even rows) or run on chip keep to it; a shape set by hand (below)
+ * replaces both. */
 FEMD_API int femd_cuda_spmv_autotune(femd_ctx ctx, femd_matrix K, int set, int *shape_out, double *us_out);
 /* Fix K's SpMV shape (0 = the built-in heuristic). */
 FEMD_API int femd_cuda_spmv_set_tpr(femd_matrix K, int shape);

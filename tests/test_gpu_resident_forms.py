@@ -42,3 +42,25 @@ def test_on_chip(fb, kind, n):
     assert conv and not brk and its >= 10 and launches <= 3
     # condition numbers below 30
     assert np.linalg.norm(x.cpu().numpy() - xd) <= 1e-10 * np.linalg.norm(xd)
+
+
+def test_a_shape_set_by_hand_is_kept_to(fb):
+    n = 5000
+    A = sp.csr_matrix(tridiagonal(n))
+    K = fb.CSRMatrix.from_arrays(n, n, A.indptr, A.indices, A.data)
+    M = fb.JacobiPreconditioner(K)
+    xd = np.random.default_rng(2).standard_normal(n)
+
+    def solve():
+        before = fb.lib.femd_cuda_kernel_launches()
+        x, conv, its, res, brk = fb.cg_solve(K, M, A @ xd, None, 1000, 1e-12)
+        assert conv and np.linalg.norm(x.cpu().numpy() - xd) <= 1e-10 * np.linalg.norm(xd)
+        return fb.lib.femd_cuda_kernel_launches() - before
+
+    assert solve() <= 3
+    K.set_spmv_tpr(4 | 1 << 8)
+    assert solve() > 30
+    K.set_spmv_tpr(0)
+    assert solve() <= 3
+    K.autotune_spmv(True)
+    assert solve() <= 3
